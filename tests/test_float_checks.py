@@ -67,3 +67,18 @@ def test_reach_bracket_float_cells_and_samples(bounds_harness):
     assert m and int(m.group(2)) == 0 and int(m.group(5)) == 0 and int(m.group(8)) == 0
     assert int(m.group(4)) > 0.6 * int(m.group(3))
     assert int(m.group(7)) > 0.9 * int(m.group(6))
+
+
+@pytest.mark.gpu
+def test_rounded_roots_and_quotients_equal_ieee(tmp_path):
+    """csrc/rounded.cuh against the device's IEEE operators: every float of
+    the admitted ranges as a root's argument and as a divisor, and 10^8
+    quotients, half of them next to a rounding boundary."""
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    out = tmp_path / "check_rounded"
+    subprocess.run([nvcc, "-gencode", "arch=compute_103a,code=sm_103a", "-O3", "-std=c++17", "-fmad=false",
+                    str(ROOT / "tests" / "float_checks" / "check_rounded.cu"), "-o", str(out)], check=True)
+    run = subprocess.run([str(out)], capture_output=True, text=True)
+    assert run.returncode == 0, run.stdout + run.stderr
+    m = re.search(r"root (\d+) reciprocal_root (\d+) reciprocal (\d+) quotient (\d+) of (\d+)", run.stdout)
+    assert m and [int(m.group(k)) for k in (1, 2, 3, 4)] == [0, 0, 0, 0]

@@ -11,7 +11,7 @@
 // 16-byte boundary whatever the brick; boxes that reach past a body's node
 // grid load zeros there and store nothing there.
 //
-// Arithmetic: solveCell on the same corners in the same order as the other
+// Arithmetic: projectCell on the same corners in the same order as the other
 // colour passes (step_device.cuh), so results are equal bit for bit.
 // Every mbarrier wait has an iteration limit; a block whose copies do not
 // arrive records a fault, waits (bounded) for what it has in flight, and
@@ -157,7 +157,9 @@ __global__ void __launch_bounds__(kTmaBlock) elasticTmaKernel(const __grid_const
                 w[c] = a.w;
                 prev[c] = xyz(Q[at[c]]);
             }
-            solveCell<false>(p, prev, w, cellConsts(bodies + e.x), lens);
+            const CellConsts k = cellConsts(bodies + e.x);
+            projectCell<false>(p, prev, w, k);
+            if (k.maxStretch > 1.0f) limitStretch(p, w, k, lens);
 #pragma unroll
             for (int c = 0; c < 8; c++) P[at[c]] = withW(p[c], w[c]);
         }

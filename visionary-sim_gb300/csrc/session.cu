@@ -125,7 +125,7 @@ __device__ __forceinline__ void runJob(const SessionJob& job, const SessionLaunc
                 for (int c = 0; c < 8; c++) {
                     const uint4* cells = a.cells + job.cellFirst[c];
                     for (uint32_t i = tid; i < job.cellCount[c]; i += threads)
-                        solveCellAt<false>(cells[i], k, a.pos, a.prev, L.lens);
+                        solveCellAt<false>(cells[i], a.bodies + body, k, a.pos, a.prev, L.lens);
                     sync();
                 }
             if (limits)
@@ -133,7 +133,7 @@ __device__ __forceinline__ void runJob(const SessionJob& job, const SessionLaunc
                     for (int c = 0; c < 8; c++) {
                         const uint4* cells = a.cells + job.cellFirst[c];
                         for (uint32_t i = tid; i < job.cellCount[c]; i += threads)
-                            solveCellAt<true>(cells[i], k, a.pos, a.prev, L.lens);
+                            solveCellAt<true>(cells[i], a.bodies + body, k, a.pos, a.prev, L.lens);
                         sync();
                     }
             if (contact) {

@@ -10,6 +10,7 @@
 #pragma once
 
 #include "kernels.cuh"
+#include "rounded.cuh"
 
 namespace vsim {
 
@@ -90,23 +91,29 @@ __device__ __forceinline__ M timesBt(const M& A, float s, float ns) {
               sparse3<kKuhn.v[t][0][2], kKuhn.v[t][1][2], kKuhn.v[t][2][2]>(A.c[0], A.c[1], A.c[2], s, ns)}};
 }
 
-// xpbdCouple.wgsl:58-71.
-__device__ __forceinline__ void couple(float cx, float cy, float ax, float ay, float relax, float rx, float ry, float gx,
-                                       float gy, float gz, float& lx, float& ly) {
+// xpbdCouple.wgsl:58-71 up to its divisions: the 2x2 system's determinant
+// and numerators.
+struct Couple2 {
+    float det, nx, ny;
+};
+
+__device__ __forceinline__ Couple2 couple2(float cx, float cy, float ax, float ay, float relax, float rx, float ry,
+                                           float gx, float gy, float gz) {
     const float stiffened = 1.0f + relax;
     const float a00 = fmaf(gx, stiffened, ax);
     const float a01 = gy * stiffened;
     const float a11 = fmaf(gz, stiffened, ay);
-    const float det = fmaf(a00, a11, -(a01 * a01));
-    if (det < 1e-20f) {
-        lx = 0.0f;
-        ly = 0.0f;
-        return;
-    }
     const float bx = -fmaf(rx, relax, cx);
     const float by = -fmaf(ry, relax, cy);
-    lx = fmaf(a11, bx, -(a01 * by)) / det;
-    ly = fmaf(a00, by, -(a01 * bx)) / det;
+    return Couple2{fmaf(a00, a11, -(a01 * a01)), fmaf(a11, bx, -(a01 * by)), fmaf(a00, by, -(a01 * bx))};
+}
+
+// xpbdCouple.wgsl:58-71.
+__device__ __forceinline__ void couple(float cx, float cy, float ax, float ay, float relax, float rx, float ry, float gx,
+                                       float gy, float gz, float& lx, float& ly) {
+    const Couple2 k = couple2(cx, cy, ax, ay, relax, rx, ry, gx, gy, gz);
+    lx = k.det < 1e-20f ? 0.0f : k.nx / k.det;
+    ly = k.det < 1e-20f ? 0.0f : k.ny / k.det;
 }
 
 // sum_i w_i e_i over a tetrahedron's four nodes, fused.
@@ -120,18 +127,33 @@ __device__ __forceinline__ V moved(V p, V d, V h, float lx, float ly, float w) {
     return fma3(fma3(h, ly, d * lx), w, p);
 }
 
-// project.wgsl:75-153, tetrahedron t of the cell held in registers.
-template <int t>
+// project.wgsl:75-153, tetrahedron t of the cell held in registers. With FAST
+// the norm's root and reciprocal and the 2x2 solve's two quotients are
+// rounded.cuh's, whose results are the IEEE operators' where `ranges` holds
+// at the end, and nothing branches, so the compiler schedules across the
+// cell's six tetrahedra: 2,650 cycles a cell against 4,250 with the IEEE
+// operators (one warp, everything in registers). The reference's two early
+// outs need no branch there: a weightless tetrahedron moves nothing, and a
+// determinant under 1e-20 is outside the ranges.
+template <int t, bool FAST>
 __device__ __forceinline__ void projectTet(V (&p)[8], const V (&prev)[8], const float (&w)[8], float s, float ns,
-                                           float alphaDev, float alphaHyd, float gamma, float relax) {
+                                           float alphaDev, float alphaHyd, float gamma, float relax,
+                                           rounded::Ranges& ranges) {
     constexpr int i0 = kTet(t, 0), i1 = kTet(t, 1), i2 = kTet(t, 2), i3 = kTet(t, 3);
     const float w0 = w[i0], w1 = w[i1], w2 = w[i2], w3 = w[i3];
-    if (w0 + w1 + w2 + w3 == 0.0f) return;
+    if (!FAST && w0 + w1 + w2 + w3 == 0.0f) return;
     const V base = p[i0];
     const M F = timesB<t>(M{{p[i1] - base, p[i2] - base, p[i3] - base}}, s, ns);
-    const float cDev = sqrtf(dot(F.c[0], F.c[0]) + dot(F.c[1], F.c[1]) + dot(F.c[2], F.c[2]));
+    const float square = dot(F.c[0], F.c[0]) + dot(F.c[1], F.c[1]) + dot(F.c[2], F.c[2]);
+    float cDev, inv;
+    if (FAST) {
+        rounded::rootAndReciprocal(square, cDev, inv);
+        ranges.reciprocalOfRoot(inv);
+    } else {
+        cDev = sqrtf(square);
+        inv = cDev > 1e-9f ? 1.0f / cDev : 0.0f;
+    }
     const float cHyd = determinant(F) - gamma;
-    const float inv = cDev > 1e-9f ? 1.0f / cDev : 0.0f;
     const M mDev = timesBt<t>(F * inv, s, ns);
     const M mHyd = timesBt<t>(M{{cross(F.c[1], F.c[2]), cross(F.c[2], F.c[0]), cross(F.c[0], F.c[1])}}, s, ns);
     const V d1 = mDev.c[0], d2 = mDev.c[1], d3 = mDev.c[2];
@@ -147,8 +169,18 @@ __device__ __forceinline__ void projectTet(V (&p)[8], const V (&prev)[8], const 
     const V x3 = p[i3] - prev[i3];
     const float rx = dot(d0, x0) + dot(d1, x1) + dot(d2, x2) + dot(d3, x3);
     const float ry = dot(h0, x0) + dot(h1, x1) + dot(h2, x2) + dot(h3, x3);
+    const Couple2 k = couple2(cDev, cHyd, alphaDev, alphaHyd, relax, rx, ry, gx, gy, gz);
     float lx, ly;
-    couple(cDev, cHyd, alphaDev, alphaHyd, relax, rx, ry, gx, gy, gz, lx, ly);
+    if (FAST) {
+        const float r = rounded::reciprocal(k.det, rounded::approxReciprocal(k.det));
+        lx = rounded::quotient(k.nx, k.det, r);
+        ly = rounded::quotient(k.ny, k.det, r);
+        ranges.arguments(square, k.det);
+        ranges.quotients(lx, ly);
+    } else {
+        lx = k.det < 1e-20f ? 0.0f : k.nx / k.det;
+        ly = k.det < 1e-20f ? 0.0f : k.ny / k.det;
+    }
     p[i0] = moved(p[i0], d0, h0, lx, ly, w0);
     p[i1] = moved(p[i1], d1, h1, lx, ly, w1);
     p[i2] = moved(p[i2], d2, h2, lx, ly, w2);
@@ -164,40 +196,55 @@ __device__ __forceinline__ CellConsts cellConsts(const DevBody* b) {
     return CellConsts{b->alphaDev, b->alphaHyd, b->gamma, b->relax, b->restScale, b->h, b->maxStretch};
 }
 
-// project.wgsl:35-184 on one cell held in registers: the six tetrahedra in
-// Kuhn order (unless LIMIT_ONLY), then, with maxStretch > 1, two sweeps of
-// the unilateral length limit over all 28 corner pairs (project.wgsl:162-179).
-template <bool LIMIT_ONLY>
-__device__ __forceinline__ void solveCell(V (&p)[8], const V (&prev)[8], const float (&w)[8], const CellConsts& k,
-                                          const StretchLengths& lens) {
-    if (!LIMIT_ONLY) {
-        const float s = k.restScale, ns = -s;
-        projectTet<0>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax);
-        projectTet<1>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax);
-        projectTet<2>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax);
-        projectTet<3>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax);
-        projectTet<4>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax);
-        projectTet<5>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax);
+// The two sweeps of the unilateral length limit over all 28 corner pairs of a
+// cell whose body limits its stretch (project.wgsl:162-179).
+__device__ __forceinline__ void limitStretch(V (&p)[8], const float (&w)[8], const CellConsts& k,
+                                             const StretchLengths& lens) {
+    float maximum[3], clear[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        maximum[d] = lens.len[d] * k.h * k.maxStretch;
+        // Squared lengths up to here have a root below the limit whatever
+        // the roundings (a relative margin of 2^-20 against a few 2^-24):
+        // such a pair, nearly every one, needs no root.
+        clear[d] = maximum[d] >= 0x1p-50f && maximum[d] <= 0x1p50f ? maximum[d] * maximum[d] * (1.0f - 0x1p-20f)
+                                                                   : -1.0f;
     }
-    if (k.maxStretch > 1.0f) {
-        for (int sweep = 0; sweep < 2; sweep++) {
+    for (int sweep = 0; sweep < 2; sweep++) {
 #pragma unroll
-            for (int a = 0; a < 8; a++) {
+        for (int a = 0; a < 8; a++) {
 #pragma unroll
-                for (int bb = a + 1; bb < 8; bb++) {
-                    const V delta = p[bb] - p[a];
-                    const float len = length(delta);
-                    const float maximum = lens.len[__popc(a ^ bb) - 1] * k.h * k.maxStretch;
-                    const float weight = w[a] + w[bb];
-                    if (len > maximum && weight > 0.0f) {
-                        const V correction = delta * ((len - maximum) / (len * weight));
-                        p[a] = p[a] + w[a] * correction;
-                        p[bb] = p[bb] - w[bb] * correction;
-                    }
+            for (int bb = a + 1; bb < 8; bb++) {
+                const int axes = __popc(a ^ bb) - 1;
+                const V delta = p[bb] - p[a];
+                const float square = dot(delta, delta);
+                if (!(square > clear[axes])) continue;
+                const float len = sqrtf(square);
+                const float weight = w[a] + w[bb];
+                if (len > maximum[axes] && weight > 0.0f) {
+                    const V correction = delta * ((len - maximum[axes]) / (len * weight));
+                    p[a] = p[a] + w[a] * correction;
+                    p[bb] = p[bb] - w[bb] * correction;
                 }
             }
         }
     }
+}
+
+// The six tetrahedra of a cell held in registers, in Kuhn order. With FAST
+// the result stands where it returns true; else the cell is to be done over
+// without.
+template <bool FAST>
+__device__ __forceinline__ bool projectCell(V (&p)[8], const V (&prev)[8], const float (&w)[8], const CellConsts& k) {
+    const float s = k.restScale, ns = -s;
+    rounded::Ranges ranges;
+    projectTet<0, FAST>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, ranges);
+    projectTet<1, FAST>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, ranges);
+    projectTet<2, FAST>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, ranges);
+    projectTet<3, FAST>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, ranges);
+    projectTet<4, FAST>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, ranges);
+    projectTet<5, FAST>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, ranges);
+    return !FAST || ranges.hold();
 }
 
 // projectTet with the cell split over the four lanes of a quad (lanes
@@ -253,7 +300,7 @@ __device__ __forceinline__ void projectTetQuad(V (&p)[8], const V (&prev)[8], co
     p[i3] = from(3);
 }
 
-// solveCell<false> with the six tetrahedra split over a quad's lanes; the
+// projectCell with the six tetrahedra split over a quad's lanes; the
 // stretch sweeps that follow run in every lane on the same values.
 __device__ __forceinline__ void solveCellQuad(V (&p)[8], const V (&prev)[8], const float (&w)[8],
                                               const CellConsts& k, const StretchLengths& lens, uint32_t q,
@@ -265,7 +312,7 @@ __device__ __forceinline__ void solveCellQuad(V (&p)[8], const V (&prev)[8], con
     projectTetQuad<3>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, q, quad);
     projectTetQuad<4>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, q, quad);
     projectTetQuad<5>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, q, quad);
-    solveCell<true>(p, prev, w, k, lens);  // the stretch sweeps only
+    if (k.maxStretch > 1.0f) limitStretch(p, w, k, lens);
 }
 
 // The eight corner nodes of a cell entry (corner-0 node, body, y stride, z
@@ -436,11 +483,49 @@ __device__ __forceinline__ float4 predictNode(const FrameParams* fp, uint32_t n,
     return P;
 }
 
-// project.wgsl:35-184 on the cell `entry` (corner-0 node, body, y stride,
-// z stride): its eight corners gathered, solved, written back.
+// The six tetrahedra of cell `entry` with the IEEE operators throughout, from
+// its nodes as they stand in memory and back to them: the cells whose
+// operands leave rounded.cuh's ranges (collapsed or enormous elements). Out of
+// line, so that the common path keeps its registers.
+static __device__ __noinline__ void projectCellAgain(uint4 entry, const DevBody* body, float4* pos,
+                                                     const float4* prevState) {
+    uint32_t ids[8];
+    cornerNodes(entry, ids);
+    V p[8], prev[8];
+    float w[8];
+    for (int c = 0; c < 8; c++) {
+        const float4 P = pos[ids[c]];
+        p[c] = xyz(P);
+        w[c] = P.w;
+        prev[c] = xyz(prevState[ids[c]]);
+    }
+    projectCell<false>(p, prev, w, cellConsts(body));
+    for (int c = 0; c < 8; c++) pos[ids[c]] = withW(p[c], w[c]);
+}
+
+// project.wgsl:35-184 on the cell `entry` (corner-0 node, body, y stride, z
+// stride) of `body`, held in registers: the six tetrahedra (unless LIMIT_ONLY),
+// then, where the body limits its stretch, the length limit; written back.
 template <bool LIMIT_ONLY>
-__device__ __forceinline__ void solveCellAt(uint4 entry, const CellConsts& k, float4* pos, const float4* prevState,
-                                            const StretchLengths& lens) {
+__device__ __forceinline__ void solveCell(uint4 entry, const DevBody* body, V (&p)[8], const V (&prev)[8],
+                                          const float (&w)[8], const CellConsts& k, float4* pos,
+                                          const float4* prevState, const StretchLengths& lens) {
+    uint32_t ids[8];
+    cornerNodes(entry, ids);
+    if (!LIMIT_ONLY && !projectCell<true>(p, prev, w, k)) {
+        projectCellAgain(entry, body, pos, prevState);
+#pragma unroll
+        for (int c = 0; c < 8; c++) p[c] = xyz(pos[ids[c]]);
+    }
+    if (k.maxStretch > 1.0f) limitStretch(p, w, k, lens);
+#pragma unroll
+    for (int c = 0; c < 8; c++) pos[ids[c]] = withW(p[c], w[c]);
+}
+
+// solveCell on a cell gathered from memory.
+template <bool LIMIT_ONLY>
+__device__ __forceinline__ void solveCellAt(uint4 entry, const DevBody* body, const CellConsts& k, float4* pos,
+                                            const float4* prevState, const StretchLengths& lens) {
     uint32_t ids[8];
     cornerNodes(entry, ids);
     V p[8], prev[8];
@@ -453,9 +538,7 @@ __device__ __forceinline__ void solveCellAt(uint4 entry, const CellConsts& k, fl
     }
 #pragma unroll
     for (int c = 0; c < 8; c++) prev[c] = xyz(prevState[ids[c]]);
-    solveCell<LIMIT_ONLY>(p, prev, w, k, lens);
-#pragma unroll
-    for (int c = 0; c < 8; c++) pos[ids[c]] = withW(p[c], w[c]);
+    solveCell<LIMIT_ONLY>(entry, body, p, prev, w, k, pos, prevState, lens);
 }
 
 // finalize.wgsl:44-74 for node n (friction and velocity factor of its

@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(512) elasticKernel(const uint4* __restrict__ c
     forEachItemAfterWait(work, pre, [&](uint32_t, const Pre& q) {
         if (!q.live) return;
         if (LIMIT_ONLY && !(q.k.maxStretch > 1.0f)) return;
-        solveCellAt<LIMIT_ONLY>(q.entry, q.k, pos, prevState, lens);
+        solveCellAt<LIMIT_ONLY>(q.entry, bodies + q.entry.y, q.k, pos, prevState, lens);
     });
 }
 
@@ -127,7 +127,7 @@ __device__ __forceinline__ void copyAsync16(float4* dst, const float4* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
 }
 
-__global__ void __launch_bounds__(kStreamBlock) elasticStreamKernel(const uint4* __restrict__ cells, uint32_t count,
+__global__ void __launch_bounds__(kStreamBlock, kStreamBlocksPerSm) elasticStreamKernel(const uint4* __restrict__ cells, uint32_t count,
                                                                     const DevBody* __restrict__ bodies,
                                                                     const uint32_t* __restrict__ bodyActive,
                                                                     float4* __restrict__ pos,
@@ -180,11 +180,7 @@ __global__ void __launch_bounds__(kStreamBlock) elasticStreamKernel(const uint4*
             fetch(entry, zero);
         }
         if (bodyActive[cur.y]) {
-            solveCell<false>(p, prev, w, cellConsts(bodies + cur.y), lens);
-            uint32_t ids[8];
-            cornerNodes(cur, ids);
-#pragma unroll
-            for (int c = 0; c < 8; c++) pos[ids[c]] = withW(p[c], w[c]);
+            solveCell<false>(cur, bodies + cur.y, p, prev, w, cellConsts(bodies + cur.y), pos, prevState, lens);
         }
         if (next >= count) break;
         slot = next;
