@@ -1,0 +1,94 @@
+"""The row pass (two colours a launch, csrc/step_kernels.cu elasticRowKernel)
+against the oracle, bit for bit, at the sizes where its links, chains and
+groups end: one to a few cells, a chain that fills a warp and one past it, a
+chain that fills a group and one past it (which takes the colours one by
+one), rows with gaps, several bodies whose chains share groups, the stretch
+limit, and cells whose operands leave the branch-free arithmetic's ranges."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def lib(vsimlib, gpu):
+    return vsimlib
+
+
+def scene_of(rows, holes=0.0, seed=0, stretch=0.0):
+    import vsim.scenes as sc
+
+    rng = np.random.default_rng(seed)
+    bodies = []
+    for b, dims in enumerate(rows):
+        occ = (rng.random(dims[0] * dims[1] * dims[2]) >= holes).astype(np.uint8)
+        occ[0] = 1
+        mat = dict(sc.DEFAULT_MATERIAL, max_stretch=stretch)
+        bodies.append(sc.Body(tuple(dims), (0.0, 0.3 * b, 0.0), sc.H, occ, mat))
+    inf = float("inf")
+    return sc.Scene(bodies, ((-inf, -inf, -inf), (inf, inf, inf)), step_duration=1 / 600, substeps=3, contact=False)
+
+
+def run(scene, pos, frames=2):
+    import pyoracle
+    from vsim import Simulator
+
+    sim, orc = Simulator(scene), pyoracle.Oracle(scene, 32)
+    vel = np.zeros_like(pos)
+    sim.write_state(pos, pos, vel)
+    orc.set_state(pos, pos, vel)
+    for frame in range(frames):
+        sim.dispatch(scene.substeps)
+        orc.dispatch(scene.substeps)
+        for name, g, o in zip(("pos", "prev", "vel"), sim.read_state(), orc.state()):
+            bad = np.flatnonzero(np.any(g != o, axis=1))
+            assert bad.size == 0, f"frame {frame}: {name} differs at {bad.size} nodes, first {bad[:5]}"
+    launches = sim.frame_launches(1)
+    sim.destroy()
+    return launches
+
+
+def strained(scene, seed=5, amount=0.15):
+    import vsim.scenes as sc
+
+    rng = np.random.default_rng(seed)
+    rest = np.concatenate([sc.rest_positions(b) for b in scene.bodies]).astype(np.float64)
+    moved = rest + amount * sc.H * rng.standard_normal(rest.shape)
+    return np.concatenate([moved, np.zeros((len(rest), 1))], 1).astype(np.float32)
+
+
+@pytest.mark.parametrize("nx", [1, 2, 3, 4, 63, 64, 65, 66, 127, 255, 256, 257, 258])
+@pytest.mark.parametrize("holes", [0.0, 0.3])
+def test_row_lengths(lib, nx, holes):
+    scene = scene_of([(nx, 3, 2)], holes, seed=nx)
+    launches = run(scene, strained(scene))
+    if holes == 0.0:
+        # predict, finalize, and the passes that have cells: two links' parities
+        # (y) of z parity 0 and 1, or past a group's chain the colours
+        assert launches == 2 + (4 if nx <= 256 else 8)
+
+
+def test_bodies_share_groups(lib):
+    scene = scene_of([(5, 4, 3), (64, 2, 2), (1, 1, 1), (130, 3, 3), (17, 9, 4)], 0.2, seed=3)
+    run(scene, strained(scene))
+
+
+def test_stretch_limit(lib):
+    scene = scene_of([(70, 3, 3), (9, 5, 4)], 0.1, seed=4, stretch=1.08)
+    run(scene, strained(scene, amount=0.2))
+
+
+def test_operands_out_of_range(lib):
+    """Elements collapsed to a point, to a line and blown up far past the
+    ranges: those cells, even and odd, are done over with the IEEE operators."""
+    import vsim.scenes as sc
+
+    scene = scene_of([(70, 3, 3)], 0.0, seed=6)
+    pos = strained(scene)
+    nx, ny, nz = scene.bodies[0].node_dims
+    grid = pos.reshape(nz, ny, nx, 4)
+    grid[:, :, 4:7, :3] = grid[0, 0, 5, :3]            # an even and an odd cell, every node at one place
+    grid[:, :, 21:23, :3] = grid[0, 0, 21, :3]         # one odd cell
+    grid[:2, :2, 40:42, :3] *= np.float32(1e-12)       # tiny
+    grid[1:, 1:, 50:52, :3] += np.float32(3e4) * sc.H  # enormous
+    run(scene, pos, frames=1)

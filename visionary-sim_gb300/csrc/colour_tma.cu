@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(kTmaBlock) elasticTmaKernel(const __grid_const
                 prev[c] = xyz(Q[at[c]]);
             }
             const CellConsts k = cellConsts(bodies + e.x);
-            projectCell<false>(p, prev, w, k);
+            projectCell(p, prev, w, k);
             if (k.maxStretch > 1.0f) limitStretch(p, w, k, lens);
 #pragma unroll
             for (int c = 0; c < 8; c++) P[at[c]] = withW(p[c], w[c]);

@@ -20,6 +20,7 @@ struct DeviceState {
     uint32_t* bodyActive = nullptr;  // 1 where a body takes part in this frame
     float4* grabs = nullptr;      // per body: drive target, drive target velocity
     uint4* cells = nullptr;       // colour-major (corner-0 node, body, y stride, z stride)
+    uint4* rows = nullptr;        // the row passes' groups, pass by pass (kRowGroup entries each)
     DevBody* bodies = nullptr;
     FrameParams* fp = nullptr;
     // contact
@@ -173,6 +174,30 @@ cudaError_t launchPredict(const LaunchCtx& c, const DeviceState& s, const Span& 
 cudaError_t launchMarkDriven(cudaStream_t st, const uint32_t* driven, uint32_t n, int32_t* drivenOf, bool clear);
 cudaError_t launchElastic(const LaunchCtx& c, const DeviceState& s, const uint4* cells, const Span& span,
                           bool limitOnly, const StretchLengths& lens);
+
+// The row pass (elasticRowKernel): two colours in one launch. The cells of a
+// colour and of the next one differ in x parity only, so in a row of cells
+// along x they alternate, and rows of one y and z parity share no node. The
+// runs of occupied cells in those rows are packed into groups of at most
+// kRowBlock even and kRowBlock odd cells, a block each: it solves its even
+// cells, then its odd ones, and hands the nodes between them on in shared
+// memory. A run never straddles groups; a scene with a run that does not fit
+// one (over 256 cells in a line) takes the colours one by one.
+constexpr uint32_t kRowBlock = 128;
+constexpr uint32_t kRowPasses = 4;
+// A group's table: kRowBlock even cells, then kRowBlock odd cells, each (node
+// of corner 0, body and kRowCell, node stride along y and two 8-bit fields,
+// node stride along z). The fields of an even cell name the odd cells of its
+// group that hold its near and its far face, kNoRowCell for none.
+constexpr uint32_t kRowGroup = 2 * kRowBlock;
+constexpr uint32_t kRowCell = 1u << 31;  // the slot holds a cell
+constexpr uint32_t kNoRowCell = kRowBlock;
+constexpr uint32_t kRowStrideBits = 13;  // a body has at most 4097 nodes along x
+constexpr uint32_t rowFields(uint32_t stride, uint32_t nearOdd, uint32_t farOdd) {
+    return stride | nearOdd << kRowStrideBits | farOdd << (kRowStrideBits + 8);
+}
+cudaError_t launchElasticRows(const LaunchCtx& c, const DeviceState& s, const uint4* groups, uint32_t count,
+                              bool limitOnly, const StretchLengths& lens);
 
 // The streaming colour pass (elasticStreamKernel): blocks of kStreamBlock
 // threads, kStreamBlocksPerSm of them per SM (what the ~127 registers of a

@@ -148,17 +148,30 @@ int syncParams(vsim_sim* s) {
     return VSIM_OK;
 }
 
+// Where each colour's cells, and each body's inside them, start in the cell
+// list.
+void countCells(vsim_sim* s) {
+    uint32_t at = 0;
+    for (int c = 0; c < 8; c++) {
+        s->colorStart[c] = at;
+        s->colourBodyStart[c].assign(s->lat.size() + 1, 0);
+        for (size_t b = 0; b < s->lat.size(); b++) {
+            s->colourBodyStart[c][b] = at - s->colorStart[c];
+            at += uint32_t(s->lat[b].cellsByColor[c].size());
+        }
+        s->colourBodyStart[c][s->lat.size()] = at - s->colorStart[c];
+    }
+    s->colorStart[8] = at;
+}
+
 // The cell list, colour-major over bodies (elasticCells.js:143-163). Inside a
 // colour and body the cells run in lattice order, or brick by brick when
 // `brick` is 4 or 8 (bricks of that many cells per axis).
-void buildCells(vsim_sim* s, std::vector<uint4>& out) {
+void buildCells(const vsim_sim* s, std::vector<uint4>& out) {
     out.clear();
     out.reserve(s->cellCount);
-    for (int c = 0; c < 8; c++) {
-        s->colorStart[c] = uint32_t(out.size());
-        s->colourBodyStart[c].assign(s->lat.size() + 1, 0);
+    for (int c = 0; c < 8; c++)
         for (size_t b = 0; b < s->lat.size(); b++) {
-            s->colourBodyStart[c][b] = uint32_t(out.size()) - s->colorStart[c];
             const Lattice& L = s->lat[b];
             std::vector<uint32_t> order(L.cellsByColor[c]);
             if (s->brick > 1) {
@@ -179,9 +192,68 @@ void buildCells(vsim_sim* s, std::vector<uint4>& out) {
                                          L.nodeDims[0], L.nodeDims[0] * L.nodeDims[1]));
             }
         }
-        s->colourBodyStart[c][s->lat.size()] = uint32_t(out.size()) - s->colorStart[c];
+}
+
+// The cell list on the device, built when a path that reads it is first
+// chosen (the row passes do not). With `again` a list that is there is
+// rewritten.
+int uploadCells(vsim_sim* s, bool again) {
+    if (s->d.cells && !again) return VSIM_OK;
+    std::vector<uint4> cells;
+    buildCells(s, cells);
+    if (!s->d.cells) CK(allocN(&s->d.cells, s->cellCount), "allocate cells");
+    CK(cudaMemcpyAsync(s->d.cells, cells.data(), cells.size() * 16, cudaMemcpyHostToDevice, s->stream), "upload cells");
+    CK(cudaStreamSynchronize(s->stream), "upload cells");
+    return VSIM_OK;
+}
+
+// The row passes' groups (kRowBlock), pass by pass (y and z parity), bodies in
+// order and rows in lattice order inside each. False when some run of cells
+// does not fit a group.
+bool buildRows(vsim_sim* s, std::vector<uint4>& out) {
+    out.clear();
+    out.reserve(size_t(s->cellCount) * 5 / 4 + kRowPasses * kRowGroup);
+    for (uint32_t pass = 0; pass < kRowPasses; pass++) {
+        s->rowStart[pass] = uint32_t(out.size() / kRowGroup);
+        uint32_t evens = kRowBlock, odds = kRowBlock;  // cells in the open group; full: none open
+        for (size_t b = 0; b < s->lat.size(); b++) {
+            const Lattice& L = s->lat[b];
+            const uint32_t nx = L.nodeDims[0], nxy = nx * L.nodeDims[1], cx = L.cellDims[0];
+            for (uint32_t k = pass >> 1; k < L.cellDims[2]; k += 2)
+                for (uint32_t j = pass & 1; j < L.cellDims[1]; j += 2) {
+                    const uint8_t* row = L.occupancy.data() + size_t(cx) * (j + size_t(L.cellDims[1]) * k);
+                    const uint32_t n0 = s->offsets[b] + nx * j + nxy * k;
+                    for (uint32_t i = 0; i < cx;) {
+                        if (!row[i]) {
+                            i++;
+                            continue;
+                        }
+                        uint32_t end = i + 1;  // the run is [i, end)
+                        while (end < cx && row[end]) end++;
+                        const uint32_t runEvens = (end + 1) / 2 - (i + 1) / 2, runOdds = end / 2 - i / 2;
+                        if (runEvens > kRowBlock || runOdds > kRowBlock) return false;
+                        if (evens + runEvens > kRowBlock || odds + runOdds > kRowBlock) {
+                            out.resize(out.size() + kRowGroup, make_uint4(0, 0, 0, 0));
+                            evens = odds = 0;
+                        }
+                        uint4* group = out.data() + out.size() - kRowGroup;
+                        const uint32_t first = i;
+                        for (; i < end; i++) {
+                            const uint32_t who = uint32_t(b) | kRowCell;
+                            if (i & 1)
+                                group[kRowBlock + odds++] = make_uint4(n0 + i, who, nx, nxy);
+                            else
+                                group[evens++] = make_uint4(n0 + i, who,
+                                                            rowFields(nx, i > first ? odds - 1 : kNoRowCell,
+                                                                      i + 1 < end ? odds : kNoRowCell),
+                                                            nxy);
+                        }
+                    }
+                }
+        }
     }
-    s->colorStart[8] = uint32_t(out.size());
+    s->rowStart[kRowPasses] = uint32_t(out.size() / kRowGroup);
+    return true;
 }
 
 // Spans over every body.
@@ -275,6 +347,30 @@ cudaError_t launchColourPass(const LaunchCtx& c, const vsim_sim* s, int col, boo
     return launchElastic(c, s->d, s->d.cells + s->colorStart[col], sp, limitOnly, lens);
 }
 
+// Whether the frame's elastic passes run as row passes (two colours each).
+bool inRows(const vsim_sim* s) { return s->rowPasses && !s->plan.chunked && !s->tma.enabled && !s->quadCells; }
+
+// One sweep over the eight colours, as four row passes or eight colour
+// passes; each(launch) is called for every pass that has cells.
+template <class Each>
+cudaError_t forEachPass(const LaunchCtx& c, const vsim_sim* s, bool limitOnly, const StretchLengths& lens, Each&& each) {
+    cudaError_t e = cudaSuccess;
+    if (inRows(s)) {
+        for (uint32_t q = 0; q < kRowPasses && !e; q++) {
+            const uint32_t groups = s->rowStart[q + 1] - s->rowStart[q];
+            if (groups)
+                e = each([&] {
+                    return launchElasticRows(c, s->d, s->d.rows + size_t(s->rowStart[q]) * kRowGroup, groups, limitOnly,
+                                             lens);
+                });
+        }
+        return e;
+    }
+    for (int col = 0; col < 8 && !e; col++)
+        if (s->plan.colour[col].grid) e = each([&] { return launchColourPass(c, s, col, limitOnly, lens); });
+    return e;
+}
+
 // stepper.js:101-108 with simulator.js:83's constraint order.
 cudaError_t encodeFrame(vsim_sim* s, cudaStream_t st, uint32_t steps, ContactMode mode = ContactMode::Solve,
                         Profiler* prof = nullptr) {
@@ -301,21 +397,18 @@ cudaError_t encodeFrame(vsim_sim* s, cudaStream_t st, uint32_t steps, ContactMod
         end();
     }
     for (uint32_t step = 0; step < steps; step++) {
-        for (uint32_t it = 0; it < s->iterations; it++)
-            for (int col = 0; col < 8; col++) {
-                if (!plan.colour[col].grid) continue;
-                begin(VSIM_KIND_ELASTIC, 1);
-                if ((e = launchColourPass(c, s, col, false, lens))) return e;
+        auto sweep = [&](bool limitOnly) {
+            return forEachPass(c, s, limitOnly, lens, [&](auto launch) {
+                begin(limitOnly ? VSIM_KIND_LIMIT : VSIM_KIND_ELASTIC, 1);
+                const cudaError_t failed = launch();
                 end();
-            }
-        if (limited)
-            for (int sweep = 0; sweep < 3; sweep++)
-                for (int col = 0; col < 8; col++) {
-                    if (!plan.colour[col].grid) continue;
-                    begin(VSIM_KIND_LIMIT, 1);
-                    if ((e = launchColourPass(c, s, col, true, lens))) return e;
-                    end();
-                }
+                return failed;
+            });
+        };
+        for (uint32_t it = 0; it < s->iterations; it++)
+            if ((e = sweep(false))) return e;
+        for (int q = 0; limited && q < 3; q++)
+            if ((e = sweep(true))) return e;
         if (contact && plan.records.grid) {
             begin(VSIM_KIND_CONTACT, kContactKernels);
             if ((e = launchContact(c, s->d, plan.records, s->surfaceCount, s->gatherMapping, mode, nullptr, 0, nullptr))) return e;
@@ -342,6 +435,7 @@ uint64_t graphKey(const vsim_sim* s, uint32_t steps) {
     k = k * 31 + uint64_t(s->gatherMapping);
     k = k * 31 + (s->tma.enabled ? 1 : 0);
     k = k * 31 + (s->quadCells ? 1 : 0);
+    k = k * 31 + (inRows(s) ? 1 : 0);
     k = k * 131 + s->plan.records.gatherPerSm;
     return k;
 }
@@ -407,7 +501,7 @@ void freeSim(vsim_sim* s) {
     DeviceState& d = s->d;
     void* ptrs[] = {d.pos, d.prev, d.vel, d.baseW, d.active, d.activeBody, d.cells, d.bodies, d.fp,
                     d.surf, d.key, d.rank, d.entries, d.count, d.start, d.cursor, d.delta, d.driven,
-                    d.drivenOffset, d.drivenOf, d.nodeRecord, d.sMeta, d.sPos, d.sMoved, d.sRec, d.sKey, d.bodyActive, d.grabs,
+                    d.drivenOffset, d.drivenOf, d.rows, d.nodeRecord, d.sMeta, d.sPos, d.sMoved, d.sRec, d.sKey, d.bodyActive, d.grabs,
                     s->chunkDev, s->staging, s->pairs, s->pairCount, s->sp.embed, s->sp.quat,
                     s->sp.scaleBody, s->sp.bodies, s->sp.meanDepth, s->sp.cov, s->sp.keys, s->sp.order,
                     s->sp.sortTemp};
@@ -571,7 +665,6 @@ int createSim(const vsim_body_desc* bodies, uint32_t n, const vsim_tank* tank, v
     CK(allocN(&d.baseW, N), "allocate masses");
     CK(allocN(&d.active, s->activeCount), "allocate active list");
     CK(allocN(&d.activeBody, s->activeCount), "allocate active list");
-    CK(allocN(&d.cells, s->cellCount), "allocate cells");
     CK(allocN(&d.bodies, n), "allocate body constants");
     CK(allocN(&d.fp, 1), "allocate frame parameters");
     CK(allocN(&d.surf, s->surfaceCount), "allocate surface");
@@ -609,10 +702,18 @@ int createSim(const vsim_body_desc* bodies, uint32_t n, const vsim_tank* tank, v
             s->restPos[4 * node + 3] = s->baseW[node];
         }
     }
-    std::vector<uint4> cells;
-    buildCells(s, cells);
+    std::vector<uint4> rows;
+    countCells(s);
     buildDensePlan(s);
     useDensePlan(s);
+    // Isolated bodies step in chunked frames, which take the colours one by one.
+    if (!isolated && buildRows(s, rows)) {
+        s->rowPasses = true;
+        CK(allocN(&d.rows, rows.size()), "allocate rows");
+        CK(cudaMemcpyAsync(d.rows, rows.data(), rows.size() * 16, cudaMemcpyHostToDevice, s->stream), "upload rows");
+    } else if (int rc = uploadCells(s, false)) {
+        return rc;
+    }
     if (isolated) {
         // Room for a chunk table over every body at once, and the spans
         // over it: blocks of kChunk threads, as many as fill the device
@@ -648,7 +749,6 @@ int createSim(const vsim_body_desc* bodies, uint32_t n, const vsim_tank* tank, v
     CK(cudaMemcpyAsync(d.active, active.data(), active.size() * 4, cudaMemcpyHostToDevice, s->stream), "upload");
     CK(cudaMemcpyAsync(d.activeBody, activeBody.data(), activeBody.size() * 4, cudaMemcpyHostToDevice, s->stream),
        "upload");
-    CK(cudaMemcpyAsync(d.cells, cells.data(), cells.size() * 16, cudaMemcpyHostToDevice, s->stream), "upload cells");
     CK(cudaMemcpyAsync(d.surf, s->surfHost.data(), s->surfHost.size() * 16, cudaMemcpyHostToDevice, s->stream),
        "upload surface");
     CK(cudaMemsetAsync(d.count, 0, s->bucketTotal * 4, s->stream), "clear grid");
@@ -728,6 +828,8 @@ int vsim_synchronize(vsim_sim* s) {
 int vsim_set_cell_lanes(vsim_sim* s, uint32_t lanes) {
     SIM_GUARD(s);
     if (lanes != 1 && lanes != 4) return fail(VSIM_ERR_RANGE, "lanes must be 1 or 4");
+    if (lanes == 4)
+        if (int rc = uploadCells(s, false)) return rc;
     s->quadCells = lanes == 4;
     return VSIM_OK;
 }
@@ -738,6 +840,8 @@ int vsim_set_tma_pass(vsim_sim* s, int enabled) {
         if (int rc = buildTmaPass(s)) return rc;
         if (!s->tma.ready) return fail(VSIM_ERR_RANGE, "the TMA colour pass takes 1 to 4 bodies");
     }
+    if (enabled)
+        if (int rc = uploadCells(s, false)) return rc;
     s->tma.enabled = enabled != 0;
     return VSIM_OK;
 }
@@ -1036,11 +1140,8 @@ int vsim_set_launch_shape(vsim_sim* s, uint32_t block, uint32_t brick) {
     s->block = block;
     if (brick != s->brick) {
         s->brick = brick;
-        std::vector<uint4> cells;
-        buildCells(s, cells);
-        CK(cudaMemcpyAsync(s->d.cells, cells.data(), cells.size() * 16, cudaMemcpyHostToDevice, s->stream),
-           "upload cells");
-        CK(cudaStreamSynchronize(s->stream), "upload cells");
+        if (s->d.cells)
+            if (int rc = uploadCells(s, true)) return rc;
     }
     buildDensePlan(s);
     if (!s->plan.chunked) useDensePlan(s);
@@ -1260,10 +1361,13 @@ int vsim_color_counts(const vsim_sim* s, uint32_t out[8]) {
 
 uint32_t vsim_frame_launches(const vsim_sim* s, uint32_t steps) {
     if (!s) return 0;
-    uint32_t colours = 0;
-    for (int c = 0; c < 8; c++) colours += s->colorStart[c + 1] > s->colorStart[c] ? 1 : 0;
-    uint32_t per = 1 + colours * s->iterations;
-    if (anyStretch(s)) per += 3 * colours;
+    uint32_t passes = 0;
+    if (inRows(s))
+        for (uint32_t q = 0; q < kRowPasses; q++) passes += s->rowStart[q + 1] > s->rowStart[q] ? 1 : 0;
+    else
+        for (int c = 0; c < 8; c++) passes += s->colorStart[c + 1] > s->colorStart[c] ? 1 : 0;
+    uint32_t per = 1 + passes * s->iterations;
+    if (anyStretch(s)) per += 3 * passes;
     if (s->contact && s->surfaceCount > 0) per += kContactKernels;
     return steps ? 1 + per * steps : 0;
 }
@@ -1296,8 +1400,7 @@ int vsim_time_colour_passes(vsim_sim* s, uint32_t sweeps, float* ms) {
         if ((e = cudaStreamBeginCapture(s->capture, cudaStreamCaptureModeThreadLocal))) return e;
         cudaError_t enc = cudaSuccess;
         for (uint32_t sweep = 0; sweep < sweeps && enc == cudaSuccess; sweep++)
-            for (int col = 0; col < 8 && enc == cudaSuccess; col++)
-                if (s->plan.colour[col].grid) enc = launchColourPass(c, s, col, false, lens);
+            enc = forEachPass(c, s, false, lens, [](auto launch) { return launch(); });
         const cudaError_t end = cudaStreamEndCapture(s->capture, &graph);
         if (enc) return enc;
         if (end) return end;

@@ -72,6 +72,8 @@ struct vsim_sim {
     std::vector<float> restPos;  // xyzw per node, w = baseW
     uint32_t nodeCount = 0, activeCount = 0, cellCount = 0, surfaceCount = 0;
     uint32_t colorStart[9] = {};
+    bool rowPasses = false;  // the row passes' groups are built (every run of cells fits one)
+    uint32_t rowStart[vsim::kRowPasses + 1] = {};  // first group of each row pass
     std::vector<uint4> surfHost;
     vsim_tank tank{};
     // Contact grids: one shared by all bodies, or one per body when the

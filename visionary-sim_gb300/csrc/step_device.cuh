@@ -59,15 +59,15 @@ __device__ __forceinline__ float kscale(float s, float ns) {
     return K > 0 ? s : ns;
 }
 
-template <int K0, int K1, int K2>
-__device__ __forceinline__ V sparse3(V a0, V a1, V a2, float s, float ns) {
+template <int K0, int K1, int K2, class Vec>
+__device__ __forceinline__ Vec sparse3(Vec a0, Vec a1, Vec a2, float s, float ns) {
     if constexpr (K0 != 0) {
-        V acc = a0 * kscale<K0>(s, ns);
+        Vec acc = a0 * kscale<K0>(s, ns);
         if constexpr (K1 != 0) acc = fma3(a1, kscale<K1>(s, ns), acc);
         if constexpr (K2 != 0) acc = fma3(a2, kscale<K2>(s, ns), acc);
         return acc;
     } else if constexpr (K1 != 0) {
-        V acc = a1 * kscale<K1>(s, ns);
+        Vec acc = a1 * kscale<K1>(s, ns);
         if constexpr (K2 != 0) acc = fma3(a2, kscale<K2>(s, ns), acc);
         return acc;
     } else {
@@ -127,33 +127,19 @@ __device__ __forceinline__ V moved(V p, V d, V h, float lx, float ly, float w) {
     return fma3(fma3(h, ly, d * lx), w, p);
 }
 
-// project.wgsl:75-153, tetrahedron t of the cell held in registers. With FAST
-// the norm's root and reciprocal and the 2x2 solve's two quotients are
-// rounded.cuh's, whose results are the IEEE operators' where `ranges` holds
-// at the end, and nothing branches, so the compiler schedules across the
-// cell's six tetrahedra: 2,650 cycles a cell against 4,250 with the IEEE
-// operators (one warp, everything in registers). The reference's two early
-// outs need no branch there: a weightless tetrahedron moves nothing, and a
-// determinant under 1e-20 is outside the ranges.
-template <int t, bool FAST>
+// project.wgsl:75-153, tetrahedron t of the cell held in registers, with the
+// IEEE operators.
+template <int t>
 __device__ __forceinline__ void projectTet(V (&p)[8], const V (&prev)[8], const float (&w)[8], float s, float ns,
-                                           float alphaDev, float alphaHyd, float gamma, float relax,
-                                           rounded::Ranges& ranges) {
+                                           float alphaDev, float alphaHyd, float gamma, float relax) {
     constexpr int i0 = kTet(t, 0), i1 = kTet(t, 1), i2 = kTet(t, 2), i3 = kTet(t, 3);
     const float w0 = w[i0], w1 = w[i1], w2 = w[i2], w3 = w[i3];
-    if (!FAST && w0 + w1 + w2 + w3 == 0.0f) return;
+    if (w0 + w1 + w2 + w3 == 0.0f) return;
     const V base = p[i0];
     const M F = timesB<t>(M{{p[i1] - base, p[i2] - base, p[i3] - base}}, s, ns);
-    const float square = dot(F.c[0], F.c[0]) + dot(F.c[1], F.c[1]) + dot(F.c[2], F.c[2]);
-    float cDev, inv;
-    if (FAST) {
-        rounded::rootAndReciprocal(square, cDev, inv);
-        ranges.reciprocalOfRoot(inv);
-    } else {
-        cDev = sqrtf(square);
-        inv = cDev > 1e-9f ? 1.0f / cDev : 0.0f;
-    }
+    const float cDev = sqrtf(dot(F.c[0], F.c[0]) + dot(F.c[1], F.c[1]) + dot(F.c[2], F.c[2]));
     const float cHyd = determinant(F) - gamma;
+    const float inv = cDev > 1e-9f ? 1.0f / cDev : 0.0f;
     const M mDev = timesBt<t>(F * inv, s, ns);
     const M mHyd = timesBt<t>(M{{cross(F.c[1], F.c[2]), cross(F.c[2], F.c[0]), cross(F.c[0], F.c[1])}}, s, ns);
     const V d1 = mDev.c[0], d2 = mDev.c[1], d3 = mDev.c[2];
@@ -169,22 +155,96 @@ __device__ __forceinline__ void projectTet(V (&p)[8], const V (&prev)[8], const 
     const V x3 = p[i3] - prev[i3];
     const float rx = dot(d0, x0) + dot(d1, x1) + dot(d2, x2) + dot(d3, x3);
     const float ry = dot(h0, x0) + dot(h1, x1) + dot(h2, x2) + dot(h3, x3);
-    const Couple2 k = couple2(cDev, cHyd, alphaDev, alphaHyd, relax, rx, ry, gx, gy, gz);
     float lx, ly;
-    if (FAST) {
-        const float r = rounded::reciprocal(k.det, rounded::approxReciprocal(k.det));
-        lx = rounded::quotient(k.nx, k.det, r);
-        ly = rounded::quotient(k.ny, k.det, r);
-        ranges.arguments(square, k.det);
-        ranges.quotients(lx, ly);
-    } else {
-        lx = k.det < 1e-20f ? 0.0f : k.nx / k.det;
-        ly = k.det < 1e-20f ? 0.0f : k.ny / k.det;
-    }
+    couple(cDev, cHyd, alphaDev, alphaHyd, relax, rx, ry, gx, gy, gz, lx, ly);
     p[i0] = moved(p[i0], d0, h0, lx, ly, w0);
     p[i1] = moved(p[i1], d1, h1, lx, ly, w1);
     p[i2] = moved(p[i2], d2, h2, lx, ly, w2);
     p[i3] = moved(p[i3], d3, h3, lx, ly, w3);
+}
+
+// The deviatoric and the hydrostatic gradient of a corner, side by side: a
+// lane each of packed FP32x2 products and fused sums. (Plain sums are taken
+// lane by lane: see fma3.)
+struct Pair3 {
+    float2 x, y, z;
+    __device__ __forceinline__ V dev() const { return mk(x.x, y.x, z.x); }
+    __device__ __forceinline__ V hyd() const { return mk(x.y, y.y, z.y); }
+};
+__device__ __forceinline__ Pair3 pairOf(V d, V h) {
+    return Pair3{make_float2(d.x, h.x), make_float2(d.y, h.y), make_float2(d.z, h.z)};
+}
+__device__ __forceinline__ Pair3 operator*(Pair3 a, float s) {
+    const float2 q = make_float2(s, s);
+    return Pair3{__fmul2_rn(a.x, q), __fmul2_rn(a.y, q), __fmul2_rn(a.z, q)};
+}
+__device__ __forceinline__ Pair3 fma3(Pair3 a, float s, Pair3 acc) {
+    const float2 q = make_float2(s, s);
+    return Pair3{__ffma2_rn(a.x, q, acc.x), __ffma2_rn(a.y, q, acc.y), __ffma2_rn(a.z, q, acc.z)};
+}
+// (dev . dev, hyd . hyd)
+__device__ __forceinline__ float2 squares(Pair3 a) {
+    return __ffma2_rn(a.z, a.z, __ffma2_rn(a.y, a.y, __fmul2_rn(a.x, a.x)));
+}
+__device__ __forceinline__ float2 weighted4(float w0, float w1, float w2, float w3, float2 e0, float2 e1, float2 e2,
+                                            float2 e3) {
+    return __ffma2_rn(make_float2(w3, w3), e3,
+                      __ffma2_rn(make_float2(w2, w2), e2,
+                                 __ffma2_rn(make_float2(w1, w1), e1, __fmul2_rn(make_float2(w0, w0), e0))));
+}
+
+// projectTet for operands in rounded.cuh's ranges: the same values as long as
+// `ranges` holds at the end. The norm's root and reciprocal and the 2x2
+// solve's two quotients are rounded.cuh's and nothing branches, so the
+// compiler schedules across the cell's six tetrahedra: 2,580 cycles a cell
+// (one warp, operands in registers) against 4,250 with the IEEE operators.
+// The two gradients are packed, for the code's size: 25 KB a cell against 28
+// KB, where an SM's instruction cache holds about 32 KB and code over it, run
+// again and again, misses on every line (two inlined projections in a loop:
+// 4,340 cycles each). The reference's two
+// early outs need no branch: a weightless tetrahedron moves nothing, and a
+// determinant under 1e-20 is outside the ranges. Corner 0's gradients are
+// minus the sum of the others'; the sum is kept and the sign moved to where
+// it is used, which rounds the same.
+template <int t, class Prev>
+__device__ __forceinline__ void projectTetInRange(V (&p)[8], Prev&& prev, const float (&w)[8], float s, float ns,
+                                                  float alphaDev, float alphaHyd, float gamma, float relax,
+                                                  rounded::Ranges& ranges) {
+    constexpr int i0 = kTet(t, 0), i1 = kTet(t, 1), i2 = kTet(t, 2), i3 = kTet(t, 3);
+    const float w0 = w[i0], w1 = w[i1], w2 = w[i2], w3 = w[i3];
+    const V base = p[i0];
+    const M F = timesB<t>(M{{difference(p[i1], base), difference(p[i2], base), difference(p[i3], base)}}, s, ns);
+    const float square = dot(F.c[0], F.c[0]) + dot(F.c[1], F.c[1]) + dot(F.c[2], F.c[2]);
+    float cDev, inv;
+    rounded::rootAndReciprocal(square, cDev, inv);
+    ranges.reciprocalOfRoot(inv);
+    const float cHyd = determinant(F) - gamma;
+    const Pair3 a0 = pairOf(F.c[0] * inv, cross(F.c[1], F.c[2]));
+    const Pair3 a1 = pairOf(F.c[1] * inv, cross(F.c[2], F.c[0]));
+    const Pair3 a2 = pairOf(F.c[2] * inv, cross(F.c[0], F.c[1]));
+    const Pair3 g1 = sparse3<kKuhn.v[t][0][0], kKuhn.v[t][1][0], kKuhn.v[t][2][0]>(a0, a1, a2, s, ns);
+    const Pair3 g2 = sparse3<kKuhn.v[t][0][1], kKuhn.v[t][1][1], kKuhn.v[t][2][1]>(a0, a1, a2, s, ns);
+    const Pair3 g3 = sparse3<kKuhn.v[t][0][2], kKuhn.v[t][1][2], kKuhn.v[t][2][2]>(a0, a1, a2, s, ns);
+    const Pair3 minus0 = pairOf(g1.dev() + g2.dev() + g3.dev(), g1.hyd() + g2.hyd() + g3.hyd());
+    const float2 gxz = weighted4(w0, w1, w2, w3, squares(minus0), squares(g1), squares(g2), squares(g3));
+    const float gy = weighted4(w0, w1, w2, w3, dot(minus0.dev(), minus0.hyd()), dot(g1.dev(), g1.hyd()),
+                               dot(g2.dev(), g2.hyd()), dot(g3.dev(), g3.hyd()));
+    const V x0 = difference(p[i0], prev(i0));
+    const V x1 = difference(p[i1], prev(i1));
+    const V x2 = difference(p[i2], prev(i2));
+    const V x3 = difference(p[i3], prev(i3));
+    const float rx = -dot(minus0.dev(), x0) + dot(g1.dev(), x1) + dot(g2.dev(), x2) + dot(g3.dev(), x3);
+    const float ry = -dot(minus0.hyd(), x0) + dot(g1.hyd(), x1) + dot(g2.hyd(), x2) + dot(g3.hyd(), x3);
+    const Couple2 k = couple2(cDev, cHyd, alphaDev, alphaHyd, relax, rx, ry, gxz.x, gy, gxz.y);
+    const float r = rounded::reciprocal(k.det, rounded::approxReciprocal(k.det));
+    const float lx = rounded::quotient(k.nx, k.det, r);
+    const float ly = rounded::quotient(k.ny, k.det, r);
+    ranges.arguments(square, k.det);
+    ranges.quotients(lx, ly);
+    p[i0] = moved(p[i0], minus0.dev(), minus0.hyd(), lx, ly, -w0);
+    p[i1] = moved(p[i1], g1.dev(), g1.hyd(), lx, ly, w1);
+    p[i2] = moved(p[i2], g2.dev(), g2.hyd(), lx, ly, w2);
+    p[i3] = moved(p[i3], g3.dev(), g3.hyd(), lx, ly, w3);
 }
 
 // The constants of a cell's body that project.wgsl:64-73 derives.
@@ -210,6 +270,17 @@ __device__ __forceinline__ void limitStretch(V (&p)[8], const float (&w)[8], con
         clear[d] = maximum[d] >= 0x1p-50f && maximum[d] <= 0x1p50f ? maximum[d] * maximum[d] * (1.0f - 0x1p-20f)
                                                                    : -1.0f;
     }
+    // Where no pair is past its limit, neither sweep moves anything: found
+    // without a branch per pair.
+    bool any = false;
+#pragma unroll
+    for (int a = 0; a < 8; a++)
+#pragma unroll
+        for (int bb = a + 1; bb < 8; bb++) {
+            const V delta = p[bb] - p[a];
+            any = any || dot(delta, delta) > clear[__popc(a ^ bb) - 1];
+        }
+    if (!any) return;
     for (int sweep = 0; sweep < 2; sweep++) {
 #pragma unroll
         for (int a = 0; a < 8; a++) {
@@ -231,20 +302,31 @@ __device__ __forceinline__ void limitStretch(V (&p)[8], const float (&w)[8], con
     }
 }
 
-// The six tetrahedra of a cell held in registers, in Kuhn order. With FAST
-// the result stands where it returns true; else the cell is to be done over
-// without.
-template <bool FAST>
-__device__ __forceinline__ bool projectCell(V (&p)[8], const V (&prev)[8], const float (&w)[8], const CellConsts& k) {
+// The six tetrahedra of a cell held in registers, in Kuhn order.
+__device__ __forceinline__ void projectCell(V (&p)[8], const V (&prev)[8], const float (&w)[8], const CellConsts& k) {
+    const float s = k.restScale, ns = -s;
+    projectTet<0>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax);
+    projectTet<1>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax);
+    projectTet<2>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax);
+    projectTet<3>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax);
+    projectTet<4>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax);
+    projectTet<5>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax);
+}
+
+// projectCell by projectTetInRange; false where an operand left the ranges, and
+// the cell is to be done over by projectCell. prev(c): corner c's previous
+// position.
+template <class Prev>
+__device__ __forceinline__ bool projectCellInRange(V (&p)[8], Prev&& prev, const float (&w)[8], const CellConsts& k) {
     const float s = k.restScale, ns = -s;
     rounded::Ranges ranges;
-    projectTet<0, FAST>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, ranges);
-    projectTet<1, FAST>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, ranges);
-    projectTet<2, FAST>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, ranges);
-    projectTet<3, FAST>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, ranges);
-    projectTet<4, FAST>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, ranges);
-    projectTet<5, FAST>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, ranges);
-    return !FAST || ranges.hold();
+    projectTetInRange<0>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, ranges);
+    projectTetInRange<1>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, ranges);
+    projectTetInRange<2>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, ranges);
+    projectTetInRange<3>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, ranges);
+    projectTetInRange<4>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, ranges);
+    projectTetInRange<5>(p, prev, w, s, ns, k.alphaDev, k.alphaHyd, k.gamma, k.relax, ranges);
+    return ranges.hold();
 }
 
 // projectTet with the cell split over the four lanes of a quad (lanes
@@ -499,7 +581,7 @@ static __device__ __noinline__ void projectCellAgain(uint4 entry, const DevBody*
         w[c] = P.w;
         prev[c] = xyz(prevState[ids[c]]);
     }
-    projectCell<false>(p, prev, w, cellConsts(body));
+    projectCell(p, prev, w, cellConsts(body));
     for (int c = 0; c < 8; c++) pos[ids[c]] = withW(p[c], w[c]);
 }
 
@@ -512,7 +594,7 @@ __device__ __forceinline__ void solveCell(uint4 entry, const DevBody* body, V (&
                                           const float4* prevState, const StretchLengths& lens) {
     uint32_t ids[8];
     cornerNodes(entry, ids);
-    if (!LIMIT_ONLY && !projectCell<true>(p, prev, w, k)) {
+    if (!LIMIT_ONLY && !projectCellInRange(p, [&](int c) { return prev[c]; }, w, k)) {
         projectCellAgain(entry, body, pos, prevState);
 #pragma unroll
         for (int c = 0; c < 8; c++) p[c] = xyz(pos[ids[c]]);

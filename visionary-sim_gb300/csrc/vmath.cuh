@@ -23,17 +23,21 @@ struct V {
 __device__ __forceinline__ V mk(float x, float y, float z) { return V{x, y, z}; }
 __device__ __forceinline__ V xyz(float4 a) { return V{a.x, a.y, a.z}; }
 
-// fma3 issues x and y as one packed FP32x2 fused multiply-add (sm_100 and
-// later), which rounds each lane to nearest exactly as fmaf does. Adds,
-// subtractions and multiplies stay scalar: their packed forms round each
-// lane exactly as the scalar operations do (checked bit for bit on the GPU,
-// subnormal and signed-zero operands included), but using them made the
-// compiler keep the colour pass's cell in local memory (a 144-byte stack
-// frame in every colour-pass kernel).
+// fma3 and difference issue x and y as one packed FP32x2 operation (sm_100
+// and later), which rounds each lane to nearest exactly as the scalar one
+// does. The rate is the scalar one's, but the code is shorter. The other
+// operations stay scalar: the compiler joins a packed multiply and a packed
+// add of its result into one fused operation even with -fmad=false and with
+// the rounding spelled out in PTX (checked on the GPU: v + g * dt differs in
+// half of random cases), so a packed sum must never have a packed product
+// for an operand. difference is for operands that are none.
 __device__ __forceinline__ float2 xyOf(V a) { return make_float2(a.x, a.y); }
 __device__ __forceinline__ V withXy(float2 xy, float z) { return V{xy.x, xy.y, z}; }
 __device__ __forceinline__ V operator+(V a, V b) { return V{a.x + b.x, a.y + b.y, a.z + b.z}; }
 __device__ __forceinline__ V operator-(V a, V b) { return V{a.x - b.x, a.y - b.y, a.z - b.z}; }
+__device__ __forceinline__ V difference(V a, V b) {
+    return withXy(__fadd2_rn(xyOf(a), make_float2(-b.x, -b.y)), a.z - b.z);
+}
 __device__ __forceinline__ V operator-(V a) { return V{-a.x, -a.y, -a.z}; }
 __device__ __forceinline__ V operator*(V a, float s) { return V{a.x * s, a.y * s, a.z * s}; }
 __device__ __forceinline__ V operator*(float s, V a) { return V{s * a.x, s * a.y, s * a.z}; }
