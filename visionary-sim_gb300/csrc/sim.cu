@@ -356,12 +356,12 @@ template <class Each>
 cudaError_t forEachPass(const LaunchCtx& c, const vsim_sim* s, bool limitOnly, const StretchLengths& lens, Each&& each) {
     cudaError_t e = cudaSuccess;
     if (inRows(s)) {
+        const RowWork work = limitOnly ? RowWork::kLimit : anyStretch(s) ? RowWork::kBoth : RowWork::kProject;
         for (uint32_t q = 0; q < kRowPasses && !e; q++) {
             const uint32_t groups = s->rowStart[q + 1] - s->rowStart[q];
             if (groups)
                 e = each([&] {
-                    return launchElasticRows(c, s->d, s->d.rows + size_t(s->rowStart[q]) * kRowGroup, groups, limitOnly,
-                                             lens);
+                    return launchElasticRows(c, s->d, s->d.rows + size_t(s->rowStart[q]) * kRowGroup, groups, work, lens);
                 });
         }
         return e;

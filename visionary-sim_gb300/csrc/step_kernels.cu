@@ -147,14 +147,17 @@ __device__ __forceinline__ V sharedXyz(const float4* record) {
 // 256 boxes (1.3M cells) 18.4 -> 13.7, a 161x150x157 blob and sheet 20.7 ->
 // 18.0.
 //
-// EARLY (many waves) lets the next kernel launch at once, so that its blocks
+// WORK: the projection of scenes in which no body limits its stretch, the
+// projection with the limit, or a limit-only sweep. (The limit's code in the
+// common pass costs it registers: 256 boxes 13.7 us a colour without, 15.0
+// with.) EARLY (many waves) lets the next kernel launch at once, so that its blocks
 // fill the SMs this pass's last wave leaves idle, and holds the registers to
 // three blocks an SM (batch and large blob with two blocks: 15.6 and 20.4 us;
 // with four, which spill: 15.5 and 19.9). Otherwise a block that becomes
 // resident beside one in mid-flight holds it up by ~1,500 cycles (3.6 against
 // 2.8 us a colour on the 64^3 blob), more than the launch it hides: the next
 // kernel may launch once the arithmetic is done.
-template <bool LIMIT_ONLY, bool EARLY>
+template <RowWork WORK, bool EARLY>
 __global__ void __launch_bounds__(kRowBlock, EARLY ? 3 : 2) elasticRowKernel(const uint4* __restrict__ groups,
                                                                              const DevBody* __restrict__ bodies,
                                                                              const uint32_t* __restrict__ bodyActive,
@@ -167,7 +170,7 @@ __global__ void __launch_bounds__(kRowBlock, EARLY ? 3 : 2) elasticRowKernel(con
     const uint4* group = groups + size_t(blockIdx.x) * kRowGroup;
     const uint4 even = group[t], odd = group[kRowBlock + t];
     auto takesPart = [&](uint4 e, float maxStretch) {
-        return (e.y & kRowCell) && bodyActive[e.y & ~kRowCell] && (!LIMIT_ONLY || maxStretch > 1.0f);
+        return (e.y & kRowCell) && bodyActive[e.y & ~kRowCell] && (WORK != RowWork::kLimit || maxStretch > 1.0f);
     };
     const uint32_t oddBody = odd.y & ~kRowCell;
     uint32_t body = even.y & ~kRowCell;  // an empty slot names body 0
@@ -248,7 +251,7 @@ __global__ void __launch_bounds__(kRowBlock, EARLY ? 3 : 2) elasticRowKernel(con
         // The previous positions stay in shared memory, read where they are
         // used: 24 registers fewer, which is a block more an SM.
         auto prev = [&](int c) { return sharedXyz(&before[second][c][t]); };
-        if (!LIMIT_ONLY && !projectCellInRange(p, prev, w, k)) {
+        if (WORK != RowWork::kLimit && !projectCellInRange(p, prev, w, k)) {
             if (second) {
 #pragma unroll
                 for (int c = 0; c < 8; c++) pos[ids[c]] = stage[c][t];
@@ -257,7 +260,7 @@ __global__ void __launch_bounds__(kRowBlock, EARLY ? 3 : 2) elasticRowKernel(con
 #pragma unroll
             for (int c = 0; c < 8; c++) p[c] = xyz(pos[ids[c]]);
         }
-        if (k.maxStretch > 1.0f) limitStretch(p, w, k, lens);
+        if (WORK != RowWork::kProject && k.maxStretch > 1.0f) limitStretch(p, w, k, lens);
     }
     if (!EARLY) pdlLaunchNext();
     if (!solve) return;
@@ -716,15 +719,22 @@ cudaError_t launchElastic(const LaunchCtx& c, const DeviceState& s, const uint4*
 }
 
 cudaError_t launchElasticRows(const LaunchCtx& c, const DeviceState& s, const uint4* groups, uint32_t count,
-                              bool limitOnly, const StretchLengths& lens) {
+                              RowWork work, const StretchLengths& lens) {
     auto go = [&](auto kernel) {
         return launch(c, kernel, count, kRowBlock, groups, (const DevBody*)s.bodies, (const uint32_t*)s.bodyActive,
                       s.pos, (const float4*)s.prev, lens);
     };
     // One block an SM or fewer: a single wave, whose launch of the next kernel
     // waits for its arithmetic.
-    if (count <= c.sms) return limitOnly ? go(elasticRowKernel<true, false>) : go(elasticRowKernel<false, false>);
-    return limitOnly ? go(elasticRowKernel<true, true>) : go(elasticRowKernel<false, true>);
+    const bool early = count > c.sms;
+    switch (work) {
+        case RowWork::kProject:
+            return early ? go(elasticRowKernel<RowWork::kProject, true>) : go(elasticRowKernel<RowWork::kProject, false>);
+        case RowWork::kBoth:
+            return early ? go(elasticRowKernel<RowWork::kBoth, true>) : go(elasticRowKernel<RowWork::kBoth, false>);
+        default:
+            return early ? go(elasticRowKernel<RowWork::kLimit, true>) : go(elasticRowKernel<RowWork::kLimit, false>);
+    }
 }
 
 cudaError_t launchFinalize(const LaunchCtx& c, const DeviceState& s, const Span& n, bool contact, bool predictNext,
