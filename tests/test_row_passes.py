@@ -92,3 +92,14 @@ def test_operands_out_of_range(lib):
     grid[:2, :2, 40:42, :3] *= np.float32(1e-12)       # tiny
     grid[1:, 1:, 50:52, :3] += np.float32(3e4) * sc.H  # enormous
     run(scene, pos, frames=1)
+
+
+@pytest.mark.parametrize("rows,stretch", [([(171, 64, 90)], 0.0), ([(171, 64, 90)], 1.1),
+                                          ([(31 + b % 7, 24, 25 - b % 5) for b in range(44)], 0.0)])
+def test_many_groups(lib, rows, stretch):
+    """Passes of more groups than three a multiprocessor, which a block takes
+    in turn: one body with gaps, with the stretch limit, and bodies that
+    change from group to group."""
+    scene = scene_of(rows, 0.15, seed=8, stretch=stretch)
+    scene.substeps = 2
+    run(scene, strained(scene, amount=0.1), frames=1)

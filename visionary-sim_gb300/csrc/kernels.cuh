@@ -37,6 +37,11 @@ struct DeviceState {
     float4* sMoved = nullptr;     //   ... its motion over the substep, its body's friction
     uint32_t* sRec = nullptr;     //   ... its record index
     uint32_t* sKey = nullptr;     //   ... its bucket
+    // the two-launch chain (launchContactSlots; null where it is not used)
+    uint4* slots = nullptr;       // per bucket: its first kSlots arrivals
+    uint32_t* over = nullptr;     // per bucket: the last arrival past those
+    uint32_t* next = nullptr;     // per record past its bucket's slots: the one that arrived before it
+    float4* recPos = nullptr;     // per record: its node's position and weight
     // drive
     uint32_t* driven = nullptr;
     float4* drivenOffset = nullptr;
@@ -228,6 +233,14 @@ cudaError_t launchFinalize(const LaunchCtx& c, const DeviceState& s, const Span&
 cudaError_t launchContact(const LaunchCtx& c, const DeviceState& s, const Span& records, uint32_t recordItems,
                           int mapping, ContactMode mode, uint32_t* pairs, uint32_t capacity,
                           unsigned long long* pairCount, cudaEvent_t* marks = nullptr);
+// The solve as two launches, over a dense span of records: bin, and a gather
+// that reads the buckets as bin left them. One grid holds every body (its
+// bucket strides along y and z).
+constexpr uint32_t kSlots = 4;
+constexpr uint32_t kSlotBuckets = 1u << 26;  // buckets at most
+constexpr uint32_t kSlotKernels = 2;
+cudaError_t launchContactSlots(const LaunchCtx& c, const DeviceState& s, const Span& records, uint32_t rowStride,
+                               uint32_t planeStride);
 // After a Solve-mode contact chain: counts the gather's work on the grid it
 // built (out[0] live records, out[1] visible candidates, out[2] occupied
 // buckets; added to) and empties the grid without applying corrections.

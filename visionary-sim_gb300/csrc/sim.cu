@@ -337,6 +337,11 @@ struct Profiler {
 
 constexpr uint32_t kContactKernels = 5;  // bin, segment, scatter, order, collide
 
+// Whether a frame's contact runs as the two-launch chain: a scene's bodies
+// sharing one grid, every one of them stepped, no gather mapping asked for.
+bool inSlots(const vsim_sim* s) { return s->d.slots && !s->plan.chunked && s->gatherMapping == VSIM_GATHER_AUTO; }
+uint32_t contactKernels(const vsim_sim* s) { return inSlots(s) ? kSlotKernels : kContactKernels; }
+
 // One colour pass: the TMA brick form for a large dense pass when it is on,
 // else launchElastic's choice.
 cudaError_t launchColourPass(const LaunchCtx& c, const vsim_sim* s, int col, bool limitOnly,
@@ -410,8 +415,12 @@ cudaError_t encodeFrame(vsim_sim* s, cudaStream_t st, uint32_t steps, ContactMod
         for (int q = 0; limited && q < 3; q++)
             if ((e = sweep(true))) return e;
         if (contact && plan.records.grid) {
-            begin(VSIM_KIND_CONTACT, kContactKernels);
-            if ((e = launchContact(c, s->d, plan.records, s->surfaceCount, s->gatherMapping, mode, nullptr, 0, nullptr))) return e;
+            begin(VSIM_KIND_CONTACT, contactKernels(s));
+            e = inSlots(s) ? launchContactSlots(c, s->d, plan.records, s->grids[0].dims[0],
+                                            s->grids[0].dims[0] * s->grids[0].dims[1])
+                           : launchContact(c, s->d, plan.records, s->surfaceCount, s->gatherMapping, mode, nullptr, 0,
+                                           nullptr);
+            if (e) return e;
             end();
         }
         begin(VSIM_KIND_FINALIZE, 1);
@@ -501,7 +510,7 @@ void freeSim(vsim_sim* s) {
     DeviceState& d = s->d;
     void* ptrs[] = {d.pos, d.prev, d.vel, d.baseW, d.active, d.activeBody, d.cells, d.bodies, d.fp,
                     d.surf, d.key, d.rank, d.entries, d.count, d.start, d.cursor, d.delta, d.driven,
-                    d.drivenOffset, d.drivenOf, d.rows, d.nodeRecord, d.sMeta, d.sPos, d.sMoved, d.sRec, d.sKey, d.bodyActive, d.grabs,
+                    d.drivenOffset, d.drivenOf, d.rows, d.slots, d.over, d.next, d.recPos, d.nodeRecord, d.sMeta, d.sPos, d.sMoved, d.sRec, d.sKey, d.bodyActive, d.grabs,
                     s->chunkDev, s->staging, s->pairs, s->pairCount, s->sp.embed, s->sp.quat,
                     s->sp.scaleBody, s->sp.bodies, s->sp.meanDepth, s->sp.cov, s->sp.keys, s->sp.order,
                     s->sp.sortTemp};
@@ -680,6 +689,12 @@ int createSim(const vsim_body_desc* bodies, uint32_t n, const vsim_tank* tank, v
     CK(allocN(&d.nodeRecord, N), "allocate node records");
     CK(allocN(&d.count, s->bucketTotal), "allocate contact grid");
     CK(allocN(&d.start, s->bucketTotal), "allocate contact grid");
+    if (!s->isolated && s->bucketTotal <= kSlotBuckets) {
+        CK(allocN(&d.slots, s->bucketTotal), "allocate contact slots");
+        CK(allocN(&d.over, s->bucketTotal), "allocate contact slots");
+        CK(allocN(&d.next, s->surfaceCount), "allocate contact slots");
+        CK(allocN(&d.recPos, s->surfaceCount), "allocate contact slots");
+    }
     CK(allocN(&d.bodyActive, s->activeHost.size()), "allocate body activity");
     CK(allocN(&d.grabs, s->grabsHost.size()), "allocate drive targets");
     CK(allocN(&d.cursor, 1), "allocate contact cursor");
@@ -1368,7 +1383,7 @@ uint32_t vsim_frame_launches(const vsim_sim* s, uint32_t steps) {
         for (int c = 0; c < 8; c++) passes += s->colorStart[c + 1] > s->colorStart[c] ? 1 : 0;
     uint32_t per = 1 + passes * s->iterations;
     if (anyStretch(s)) per += 3 * passes;
-    if (s->contact && s->surfaceCount > 0) per += kContactKernels;
+    if (s->contact && s->surfaceCount > 0) per += contactKernels(s);
     return steps ? 1 + per * steps : 0;
 }
 

@@ -554,6 +554,258 @@ __global__ void __launch_bounds__(kCollideBlock, 5) collideKernel(
         collideWarp<EMIT>(i, arrays, selfContact, runAt[threadIdx.x >> 5], emit);
 }
 
+// ------------------------------------------- contact in two launches --
+//
+// The chain above takes five dependent launches, of which segments, scatter
+// and order only lay the buckets out. A bucket rarely holds more than a few
+// records (edge h, about one surface node each at rest), so here bin stores a
+// record straight into its bucket: the first kSlots arrivals in the bucket's
+// own slots, later ones in a list threaded through the records. The gather
+// reads the buckets around a record as bin left them and orders each one's
+// few entries itself, as sort.wgsl:14-53 would: ascending, the 32 lowest.
+// Two launches against five: the 64^3 blob's frame (49k records) 569 -> 465
+// us, a six-body pile's (8.9k) 322 -> 285 us, a 161x150x157 scene's (352k) 9.10
+// -> 8.66 ms.
+//
+// Nothing is reset but the counts (by the closing pass): slots past a
+// bucket's count and the list past its overflow are never read.
+//
+// The bodies share one grid of at most kSlotBuckets buckets, so a record's
+// bucket and which faces of the grid it lies on fit one word.
+
+__global__ void binSlotsKernel(Work work, const uint4* __restrict__ surf, const DevBody* __restrict__ bodies,
+                               const uint32_t* __restrict__ bodyActive, const float4* __restrict__ pos,
+                               uint32_t* __restrict__ key, uint32_t* __restrict__ place, uint32_t* __restrict__ count,
+                               uint32_t* __restrict__ slots, uint32_t* __restrict__ over, uint32_t* __restrict__ next,
+                               float4* __restrict__ recPos) {
+    struct Pre {
+        uint4 rec;
+        uint32_t live;
+    };
+    auto pre = [&](uint32_t r) {
+        const uint4 rec = surf[r];
+        return Pre{rec, bodyActive[rec.y]};
+    };
+    forEachItemAfterWait(work, pre, [&](uint32_t r, const Pre& q) {
+        if (!q.live) {
+            key[r] = kIdle;
+            place[r] = kIdle;
+            return;
+        }
+        const float4 P = pos[q.rec.x];
+        const DevBody* grid = bodies + q.rec.y;
+        int coord[3];
+        const uint32_t b = bucketOf(grid, xyz(P), coord);
+        const uint32_t rank = atomicAdd(&count[b], 1u);
+        uint32_t faces = 0;
+#pragma unroll
+        for (int a = 0; a < 3; a++)
+            faces |= (coord[a] == 0 ? 1u : 0u) << (2 * a) | (coord[a] + 1 == int(grid->gridDims[a]) ? 2u : 0u) << (2 * a);
+        key[r] = b;
+        place[r] = b | faces * kSlotBuckets;
+        recPos[r] = P;
+        if (rank < kSlots)
+            slots[kSlots * size_t(b) + rank] = r;
+        else
+            next[r] = atomicExch(&over[b], r);
+    });
+}
+
+constexpr uint32_t kSlotsBlock = 128;   // threads of a gather block
+constexpr uint32_t kGatherLanes = 9;    // lanes a record: one per row of three buckets along x
+constexpr uint32_t kGatherRecords = 3;  // records a warp
+constexpr uint32_t kGatherList = 96;    // candidates of a record its lanes go through together
+
+// The smallest record of bucket b above `last` (kIdle: none), for the records
+// with more candidates than the list holds.
+__device__ uint32_t nextInBucket(uint32_t b, uint32_t n, uint32_t last, bool any, const uint4* slots,
+                                 const uint32_t* over, const uint32_t* next) {
+    uint32_t best = kIdle;
+    uint32_t e = 0;
+    for (uint32_t i = 0; i < n; i++) {
+        if (i < kSlots)
+            e = reinterpret_cast<const uint32_t*>(slots + b)[i];
+        else
+            e = i == kSlots ? over[b] : next[e];
+        if ((any || e > last) && e < best) best = e;
+    }
+    return best;
+}
+
+// collide.wgsl:16-125 for every live record. Nine lanes share a record, three
+// records a warp: a lane sizes and orders the three buckets of its row
+// (dy, dz), the entries go into one list in the reference's candidate order
+// (dz, dy, dx, then ascending), and the lanes take the list eighteen at a
+// time; hits are added in list order. Against a warp a record this is 190
+// warp instructions a record instead of 430, and everything a candidate
+// needs but its record index is one load deep: bin left each record's
+// position by record. Bound by the latency of its four dependent loads (own
+// record, buckets, candidates, a hit's motion) at half issue: 128 threads
+// and 64 registers, eight blocks an SM, measured best (the 64^3 blob's frame
+// 465 us; with ten blocks, which spill, 484).
+//
+// A record with more than kGatherList candidates, or next to a bucket of
+// more than 32, is gone through by its first lane alone.
+__global__ void __launch_bounds__(kSlotsBlock, 8) collideSlotsKernel(
+    const FrameParams* __restrict__ fp, uint32_t records, uint32_t rowStride, uint32_t planeStride,
+    const uint4* __restrict__ surf, const DevBody* __restrict__ bodies, const uint32_t* __restrict__ place,
+    const uint32_t* __restrict__ count, const uint4* __restrict__ slots, const uint32_t* __restrict__ over,
+    const uint32_t* __restrict__ next, const float4* __restrict__ recPos, const float4* __restrict__ prevState,
+    float4* __restrict__ delta) {
+    constexpr unsigned kAll = 0xffffffffu;
+    constexpr uint32_t kGroup = (1u << kGatherLanes) - 1u;
+    __shared__ uint32_t lists[kSlotsBlock / 32][kGatherRecords][kGatherList];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t group = lane / kGatherLanes, q = lane - group * kGatherLanes;
+    const uint32_t r = (blockIdx.x * (kSlotsBlock / 32) + warp) * kGatherRecords + group;
+    const bool valid = group < kGatherRecords && r < records;
+    Contactor c;
+    c.me = valid ? surf[r] : make_uint4(0, 0, 0, 0);
+    c.node = c.me.x;
+    c.radius = __uint_as_float(c.me.w);
+    const uint32_t selfContact = fp->selfContact;
+    pdlWait();
+    const uint32_t home = valid ? place[r] : kIdle;
+    const bool live = home != kIdle;
+    const float4 P = live ? recPos[r] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    c.pi = xyz(P);
+    c.wi = P.w;
+    // Whether row `row` (dy + 3 dz, offsets + 1) of the record's buckets is in
+    // the grid, and its middle bucket; whether its bucket d (dx + 1) is.
+    auto rowOf = [&](uint32_t row, uint32_t& middle) {
+        const uint32_t dy = row % 3, dz = row / 3, faces = home / kSlotBuckets;
+        middle = (home & (kSlotBuckets - 1)) + (dy - 1) * rowStride + (dz - 1) * planeStride;
+        return !((dy == 0 && faces & 4u) || (dy == 2 && faces & 8u) || (dz == 0 && faces & 16u) ||
+                 (dz == 2 && faces & 32u));
+    };
+    auto inRow = [&](uint32_t d) { return !((d == 0 && home & kSlotBuckets) || (d == 2 && home & (2 * kSlotBuckets))); };
+    uint32_t held[3] = {0, 0, 0}, middle = 0;
+    uint4 entry[3] = {};
+    if (live && rowOf(q, middle)) {
+#pragma unroll
+        for (uint32_t d = 0; d < 3; d++) {
+            if (!inRow(d)) continue;
+            held[d] = count[middle + d - 1];
+            entry[d] = slots[middle + d - 1];  // read with the count: past it, left over and unused
+        }
+    }
+    // Where the lane's entries go in the record's list.
+    const uint32_t mine = held[0] + held[1] + held[2];
+    uint32_t end = mine;
+#pragma unroll
+    for (uint32_t d = 1; d < kGatherLanes; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(kAll, end, d);
+        if (q >= d) end += v;
+    }
+    const uint32_t groupAt = group * kGatherLanes;
+    const uint32_t total = __shfl_sync(kAll, end, min(groupAt + kGatherLanes - 1, 31u));
+    const uint32_t crowded = __ballot_sync(kAll, max(held[0], max(held[1], held[2])) > kBucketSlots);
+    const bool listed = live && total <= kGatherList && (crowded >> groupAt & kGroup) == 0;
+    uint32_t* list = lists[warp][min(group, kGatherRecords - 1)];
+    if (listed) {
+        uint32_t at = end - mine;
+#pragma unroll
+        for (uint32_t d = 0; d < 3; d++) {
+            const uint32_t n = held[d];
+            // The slots' records in ascending order, left-overs last.
+            uint32_t e0 = n > 0 ? entry[d].x : kIdle, e1 = n > 1 ? entry[d].y : kIdle;
+            uint32_t e2 = n > 2 ? entry[d].z : kIdle, e3 = n > 3 ? entry[d].w : kIdle;
+            auto ascend = [](uint32_t& a, uint32_t& b) {
+                const uint32_t low = min(a, b);
+                b = max(a, b);
+                a = low;
+            };
+            ascend(e0, e1);
+            ascend(e2, e3);
+            ascend(e0, e2);
+            ascend(e1, e3);
+            ascend(e1, e2);
+            if (n > 0) list[at] = e0;
+            if (n > 1) list[at + 1] = e1;
+            if (n > 2) list[at + 2] = e2;
+            if (n > 3) list[at + 3] = e3;
+            uint32_t more = 0;
+            for (uint32_t i = kSlots; i < n; i++) {  // the few past the slots, by insertion
+                more = i == kSlots ? over[middle + d - 1] : next[more];
+                uint32_t to = at + i;
+                while (to > at && list[to - 1] > more) {
+                    list[to] = list[to - 1];
+                    to--;
+                }
+                list[to] = more;
+            }
+            at += n;
+        }
+    }
+    __syncwarp();
+    V sum = mk(0.0f, 0.0f, 0.0f);
+    float hits = 0.0f;
+    // The correction of a hit.
+    auto correct = [&](uint4 them, float4 Q, float dist2) {
+        c.movedI = c.pi - xyz(prevState[c.node]);
+        c.frictionI = bodies[c.me.y].friction;
+        const V moved = xyz(Q) - xyz(prevState[them.x]);
+        return contactCorrection(c, them, Q, withW(moved, bodies[them.y].friction), dist2);
+    };
+    const uint32_t longest = __reduce_max_sync(kAll, listed ? total : 0u);
+    for (uint32_t round = 0; round < longest; round += 2 * kGatherLanes) {
+        // Two candidates a lane, nine apart, their records loaded together.
+        uint4 them[2];
+        float4 Q[2];
+        bool has[2];
+#pragma unroll
+        for (uint32_t h = 0; h < 2; h++) {
+            const uint32_t j = round + h * kGatherLanes + q;
+            has[h] = listed && j < total;
+            if (has[h]) {
+                const uint32_t other = list[j];
+                them[h] = surf[other];
+                Q[h] = recPos[other];
+            }
+        }
+#pragma unroll
+        for (uint32_t h = 0; h < 2; h++) {
+            float dist2 = 0.0f;
+            const bool hit = has[h] && contactHit(c, them[h], Q[h], selfContact, dist2);
+            uint32_t bits = __ballot_sync(kAll, hit);
+            if (bits == 0) continue;
+            V correction = mk(0.0f, 0.0f, 0.0f);
+            if (hit) correction = correct(them[h], Q[h], dist2);
+            bits = group < kGatherRecords ? bits >> groupAt & kGroup : 0u;
+            while (__any_sync(kAll, bits != 0)) {
+                const uint32_t from = bits ? groupAt + __ffs(bits) - 1 : lane;
+                const V add = mk(__shfl_sync(kAll, correction.x, from), __shfl_sync(kAll, correction.y, from),
+                                 __shfl_sync(kAll, correction.z, from));
+                if (!bits) continue;
+                sum = sum + add;
+                hits = hits + 1.0f;
+                bits &= bits - 1;
+            }
+        }
+    }
+    if (live && !listed && q == 0) {
+        for (uint32_t row = 0; row < kGatherLanes; row++) {
+            if (!rowOf(row, middle)) continue;
+            for (uint32_t d = 0; d < 3; d++) {
+                if (!inRow(d)) continue;
+                const uint32_t b = middle + d - 1, n = count[b];
+                uint32_t last = 0;
+                for (uint32_t i = 0; i < min(n, kBucketSlots); i++) {
+                    last = nextInBucket(b, n, last, i == 0, slots, over, next);
+                    const uint4 them = surf[last];
+                    const float4 Q = recPos[last];
+                    float dist2;
+                    if (!contactHit(c, them, Q, selfContact, dist2)) continue;
+                    sum = sum + correct(them, Q, dist2);
+                    hits = hits + 1.0f;
+                }
+            }
+        }
+    }
+    if (live && q == 0) delta[r] = withW(sum, hits);
+    pdlLaunchNext();
+}
+
 // settle.wgsl:20-36 (gain 1, bodyContact.js:48), then empties the buckets
 // this substep used and the segment cursor, restoring the empty grid.
 __global__ void settleKernel(const FrameParams* __restrict__ fp, Work work, const uint4* __restrict__ surf,
@@ -807,6 +1059,19 @@ cudaError_t launchContact(const LaunchCtx& c, const DeviceState& s, const Span& 
     }
     if ((e = collide(collideKernel<false>, (uint32_t*)nullptr, 0u, (unsigned long long*)nullptr))) return e;
     return mark(5);
+}
+
+cudaError_t launchContactSlots(const LaunchCtx& c, const DeviceState& s, const Span& r, uint32_t rowStride,
+                               uint32_t planeStride) {
+    cudaError_t e;
+    if ((e = launch(c, binSlotsKernel, r.grid, r.block, r.work, s.surf, (const DevBody*)s.bodies,
+                    (const uint32_t*)s.bodyActive, (const float4*)s.pos, s.key, s.rank, s.count,
+                    reinterpret_cast<uint32_t*>(s.slots), s.over, s.next, s.recPos)))
+        return e;
+    return launch(c, collideSlotsKernel, blocks(r.work.count, kGatherRecords * (kSlotsBlock / 32)), kSlotsBlock, s.fp,
+                  r.work.count, rowStride, planeStride, s.surf, (const DevBody*)s.bodies, (const uint32_t*)s.rank,
+                  (const uint32_t*)s.count, (const uint4*)s.slots, (const uint32_t*)s.over, (const uint32_t*)s.next,
+                  (const float4*)s.recPos, (const float4*)s.prev, s.delta);
 }
 
 cudaError_t launchCensus(const LaunchCtx& c, const DeviceState& s, const Span& r, unsigned long long* out) {
