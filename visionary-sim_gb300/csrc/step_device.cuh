@@ -707,57 +707,29 @@ struct ContactArrays {
     float4* delta;
 };
 
-// sort.wgsl:14-53 for binned record r (see canonKernel): a record of a
-// bucket of at most kBucketSlots entries copies itself to its place; in a
-// larger bucket the first-arriving record orders and copies them all.
-__device__ __forceinline__ void canonRecord(uint32_t r, const ContactArrays& a, uint32_t* entries,
+// sort.wgsl:14-53 for binned record r (see canonKernel): it copies itself to
+// its place in its bucket, the number of the bucket's records with a lower
+// index. In a bucket past kBucketSlots entries that keeps the lowest in front,
+// which is all the gather looks at; every record still has a place of its own.
+// (Ordering such a bucket by one of its records alone is a serial chain over
+// memory: sessions dragged into a heap, with hundreds of records in a bucket,
+// spent most of their time in it.)
+__device__ __forceinline__ void canonRecord(uint32_t r, const ContactArrays& a, const uint32_t* entries,
                                             const SortedEntries& out, const float4* pos, const float4* prevState) {
     const uint32_t b = a.key[r];
     const uint32_t n = a.count[b];
     const uint32_t base = a.start[b];
-    uint32_t* e = entries + base;
-    auto copyOut = [&](uint32_t at, uint32_t record, uint4 rec) {
-        const float4 P = pos[rec.x], R = prevState[rec.x];
-        out.sMeta[at] = rec;
-        out.sPos[at] = P;
-        out.sMoved[at] = withW(xyz(P) - xyz(R), a.bodies[rec.y].friction);
-        out.sRec[at] = record;
-        out.sKey[at] = b;
-    };
-    if (n <= kBucketSlots) {
-        const uint4 mine = a.surf[r];
-        uint32_t place = 0;
-        for (uint32_t j = 0; j < n; j++) place += e[j] < r ? 1u : 0u;
-        copyOut(base + place, r, mine);
-        return;
-    }
-    if (a.rank[r] != 0) return;
-    const uint32_t m = kBucketSlots;
-    for (uint32_t i = 1; i < m; i++) {
-        const uint32_t v = e[i];
-        uint32_t at = i;
-        while (at > 0 && e[at - 1] > v) {
-            e[at] = e[at - 1];
-            at--;
-        }
-        e[at] = v;
-    }
-    // Past capacity, keep the lowest kBucketSlots in the visible prefix.
-    for (uint32_t i = m; i < n; i++) {
-        const uint32_t v = e[i];
-        if (v >= e[m - 1]) continue;
-        e[i] = e[m - 1];
-        uint32_t at = m - 1;
-        while (at > 0 && e[at - 1] > v) {
-            e[at] = e[at - 1];
-            at--;
-        }
-        e[at] = v;
-    }
-    for (uint32_t k = 0; k < n; k++) {
-        const uint32_t other = e[k];
-        copyOut(base + k, other, a.surf[other]);
-    }
+    const uint32_t* e = entries + base;
+    const uint4 rec = a.surf[r];
+    uint32_t place = base;
+#pragma unroll 4
+    for (uint32_t j = 0; j < n; j++) place += e[j] < r ? 1u : 0u;
+    const float4 P = pos[rec.x], R = prevState[rec.x];
+    out.sMeta[place] = rec;
+    out.sPos[place] = P;
+    out.sMoved[place] = withW(xyz(P) - xyz(R), a.bodies[rec.y].friction);
+    out.sRec[place] = r;
+    out.sKey[place] = b;
 }
 
 // Entry i of the bucket order: its record r, position, motion and bucket as

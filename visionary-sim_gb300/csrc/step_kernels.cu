@@ -471,15 +471,11 @@ __global__ void scatterKernel(const FrameParams* __restrict__ fp, Work work, con
 // contiguous run and both a record's own data and a candidate's one load
 // deep.
 //
-// A bucket of at most kBucketSlots entries is all visible: each of its
-// records finds its own place (how many of the bucket's records have a lower
-// index) and copies itself there, all records at once. A larger bucket is
-// ordered by its first-arriving record alone, an insertion sort that keeps
-// the lowest kBucketSlots in front (rare: 32 surface nodes in one bucket of
-// edge h).
+// Each record finds its own place, how many of the bucket's records have a
+// lower index, and copies itself there, all records at once.
 __global__ void canonKernel(const FrameParams* __restrict__ fp, Work work, const uint32_t* __restrict__ key,
                             const uint32_t* __restrict__ rank, const uint32_t* __restrict__ start,
-                            const uint32_t* __restrict__ count, uint32_t* __restrict__ entries,
+                            const uint32_t* __restrict__ count, const uint32_t* __restrict__ entries,
                             const uint4* __restrict__ surf, const float4* __restrict__ pos,
                             const float4* __restrict__ prevState, const DevBody* __restrict__ bodies,
                             uint4* __restrict__ sMeta, float4* __restrict__ sPos, float4* __restrict__ sMoved,
@@ -1026,7 +1022,7 @@ cudaError_t launchContact(const LaunchCtx& c, const DeviceState& s, const Span& 
         return e;
     if ((e = mark(3))) return e;
     if ((e = launch(c, canonKernel, g, b, s.fp, w, (const uint32_t*)s.key, (const uint32_t*)s.rank,
-                    (const uint32_t*)s.start, (const uint32_t*)s.count, s.entries, (const uint4*)s.surf,
+                    (const uint32_t*)s.start, (const uint32_t*)s.count, (const uint32_t*)s.entries, (const uint4*)s.surf,
                     (const float4*)s.pos, (const float4*)s.prev, (const DevBody*)s.bodies, s.sMeta, s.sPos,
                     s.sMoved, s.sRec, s.sKey)))
         return e;
