@@ -364,14 +364,14 @@ struct SplatState {
     float4* quat = nullptr;     // xyzw
     float4* scaleBody = nullptr;  // (sx, sy, sz, body as bits)
     SplatBody* bodies = nullptr;
-    float4* meanDepth = nullptr;  // deformed mean, depth along the view
-    float2* cov = nullptr;        // 3 x float2 per splat: (xx, xy), (xz, yy), (yz, zz)
+    float* means = nullptr;       // deformed means, xyz each (vsim_splats_read's layout)
+    float2* cov = nullptr;        // 3 x float2 per splat: (xx, xy), (xz, yy), (yz, zz) (the ABI's cov6)
     uint32_t* keys = nullptr;
     uint32_t* order = nullptr;
     void* sortTemp = nullptr;
     size_t sortTempBytes = 0;
     float4* axesRotation = nullptr;  // per splat: the deformed ellipsoid's unit quaternion xyzw
-    float4* axesScale = nullptr;     //   ... and its axis lengths xyz (allocated on first use)
+    float* axesScale = nullptr;      //   ... and its axis lengths xyz (allocated on first use)
 };
 
 // With `axes` the deformation also takes each covariance apart into a

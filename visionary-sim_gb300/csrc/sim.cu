@@ -512,8 +512,8 @@ void freeSim(vsim_sim* s) {
                     d.surf, d.key, d.rank, d.entries, d.count, d.start, d.cursor, d.delta, d.driven,
                     d.drivenOffset, d.drivenOf, d.rows, d.slots, d.over, d.next, d.recPos, d.nodeRecord, d.sMeta, d.sPos, d.sMoved, d.sRec, d.sKey, d.bodyActive, d.grabs,
                     s->chunkDev, s->staging, s->pairs, s->pairCount, s->sp.embed, s->sp.quat,
-                    s->sp.scaleBody, s->sp.bodies, s->sp.meanDepth, s->sp.cov, s->sp.keys, s->sp.order,
-                    s->sp.sortTemp};
+                    s->sp.scaleBody, s->sp.bodies, s->sp.means, s->sp.cov, s->sp.keys, s->sp.order,
+                    s->sp.sortTemp, s->sp.axesRotation, s->sp.axesScale};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     freeTmaPass(s->tma);
@@ -1490,7 +1490,7 @@ namespace {
 
 int rebuildSplats(vsim_sim* s) {
     SplatState& sp = s->sp;
-    void* old[] = {sp.embed,  sp.quat,  sp.scaleBody, sp.bodies,       sp.meanDepth, sp.cov,
+    void* old[] = {sp.embed,  sp.quat,  sp.scaleBody, sp.bodies,       sp.means, sp.cov,
                    sp.keys,   sp.order, sp.sortTemp,  sp.axesRotation, sp.axesScale};
     CK(cudaStreamSynchronize(s->stream), "rebind splats");
     for (void* p : old)
@@ -1538,7 +1538,7 @@ int rebuildSplats(vsim_sim* s) {
     CK(allocN(&sp.quat, n), "allocate splats");
     CK(allocN(&sp.scaleBody, n), "allocate splats");
     CK(allocN(&sp.bodies, bodies.size()), "allocate splats");
-    CK(allocN(&sp.meanDepth, n), "allocate splats");
+    CK(allocN(&sp.means, 3 * n), "allocate splats");
     CK(allocN(&sp.cov, 3 * n), "allocate splats");
     CK(allocN(&sp.keys, n), "allocate splats");
     CK(allocN(&sp.order, n), "allocate splats");
@@ -1584,7 +1584,7 @@ int vsim_splats_deform_axes(vsim_sim* s, const float view_dir[3]) {
     if (s->splatCount == 0) return VSIM_OK;
     if (!s->sp.axesRotation) {
         CK(allocN(&s->sp.axesRotation, s->splatCount), "allocate splat axes");
-        CK(allocN(&s->sp.axesScale, s->splatCount), "allocate splat axes");
+        CK(allocN(&s->sp.axesScale, 3 * size_t(s->splatCount)), "allocate splat axes");
     }
     CK(launchSplatDeform(s->stream, s->sp, s->d.pos, s->splatCount, view_dir[0], view_dir[1], view_dir[2], true),
        "deform splats");
@@ -1596,23 +1596,10 @@ int vsim_splats_read_axes(vsim_sim* s, float* rotation, float* scale, size_t cou
     if (count != s->splatCount) return fail(VSIM_ERR_CAPACITY, "count does not match the bound splats");
     if (count == 0) return VSIM_OK;
     if (!s->sp.axesRotation) return fail(VSIM_ERR_INVALID, "no axes yet: call vsim_splats_deform_axes first");
-    std::vector<float4> rot(count), sc(count);
-    CK(cudaMemcpyAsync(rot.data(), s->sp.axesRotation, count * 16, cudaMemcpyDeviceToHost, s->stream), "read axes");
-    CK(cudaMemcpyAsync(sc.data(), s->sp.axesScale, count * 16, cudaMemcpyDeviceToHost, s->stream), "read axes");
+    if (rotation)
+        CK(cudaMemcpyAsync(rotation, s->sp.axesRotation, count * 16, cudaMemcpyDeviceToHost, s->stream), "read axes");
+    if (scale) CK(cudaMemcpyAsync(scale, s->sp.axesScale, count * 12, cudaMemcpyDeviceToHost, s->stream), "read axes");
     CK(cudaStreamSynchronize(s->stream), "read axes");
-    for (size_t i = 0; i < count; i++) {
-        if (rotation) {
-            rotation[4 * i] = rot[i].x;
-            rotation[4 * i + 1] = rot[i].y;
-            rotation[4 * i + 2] = rot[i].z;
-            rotation[4 * i + 3] = rot[i].w;
-        }
-        if (scale) {
-            scale[3 * i] = sc[i].x;
-            scale[3 * i + 1] = sc[i].y;
-            scale[3 * i + 2] = sc[i].z;
-        }
-    }
     return VSIM_OK;
 }
 
@@ -1628,32 +1615,11 @@ int vsim_splats_read(vsim_sim* s, float* means, float* cov6, uint32_t* order, si
     SIM_GUARD(s);
     if (count != s->splatCount) return fail(VSIM_ERR_CAPACITY, "count does not match the bound splats");
     if (count == 0) return VSIM_OK;
-    if (means || cov6) {
-        std::vector<float4> md(count);
-        std::vector<float2> cv(3 * count);
-        CK(cudaMemcpyAsync(md.data(), s->sp.meanDepth, count * 16, cudaMemcpyDeviceToHost, s->stream), "read splats");
-        CK(cudaMemcpyAsync(cv.data(), s->sp.cov, count * 24, cudaMemcpyDeviceToHost, s->stream), "read splats");
-        CK(cudaStreamSynchronize(s->stream), "read splats");
-        for (size_t i = 0; i < count; i++) {
-            if (means) {
-                means[3 * i] = md[i].x;
-                means[3 * i + 1] = md[i].y;
-                means[3 * i + 2] = md[i].z;
-            }
-            if (cov6) {
-                cov6[6 * i] = cv[3 * i].x;
-                cov6[6 * i + 1] = cv[3 * i].y;
-                cov6[6 * i + 2] = cv[3 * i + 1].x;
-                cov6[6 * i + 3] = cv[3 * i + 1].y;
-                cov6[6 * i + 4] = cv[3 * i + 2].x;
-                cov6[6 * i + 5] = cv[3 * i + 2].y;
-            }
-        }
-    }
-    if (order) {
-        CK(cudaMemcpyAsync(order, s->sp.order, count * 4, cudaMemcpyDeviceToHost, s->stream), "read order");
-        CK(cudaStreamSynchronize(s->stream), "read order");
-    }
+    // Each output lies on the device as the ABI gives it: one copy each.
+    if (means) CK(cudaMemcpyAsync(means, s->sp.means, count * 12, cudaMemcpyDeviceToHost, s->stream), "read splats");
+    if (cov6) CK(cudaMemcpyAsync(cov6, s->sp.cov, count * 24, cudaMemcpyDeviceToHost, s->stream), "read splats");
+    if (order) CK(cudaMemcpyAsync(order, s->sp.order, count * 4, cudaMemcpyDeviceToHost, s->stream), "read order");
+    CK(cudaStreamSynchronize(s->stream), "read splats");
     return VSIM_OK;
 }
 

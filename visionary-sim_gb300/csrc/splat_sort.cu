@@ -26,7 +26,7 @@ __device__ __forceinline__ uint32_t depthKey(float depth) {
 // inverseSqrt is 1 / sqrt and normalize is q / sqrt(|q|^2) with |q|^2 fused
 // as dot is; every other operation rounds once -- the CPU restatement's
 // evaluation, so the two agree bit for bit.
-__device__ __forceinline__ void ellipsoidAxes(const float cov[6], float4& rotation, float4& scale) {
+__device__ __forceinline__ void ellipsoidAxes(const float cov[6], float4& rotation, V& scale) {
     float a[9] = {cov[0], cov[1], cov[2], cov[1], cov[3], cov[4], cov[2], cov[4], cov[5]};
     float q[4] = {0.0f, 0.0f, 0.0f, 1.0f};
 #pragma unroll
@@ -69,22 +69,48 @@ __device__ __forceinline__ void ellipsoidAxes(const float cov[6], float4& rotati
         }
     }
     rotation = make_float4(q[0], q[1], q[2], q[3]);
-    scale = make_float4(sqrtf(fmaxf(a[0], 0.0f)), sqrtf(fmaxf(a[4], 0.0f)), sqrtf(fmaxf(a[8], 0.0f)), 0.0f);
+    scale = mk(sqrtf(fmaxf(a[0], 0.0f)), sqrtf(fmaxf(a[4], 0.0f)), sqrtf(fmaxf(a[8], 0.0f)));
+}
+
+constexpr uint32_t kDeformBlock = 256;
+
+// Stores the warp's 32 vectors, lane l's at out[3 (first + l)], as whole
+// 16-byte words through 96 words of shared memory. `first` is a multiple of
+// 32; vectors from `n` on are left out. The caller's next use of `words` must
+// wait for the warp.
+__device__ __forceinline__ void storeXyz(float* out, uint32_t first, uint32_t n, V v, float* words) {
+    const uint32_t lane = threadIdx.x & 31;
+    words[3 * lane] = v.x;
+    words[3 * lane + 1] = v.y;
+    words[3 * lane + 2] = v.z;
+    __syncwarp();
+    if (first + 32 <= n) {
+        if (lane < 24)
+            __stcs(reinterpret_cast<float4*>(out + 3 * size_t(first)) + lane, reinterpret_cast<const float4*>(words)[lane]);
+    } else {
+        for (uint32_t q = lane; q < 3 * (n - first); q += 32) out[3 * size_t(first) + q] = words[q];
+    }
+    __syncwarp();
 }
 
 template <bool AXES>
-__global__ void __launch_bounds__(256) splatDeformKernel(const float4* __restrict__ embed,
+__global__ void __launch_bounds__(kDeformBlock) splatDeformKernel(const float4* __restrict__ embed,
                                                          const float4* __restrict__ quat,
                                                          const float4* __restrict__ scaleBody,
                                                          const SplatBody* __restrict__ bodies,
                                                          const float4* __restrict__ pos, uint32_t n, float vx,
-                                                         float vy, float vz, float4* __restrict__ meanDepth,
+                                                         float vy, float vz, float* __restrict__ means,
                                                          float2* __restrict__ cov, uint32_t* __restrict__ keys,
                                                          uint32_t* __restrict__ order,
                                                          float4* __restrict__ axesRotation,
-                                                         float4* __restrict__ axesScale) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+                                                         float* __restrict__ axesScale) {
+    __shared__ __align__(16) float words[kDeformBlock / 32][96];
+    const uint32_t at = blockIdx.x * blockDim.x + threadIdx.x, first = at & ~31u;
+    if (first >= n) return;
+    // The last warp's lanes past the end go through the last splat again and
+    // store nothing.
+    const uint32_t i = min(at, n - 1);
+    const bool mine = at < n;
     // The splat's embedding, scale and rotation do not change between
     // frames: loaded before waiting for the frame that moves the nodes.
     // The splat streams are read and written once, marked evict-first
@@ -131,15 +157,21 @@ __global__ void __launch_bounds__(256) splatDeformKernel(const float4* __restric
     const float yz = fmaf(a2.z, a2.y, fmaf(a1.z, a1.y, a0.z * a0.y));
     const float zz = fmaf(a2.z, a2.z, fmaf(a1.z, a1.z, a0.z * a0.z));
     const float depth = position.x * vx + position.y * vy + position.z * vz;
-    __stcs(meanDepth + i, make_float4(position.x, position.y, position.z, depth));
-    __stcs(cov + 3 * i, make_float2(xx, xy));
-    __stcs(cov + 3 * i + 1, make_float2(xz, yy));
-    __stcs(cov + 3 * i + 2, make_float2(yz, zz));
-    keys[i] = depthKey(depth);
+    storeXyz(means, first, n, position, words[threadIdx.x >> 5]);
+    if (mine) {
+        __stcs(cov + 3 * size_t(i), make_float2(xx, xy));
+        __stcs(cov + 3 * size_t(i) + 1, make_float2(xz, yy));
+        __stcs(cov + 3 * size_t(i) + 2, make_float2(yz, zz));
+        keys[i] = depthKey(depth);
+    }
     (void)order;
     if (AXES) {
         const float c6[6] = {xx, xy, xz, yy, yz, zz};
-        ellipsoidAxes(c6, axesRotation[i], axesScale[i]);
+        float4 rotation;
+        V scale;
+        ellipsoidAxes(c6, rotation, scale);
+        if (mine) axesRotation[i] = rotation;
+        storeXyz(axesScale, first, n, scale, words[threadIdx.x >> 5]);
     }
 }
 
@@ -149,8 +181,8 @@ cudaError_t launchSplatDeform(cudaStream_t st, const SplatState& s, const float4
     // Programmatic dependent launch: the constant loads above overlap the
     // tail of the frame's last kernel.
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((n + 255) / 256);
-    cfg.blockDim = dim3(256);
+    cfg.gridDim = dim3((n + kDeformBlock - 1) / kDeformBlock);
+    cfg.blockDim = dim3(kDeformBlock);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -160,10 +192,10 @@ cudaError_t launchSplatDeform(cudaStream_t st, const SplatState& s, const float4
     if (axes)
         return cudaLaunchKernelEx(&cfg, splatDeformKernel<true>, (const float4*)s.embed, (const float4*)s.quat,
                                   (const float4*)s.scaleBody, (const SplatBody*)s.bodies, pos, n, vx, vy, vz,
-                                  s.meanDepth, s.cov, s.keys, s.order, s.axesRotation, s.axesScale);
+                                  s.means, s.cov, s.keys, s.order, s.axesRotation, s.axesScale);
     return cudaLaunchKernelEx(&cfg, splatDeformKernel<false>, (const float4*)s.embed, (const float4*)s.quat,
-                              (const float4*)s.scaleBody, (const SplatBody*)s.bodies, pos, n, vx, vy, vz, s.meanDepth,
-                              s.cov, s.keys, s.order, (float4*)nullptr, (float4*)nullptr);
+                              (const float4*)s.scaleBody, (const SplatBody*)s.bodies, pos, n, vx, vy, vz, s.means,
+                              s.cov, s.keys, s.order, (float4*)nullptr, (float*)nullptr);
 }
 
 // --------------------------------------------------------- radix sort --
