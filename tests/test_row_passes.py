@@ -63,9 +63,9 @@ def test_row_lengths(lib, nx, holes):
     scene = scene_of([(nx, 3, 2)], holes, seed=nx)
     launches = run(scene, strained(scene))
     if holes == 0.0:
-        # predict, finalize, and the passes that have cells: two links' parities
-        # (y) of z parity 0 and 1, or past a group's chain the colours
-        assert launches == 2 + (4 if nx <= 256 else 8)
+        # a pass's two rows in one group: the frame in one launch; in two:
+        # predict, close and the row passes; a run past a group: the colours
+        assert launches == (1 if nx <= 128 else 6 if nx <= 256 else 10)
 
 
 def test_bodies_share_groups(lib):

@@ -211,6 +211,19 @@ enum class RowWork { kProject, kBoth, kLimit };
 cudaError_t launchElasticRows(const LaunchCtx& c, const DeviceState& s, const uint4* groups, uint32_t count,
                               RowWork work, const StretchLengths& lens);
 
+// A whole frame of a small scene without contact in one launch (small_frame.cu):
+// every row pass at most one group, at most kSmallNodes nodes.
+constexpr uint32_t kSmallNodes = 4096;  // 192 KB of shared memory
+struct SmallFrame {
+    uint32_t rowStart[kRowPasses + 1];
+    uint32_t nodeCount, activeCount;
+    uint32_t steps, iterations;
+    bool limited;  // any body limits its stretch
+    bool driving;  // nodes are held
+    StretchLengths lens;
+};
+cudaError_t launchSmallFrame(cudaStream_t st, const DeviceState& s, const SmallFrame& f);
+
 // The streaming colour pass (elasticStreamKernel): blocks of kStreamBlock
 // threads, kStreamBlocksPerSm of them per SM (what the ~127 registers of a
 // cell allow). A dense pass of at least two cells per resident thread

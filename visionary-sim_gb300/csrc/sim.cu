@@ -376,6 +376,20 @@ cudaError_t forEachPass(const LaunchCtx& c, const vsim_sim* s, bool limitOnly, c
     return e;
 }
 
+// Whether contact can touch anything: it is on, and there are bodies that may
+// meet or a body that may meet itself.
+bool contactMatters(const vsim_sim* s) {
+    return s->contact && s->surfaceCount > 0 && (s->selfContact || (!s->isolated && s->lat.size() > 1));
+}
+
+// Whether the frame runs in one launch (small_frame.cu).
+bool inOneLaunch(const vsim_sim* s) {
+    if (!inRows(s) || contactMatters(s) || s->nodeCount > kSmallNodes) return false;
+    for (uint32_t q = 0; q < kRowPasses; q++)
+        if (s->rowStart[q + 1] - s->rowStart[q] > 1) return false;
+    return true;
+}
+
 // stepper.js:101-108 with simulator.js:83's constraint order.
 cudaError_t encodeFrame(vsim_sim* s, cudaStream_t st, uint32_t steps, ContactMode mode = ContactMode::Solve,
                         Profiler* prof = nullptr) {
@@ -383,8 +397,20 @@ cudaError_t encodeFrame(vsim_sim* s, cudaStream_t st, uint32_t steps, ContactMod
     const StretchLengths lens = stretchLengths();
     const bool limited = anyStretch(s);
     const bool driving = !s->held.empty();
-    const bool contact = s->contact && s->surfaceCount > 0;
+    const bool contact = contactMatters(s);
     cudaError_t e;
+    if (!prof && steps > 0 && inOneLaunch(s)) {
+        SmallFrame f{};
+        std::copy(s->rowStart, s->rowStart + kRowPasses + 1, f.rowStart);
+        f.nodeCount = s->nodeCount;
+        f.activeCount = s->activeCount;
+        f.steps = steps;
+        f.iterations = s->iterations;
+        f.limited = limited;
+        f.driving = driving;
+        f.lens = lens;
+        return launchSmallFrame(st, s->d, f);
+    }
     auto begin = [&](int kind, uint32_t launches) {
         if (prof) prof->begin(kind, launches);
     };
@@ -435,7 +461,7 @@ cudaError_t encodeFrame(vsim_sim* s, cudaStream_t st, uint32_t steps, ContactMod
 uint64_t graphKey(const vsim_sim* s, uint32_t steps) {
     uint64_t k = steps;
     k = k * 31 + (s->held.empty() ? 0 : 1);
-    k = k * 31 + ((s->contact && s->surfaceCount > 0) ? 1 : 0);
+    k = k * 31 + (contactMatters(s) ? 1 : 0);
     k = k * 31 + s->iterations;
     k = k * 31 + (anyStretch(s) ? 1 : 0);
     k = k * 1031 + s->block;
@@ -1383,7 +1409,8 @@ uint32_t vsim_frame_launches(const vsim_sim* s, uint32_t steps) {
         for (int c = 0; c < 8; c++) passes += s->colorStart[c + 1] > s->colorStart[c] ? 1 : 0;
     uint32_t per = 1 + passes * s->iterations;
     if (anyStretch(s)) per += 3 * passes;
-    if (s->contact && s->surfaceCount > 0) per += contactKernels(s);
+    if (contactMatters(s)) per += contactKernels(s);
+    if (steps && inOneLaunch(s)) return 1;
     return steps ? 1 + per * steps : 0;
 }
 

@@ -6,7 +6,7 @@
 // inverse mass as the solver sees it (the reference's separate nodeInvMass
 // buffer, particles.js:206-215), so one 16-byte load brings a node's
 // position and weight together; every kernel that writes pos keeps w.
-#include "step_device.cuh"
+#include "row_pass.cuh"
 
 namespace vsim {
 
@@ -115,29 +115,10 @@ __global__ void __launch_bounds__(128) elasticQuadKernel(const uint4* __restrict
         if ((c & 3) == int(q)) pos[ids[c]] = withW(p[c], w[c]);
 }
 
-__device__ __forceinline__ void copyAsync16(float4* dst, const float4* src) {
-    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-}
-
-// A record's x, y and z in shared memory, read anew at every call (the
-// compiler would keep it in registers from its first use to its last).
-__device__ __forceinline__ V sharedXyz(const float4* record) {
-    float x, y, z, w;
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(x), "=f"(y), "=f"(z), "=f"(w)
-                 : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(record))));
-    return mk(x, y, z);
-}
-
 // project.wgsl:35-184, two colours a launch: a block per group of runs (see
-// kRowBlock), a thread per even cell, then a thread per odd cell. The odd
-// cells' sixteen node records are copied to shared memory (cp.async) while the
-// even cells are solved; each even cell then puts the faces that an odd cell
-// holds into that cell's copy, and stores the others. So every node is loaded
-// about once and stored once for the two colours, and a substep has four
-// dependent launches where it had eight. No two blocks share a node: the
-// update is in place.
+// kRowBlock), a thread per even cell, then a thread per odd cell (rowGroup). A
+// substep has four dependent launches where it had eight. No two blocks share
+// a node: the update is in place.
 //
 // What bounds it: at a pass under a wave of blocks, the chain of one launch
 // (~1 us), the loads (~0.6 us) and two cells' arithmetic (1.3 us each, see
@@ -164,108 +145,17 @@ __global__ void __launch_bounds__(kRowBlock, EARLY ? 3 : 2) elasticRowKernel(con
                                                                              float4* __restrict__ pos,
                                                                              const float4* __restrict__ prevState,
                                                                              StretchLengths lens) {
-    __shared__ float4 stage[8][kRowBlock];    // the odd cells' positions, by corner
-    __shared__ float4 before[2][8][kRowBlock];  // the even and the odd cells' previous positions
-    const uint32_t t = threadIdx.x;
-    const uint4* group = groups + size_t(blockIdx.x) * kRowGroup;
-    const uint4 even = group[t], odd = group[kRowBlock + t];
-    auto takesPart = [&](uint4 e, float maxStretch) {
-        return (e.y & kRowCell) && bodyActive[e.y & ~kRowCell] && (WORK != RowWork::kLimit || maxStretch > 1.0f);
-    };
-    const uint32_t oddBody = odd.y & ~kRowCell;
-    uint32_t body = even.y & ~kRowCell;  // an empty slot names body 0
-    CellConsts k = cellConsts(bodies + body);
-    bool solve = takesPart(even, k.maxStretch);
-    const bool solveOdd = takesPart(odd, bodies[oddBody].maxStretch);
-    constexpr uint32_t kStride = (1u << kRowStrideBits) - 1;
-    const uint32_t nearOdd = even.z >> kRowStrideBits & 0xffu, farOdd = even.z >> (kRowStrideBits + 8) & 0xffu;
-    uint4 cell = make_uint4(even.x, body, even.z & kStride, even.w);
-    uint32_t ids[8];
-    cornerNodes(cell, ids);
-    pdlWait();
-    if (EARLY) pdlLaunchNext();
-    V p[8];
-    float w[8];
-    if (solve) {
-#pragma unroll
-        for (int c = 0; c < 8; c++) {
-            copyAsync16(&before[0][c][t], prevState + ids[c]);
-            const float4 P = pos[ids[c]];
-            p[c] = xyz(P);
-            w[c] = P.w;
-        }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    if (solveOdd) {
-        uint32_t at[8];
-        cornerNodes(make_uint4(odd.x, 0, odd.z & kStride, odd.w), at);
-#pragma unroll
-        for (int c = 0; c < 8; c++) {
-            copyAsync16(&stage[c][t], pos + at[c]);
-            copyAsync16(&before[1][c][t], prevState + at[c]);
-        }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 1;" ::: "memory");  // the even cells' copies have landed
-    // One copy of the projection's code for both cells: two would not stay in
-    // the instruction cache.
-#pragma unroll 1
-    for (uint32_t second = 0; second < 2; second++) {
-        if (second) {
-            asm volatile("cp.async.wait_all;" ::: "memory");
-            __syncthreads();  // every copy has landed
-            if (solve) {
-#pragma unroll
-                for (int c = 0; c < 8; c++) {
-                    const uint32_t holder = c & 1 ? farOdd : nearOdd;
-                    const float4 P = withW(p[c], w[c]);
-                    // the odd cell's face on the other side of the plane
-                    if (holder != kNoRowCell)
-                        stage[c ^ 1][holder] = P;
-                    else
-                        pos[ids[c]] = P;
-                }
-            }
-            __syncthreads();
-            solve = solveOdd;
-            cell.x = odd.x;
-            // The even cell's body and strides serve but at a few cells: the
-            // next body's first ones, a group's unpaired ones.
-            if (solve && (oddBody != body || !(even.y & kRowCell))) {
-                body = oddBody;
-                k = cellConsts(bodies + body);
-                const uint4 again = group[kRowBlock + t];
-                cell = make_uint4(again.x, body, again.z, again.w);
-            }
-            cornerNodes(cell, ids);
-            if (solve) {
-#pragma unroll
-                for (int c = 0; c < 8; c++) {
-                    const float4 P = stage[c][t];
-                    p[c] = xyz(P);
-                    w[c] = P.w;
-                }
-            }
-        }
-        if (!solve) continue;
-        // The previous positions stay in shared memory, read where they are
-        // used: 24 registers fewer, which is a block more an SM.
-        auto prev = [&](int c) { return sharedXyz(&before[second][c][t]); };
-        if (WORK != RowWork::kLimit && !projectCellInRange(p, prev, w, k)) {
-            if (second) {
-#pragma unroll
-                for (int c = 0; c < 8; c++) pos[ids[c]] = stage[c][t];
-            }
-            projectCellAgain(cell, bodies + body, pos, prevState);
-#pragma unroll
-            for (int c = 0; c < 8; c++) p[c] = xyz(pos[ids[c]]);
-        }
-        if (WORK != RowWork::kProject && k.maxStretch > 1.0f) limitStretch(p, w, k, lens);
-    }
-    if (!EARLY) pdlLaunchNext();
-    if (!solve) return;
-#pragma unroll
-    for (int c = 0; c < 8; c++) pos[ids[c]] = withW(p[c], w[c]);
+    __shared__ RowShared shared;
+    rowGroup(
+        groups + size_t(blockIdx.x) * kRowGroup, bodies, bodyActive, pos, prevState, lens, WORK != RowWork::kLimit,
+        WORK != RowWork::kProject, shared,
+        [] {
+            pdlWait();
+            if (EARLY) pdlLaunchNext();
+        },
+        [] {
+            if (!EARLY) pdlLaunchNext();
+        });
 }
 
 // The colour pass for passes much larger than the GPU: each thread solves
