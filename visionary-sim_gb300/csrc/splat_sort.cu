@@ -208,26 +208,41 @@ cudaError_t launchSplatDeform(cudaStream_t st, const SplatState& s, const float4
 // - one launch counts every pass's digits over all the keys at once (a
 //   pass's digit totals do not depend on the order earlier passes leave);
 // - then one launch per pass. Each block takes the next tile from a ticket,
-//   so tiles start in order; it ranks its 4096 keys per digit (every warp
-//   its 512 with __match_any_sync) and publishes the tile's count of each
-//   digit in a status word (count and a flag packed in 32 bits, so one store
-//   carries both). Then each digit's thread walks back over the tiles before
-//   it, adding their counts until it meets a word that already holds an
-//   inclusive prefix, and publishes the tile's own. A tile waits only on
-//   tiles that started before it, which publish their counts without
-//   waiting on anything, so every walk ends. With the digit's global start
-//   (the histogram, scanned) the block writes the tile out in runs that are
-//   contiguous per digit.
+//   so tiles start in order; it ranks its keys per digit (a warp its own,
+//   rankKeys) and publishes the tile's count of each digit in a status word
+//   (count and a flag packed in 32 bits, so one store carries both). While
+//   the words of the tiles before it arrive, it sorts the tile in shared
+//   memory; then each digit's thread walks back over those tiles, adding
+//   their counts until it meets a word that already holds an inclusive
+//   prefix, and publishes the tile's own. A tile waits only on tiles that
+//   started before it, which publish their counts without waiting on
+//   anything, so every walk ends. The block writes the tile out in runs that
+//   are contiguous per digit.
+//
+// What bounds a pass is instructions, most of them the ranking's ballots (20M
+// keys: 124 warp instructions per 32 keys, the ALU pipe 60 % and the
+// shared-memory pipe 45 % active, 2 TB/s of DRAM). Against ranking with
+// __match_any_sync, key by key with its load and its counter's round trip,
+// looking back one word a trip before the tile is sorted, and two look-ups a
+// key: 20M keys in 492 us where they took 746, 1M in 52 where 83.
+//
+// The tile: past two tiles of 4096 keys an SM the passes take several waves,
+// and fewer, larger tiles are worth the longer first one (20M keys: 582 us
+// with tiles of 4096 keys, 500 with 6144 and 8192, whose keys spill; 4M: 141,
+// 130 and 139). Within one wave a tile's latency is the pass (1M keys: 52, 61
+// and 70 us).
 //
 // Tiles and ranks follow input order, so each pass -- and the sort -- is
 // stable. The status words, digit totals and tickets are cleared by one
 // memset at the start of a sort; every other scratch word is written before
 // it is read.
 
-constexpr uint32_t kSortThreads = 256;
-constexpr uint32_t kSortItems = 16;
-constexpr uint32_t kSortTile = kSortThreads * kSortItems;  // 4096 keys
-constexpr uint32_t kWarps = kSortThreads / 32;
+constexpr uint32_t kCountThreads = 256;
+constexpr uint32_t kSortThreads = 512;
+constexpr uint32_t kSortItems = 8;        // keys a thread while the tiles are one wave
+constexpr uint32_t kSortLargeItems = 12;  // and past that
+constexpr uint32_t kSortTile = kSortThreads * kSortItems;            // 4096 keys
+constexpr uint32_t kSortLargeTile = kSortThreads * kSortLargeItems;  // 6144
 constexpr uint32_t kSortMaxPasses = 4;
 constexpr uint32_t kStatusCount = 1u << 30;     // the word holds the tile's own count
 constexpr uint32_t kStatusPrefix = 2u << 30;    // the word holds the inclusive prefix
@@ -237,21 +252,17 @@ constexpr uint32_t kLookbackSpinLimit = 1u << 22;
 namespace {
 constexpr size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 constexpr uint32_t tilesOf(uint32_t n) { return (n + kSortTile - 1) / kSortTile; }
-// Cleared at the start of a sort: per pass, a status word per (tile, digit);
-// the digit totals of every pass; a ticket per pass and the failure word.
-constexpr size_t sortStatusBytes(uint32_t n) { return align256(size_t(kSortMaxPasses) * tilesOf(n) * 256 * 4); }
+// Cleared at the start of a sort: the digit totals of every pass, a ticket
+// per pass and the failure word; then, per pass, a status word per (tile,
+// digit).
+constexpr size_t kSortHeadBytes = align256(kSortMaxPasses * 256 * 4) + 256;
 constexpr size_t sortClearedBytes(uint32_t n) {
-    return sortStatusBytes(n) + align256(kSortMaxPasses * 256 * 4) + 256;
+    return kSortHeadBytes + align256(size_t(kSortMaxPasses) * tilesOf(n) * 256 * 4);
 }
 constexpr size_t sortTempBytes(uint32_t n) { return 4 * align256(size_t(n) * 4) + sortClearedBytes(n); }
 }  // namespace
 
 size_t radixSortTempBytes(uint32_t n) { return sortTempBytes(n); }
-
-uint32_t radixSortLaunches(uint32_t n, uint32_t keyBits) {
-    if (n == 0) return 0;
-    return 1 + (keyBits + 7) / 8;  // the digit counts, then one launch per pass
-}
 
 __device__ __forceinline__ uint32_t loadRelaxed(const uint32_t* p) {
     uint32_t v;
@@ -264,11 +275,11 @@ __device__ __forceinline__ void storeRelaxed(uint32_t* p, uint32_t v) {
 
 // Every pass's digit counts over all keys: per block in shared memory, then
 // added into totals[pass * 256 + digit].
-__global__ void __launch_bounds__(kSortThreads) sortDigitCountKernel(const uint32_t* __restrict__ keys, uint32_t n,
+__global__ void __launch_bounds__(kCountThreads) sortDigitCountKernel(const uint32_t* __restrict__ keys, uint32_t n,
                                                                      uint32_t keyBits,
                                                                      uint32_t* __restrict__ totals) {
     __shared__ uint32_t bins[kSortMaxPasses * 256];
-    for (uint32_t i = threadIdx.x; i < kSortMaxPasses * 256; i += kSortThreads) bins[i] = 0;
+    for (uint32_t i = threadIdx.x; i < kSortMaxPasses * 256; i += kCountThreads) bins[i] = 0;
     pdlWait();  // the keys come from the kernel before
     pdlLaunchNext();
     __syncthreads();
@@ -281,26 +292,82 @@ __global__ void __launch_bounds__(kSortThreads) sortDigitCountKernel(const uint3
             atomicAdd(&bins[p * 256 + ((k >> (8 * p)) & ((1u << bits) - 1u))], 1u);
         }
     };
-    const uint32_t stride = gridDim.x * kSortThreads;
+    const uint32_t stride = gridDim.x * kCountThreads;
     // four keys per load where the keys start on a 16-byte boundary
     const uint32_t quads = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0 ? n / 4 : 0;
     const uint4* k4 = reinterpret_cast<const uint4*>(keys);
-    for (uint32_t i = blockIdx.x * kSortThreads + threadIdx.x; i < quads; i += stride) {
+    for (uint32_t i = blockIdx.x * kCountThreads + threadIdx.x; i < quads; i += stride) {
         const uint4 q = k4[i];
         count(q.x);
         count(q.y);
         count(q.z);
         count(q.w);
     }
-    for (uint32_t i = 4 * quads + blockIdx.x * kSortThreads + threadIdx.x; i < n; i += stride) count(keys[i]);
+    for (uint32_t i = 4 * quads + blockIdx.x * kCountThreads + threadIdx.x; i < n; i += stride) count(keys[i]);
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < passes * 256; i += kSortThreads)
+    for (uint32_t i = threadIdx.x; i < passes * 256; i += kCountThreads)
         if (bins[i]) atomicAdd(&totals[i], bins[i]);
 }
 
-// Block-wide exclusive scan of one value per thread (256 threads); returns
-// the block total through `total`.
-__device__ __forceinline__ uint32_t blockExclusiveScan(uint32_t v, uint32_t* warpSums, uint32_t& total) {
+// The lanes of `active` whose 8-bit digit equals this lane's: one ballot a bit.
+__device__ __forceinline__ uint32_t peersOf(uint32_t digit, uint32_t active) {
+    uint32_t peers = active;
+#pragma unroll
+    for (uint32_t b = 0; b < 8; b++) {
+        const bool bit = digit >> b & 1u;
+        const uint32_t set = __ballot_sync(0xffffffffu, bit);
+        peers &= bit ? set : ~set;
+    }
+    return peers;
+}
+
+// Ranks a warp's keys of each digit: key r of a lane comes after the keys
+// before it in (r, lane) order, and rank(r) counts those of its digit. `hist`,
+// the warp's 256 counters, zero before, holds its digit counts after. The
+// lowest lane of each digit adds for all of its peers, in order of r, and
+// hands them the count before; in two loops, so that no key's ballots wait on
+// the counters' round trip for the one before. A rank fits 16 bits, and so
+// does what the second loop needs of the first: two keys share a register.
+template <uint32_t ITEMS>
+struct Ranks {
+    uint32_t packed[(ITEMS + 1) / 2];
+    __device__ __forceinline__ uint32_t operator()(uint32_t r) const { return packed[r / 2] >> 16 * (r % 2) & 0xffffu; }
+    __device__ __forceinline__ void set(uint32_t r, uint32_t v) {
+        packed[r / 2] = r % 2 ? (packed[r / 2] & 0xffffu) | v << 16 : (packed[r / 2] & 0xffff0000u) | v;
+    }
+};
+
+template <bool FULL, uint32_t ITEMS>
+__device__ __forceinline__ void rankKeys(const uint32_t (&key)[ITEMS], uint32_t first, uint32_t n, uint32_t shift,
+                                         uint32_t mask, uint32_t* hist, Ranks<ITEMS>& rank) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    uint32_t before[ITEMS];
+#pragma unroll
+    for (uint32_t r = 0; r < (ITEMS + 1) / 2; r++) rank.packed[r] = 0;
+#pragma unroll
+    for (uint32_t r = 0; r < ITEMS; r++) {
+        const bool valid = FULL || first + r * 32 + lane < n;
+        const uint32_t digit = key[r] >> shift & mask;
+        const uint32_t peers = peersOf(digit, FULL ? 0xffffffffu : __ballot_sync(0xffffffffu, valid));
+        before[r] = 0;
+        if (valid && (peers & lt) == 0) before[r] = atomicAdd(hist + digit, uint32_t(__popc(peers)));
+        // A lane past the end hands itself its zero.
+        const uint32_t leader = valid ? __ffs(int(peers)) - 1 : lane;
+        rank.set(r, leader | __popc(peers & lt) << 8);
+        asm volatile("" : "+r"(rank.packed[r / 2]));  // packed now, not where it is read
+        __syncwarp();
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < ITEMS; r++) {
+        const uint32_t info = rank(r);
+        rank.set(r, __shfl_sync(0xffffffffu, before[r], int(info & 31u)) + (info >> 8));
+    }
+}
+
+// The exclusive scan of one value a thread over the first 256 threads of a
+// block; all of its threads call it.
+__device__ __forceinline__ uint32_t scanDigits(uint32_t v, uint32_t* warpSums) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t incl = v;
 #pragma unroll
@@ -308,165 +375,185 @@ __device__ __forceinline__ uint32_t blockExclusiveScan(uint32_t v, uint32_t* war
         const uint32_t u = __shfl_up_sync(0xffffffffu, incl, d);
         if (lane >= uint32_t(d)) incl += u;
     }
-    if (lane == 31) warpSums[warp] = incl;
+    if (lane == 31 && warp < 8) warpSums[warp] = incl;
     __syncthreads();
-    if (warp == 0) {
-        const uint32_t s = lane < kWarps ? warpSums[lane] : 0;
-        uint32_t sc = s;
+    uint32_t base = 0;
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t u = __shfl_up_sync(0xffffffffu, sc, d);
-            if (lane >= uint32_t(d)) sc += u;
-        }
-        if (lane < kWarps) warpSums[lane] = sc - s;
-        if (lane == kWarps - 1) warpSums[kWarps] = sc;
-    }
-    __syncthreads();
-    total = warpSums[kWarps];
-    const uint32_t out = warpSums[warp] + incl - v;
-    __syncthreads();
-    return out;
+    for (uint32_t w = 0; w < 7; w++)
+        if (w < warp) base += warpSums[w];
+    return base + incl - v;
 }
 
-// One pass: rank a tile, find its digits' global offsets by decoupled
-// look-back, scatter. `status` is this pass's (tile, digit) words, `totals`
-// its 256 digit counts over all keys.
-__device__ __forceinline__ void sortPass(const uint32_t* __restrict__ keysIn, const uint32_t* __restrict__ valsIn,
+template <uint32_t ITEMS>
+struct PassShared {
+    uint2 pairs[kSortThreads * ITEMS];  // key, value
+    uint32_t warpHist[kSortThreads / 32][256];
+    uint32_t part[kSortThreads / 256][256];  // digit counts over eight warps each
+    uint32_t place[256];                // what takes a key's place in the tile to its place in the output
+    uint32_t warpSums[2][8];
+    uint32_t tile;
+};
+
+// One pass over one tile: rank it, find its digits' global offsets by
+// decoupled look-back, scatter. `status` is the pass's (tile, digit) words,
+// `totals` its 256 digit counts over all keys.
+template <bool FULL, uint32_t ITEMS>
+__device__ __forceinline__ void sortTile(PassShared<ITEMS>& sh, uint32_t tile,
+                                         const uint32_t* __restrict__ keysIn, const uint32_t* __restrict__ valsIn,
                                          uint32_t n, uint32_t shift, uint32_t mask,
                                          const uint32_t* __restrict__ totals, uint32_t* __restrict__ status,
-                                         uint32_t* __restrict__ ticket, uint32_t* __restrict__ error,
-                                         uint32_t* __restrict__ keysOut, uint32_t* __restrict__ valsOut) {
-    __shared__ uint32_t sKeys[kSortTile];
-    __shared__ uint32_t sVals[kSortTile];
-    __shared__ uint32_t warpHist[kWarps][256];
-    __shared__ uint32_t digitStart[256];
-    __shared__ uint32_t globalStart[256];
-    __shared__ uint32_t warpSums[kWarps + 1];
-    __shared__ uint32_t sTile;
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+                                         uint32_t* __restrict__ error, uint32_t* __restrict__ keysOut,
+                                         uint32_t* __restrict__ valsOut) {
+    constexpr uint32_t kTile = kSortThreads * ITEMS;
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const uint32_t tileBase = tile * kTile;
+    const uint32_t first = tileBase + warp * 32 * ITEMS;
+    uint32_t key[ITEMS], val[ITEMS];
+    Ranks<ITEMS> rank;
+    const uint32_t* keyAt = keysIn + first + lane;
+#pragma unroll
+    for (uint32_t r = 0; r < ITEMS; r++) key[r] = FULL || first + r * 32 + lane < n ? keyAt[r * 32] : 0u;
+    rankKeys<FULL, ITEMS>(key, first, n, shift, mask, sh.warpHist[warp], rank);
+    __syncthreads();
+    if (valsIn) {
+        const uint32_t* valAt = valsIn + first + lane;
+#pragma unroll
+        for (uint32_t r = 0; r < ITEMS; r++) val[r] = FULL || first + r * 32 + lane < n ? valAt[r * 32] : 0u;
+    } else {
+#pragma unroll
+        for (uint32_t r = 0; r < ITEMS; r++) val[r] = first + r * 32 + lane;
+    }
+    // Per digit, eight warps' counts a thread: the tile's count of the digit,
+    // and where each warp's keys of it start in the tile.
+    const uint32_t digit = t & 255, part = t >> 8;
+    constexpr uint32_t kParts = kSortThreads / 256, kEach = 8;
+    uint32_t of[kEach], count = 0, run = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kEach; w++) count += of[w] = sh.warpHist[part * kEach + w][digit];
+    if (kParts > 1) {
+        sh.part[part][digit] = count;
+        __syncthreads();
+        count = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < kParts; q++) {
+            const uint32_t c = sh.part[q][digit];
+            if (q < part) run += c;
+            count += c;
+        }
+    }
+    // The first tile starts from the digit's place in the whole output, so
+    // that every prefix that follows holds it.
+    uint32_t before = 0;
+    if (tile == 0) {
+        before = scanDigits(t < 256 ? totals[t] : 0u, sh.warpSums[1]);
+        if (t < 256) storeRelaxed(status + t, kStatusPrefix | (before + count));
+    } else if (t < 256) {
+        storeRelaxed(status + size_t(tile) * 256 + t, kStatusCount | count);
+    }
+    uint32_t start = scanDigits(t < 256 ? count : 0u, sh.warpSums[0]);
+    if (kParts > 1) {
+        if (t < 256) sh.place[t] = start;
+        __syncthreads();
+        start = sh.place[digit];
+    }
+    run += start;
+#pragma unroll
+    for (uint32_t w = 0; w < kEach; w++) {
+        sh.warpHist[part * kEach + w][digit] = run;
+        run += of[w];
+    }
+    __syncthreads();
+    // The digits again, from a shift that the compiler takes for another:
+    // kept from the ranking they would cost a register a key.
+    uint32_t shiftAgain = shift;
+    asm volatile("" : "+r"(shiftAgain));
+#pragma unroll
+    for (uint32_t r = 0; r < ITEMS; r++) {
+        if (FULL || first + r * 32 + lane < n)
+            sh.pairs[sh.warpHist[warp][key[r] >> shiftAgain & mask] + rank(r)] = make_uint2(key[r], val[r]);
+    }
+    if (t < 256) {
+        // Decoupled look-back over the tiles before this one, whose words
+        // have had the scatter's time to be published; several words a trip.
+        constexpr uint32_t kTrip = 4;
+        uint32_t polls = 0;
+        bool found = tile == 0;
+        for (uint32_t j = tile; !found && j > 0;) {
+            uint32_t word[kTrip], taken = 0;
+#pragma unroll
+            for (uint32_t k = 0; k < kTrip; k++)
+                word[k] = k < j ? loadRelaxed(status + size_t(j - 1 - k) * 256 + t) : 0u;
+            bool more = true;
+#pragma unroll
+            for (uint32_t k = 0; k < kTrip; k++) {
+                more = more && (word[k] & ~kStatusValue) != 0;  // else tile j - 1 - k has not published yet
+                if (!more) continue;
+                before += word[k] & kStatusValue;
+                taken++;
+                found = (word[k] & ~kStatusValue) == kStatusPrefix;
+                more = !found;
+            }
+            j -= taken;
+            if (taken == 0) {
+                if (++polls > kLookbackSpinLimit) {
+                    atomicOr(error, 1u);
+                    break;
+                }
+                __nanosleep(32);
+            }
+        }
+        if (tile > 0) storeRelaxed(status + size_t(tile) * 256 + t, kStatusPrefix | (before + count));
+        sh.place[t] = before - start;
+    }
+    __syncthreads();
+    const uint32_t held = FULL ? kTile : n - tileBase;
+    uint32_t j = t;
+#pragma unroll 4
+    for (uint32_t r = 0; r < ITEMS; r++, j += kSortThreads) {
+        if (FULL || j < held) {
+            const uint2 pair = sh.pairs[j];
+            const uint32_t out = sh.place[pair.x >> shiftAgain & mask] + j;
+            if (keysOut) keysOut[out] = pair.x;
+            valsOut[out] = pair.y;
+        }
+    }
+}
+
+template <uint32_t ITEMS>
+__global__ void __launch_bounds__(kSortThreads, 2) sortPassKernel(const uint32_t* __restrict__ keysIn,
+                                                                  const uint32_t* __restrict__ valsIn, uint32_t n,
+                                                                  uint32_t shift, uint32_t mask,
+                                                                  const uint32_t* __restrict__ totals,
+                                                                  uint32_t* __restrict__ status,
+                                                                  uint32_t* __restrict__ ticket,
+                                                                  uint32_t* __restrict__ error,
+                                                                  uint32_t* __restrict__ keysOut,
+                                                                  uint32_t* __restrict__ valsOut) {
+    extern __shared__ __align__(16) unsigned char raw[];
+    auto& sh = *reinterpret_cast<PassShared<ITEMS>*>(raw);
     // The ticket counter was cleared before the sort's first launch, which
     // this one follows in stream order: safe to take before the wait.
-    if (threadIdx.x == 0) sTile = atomicAdd(ticket, 1u);
-    for (uint32_t i = threadIdx.x; i < kWarps * 256; i += kSortThreads) (&warpHist[0][0])[i] = 0;
+    if (threadIdx.x == 0) sh.tile = atomicAdd(ticket, 1u);
+    for (uint32_t i = threadIdx.x; i < kSortThreads / 32 * 256; i += kSortThreads) (&sh.warpHist[0][0])[i] = 0;
     pdlWait();  // the keys and totals come from the kernels before
     pdlLaunchNext();
     __syncthreads();
-    const uint32_t tile = sTile;
-    const uint32_t tileBase = tile * kSortTile;
-    const uint32_t warpBase = tileBase + warp * 32 * kSortItems;
-    const uint32_t lt = (1u << lane) - 1u;
-    uint32_t key[kSortItems], val[kSortItems], rank[kSortItems];
-#pragma unroll
-    for (uint32_t r = 0; r < kSortItems; r++) {
-        const uint32_t idx = warpBase + r * 32 + lane;
-        const bool valid = idx < n;
-        key[r] = valid ? keysIn[idx] : 0u;
-        val[r] = valid ? (valsIn ? valsIn[idx] : idx) : 0u;
-        const uint32_t digit = valid ? (key[r] >> shift) & mask : 256u;
-        const uint32_t peers = __match_any_sync(0xffffffffu, digit);
-        const uint32_t before = valid ? warpHist[warp][digit] : 0u;
-        __syncwarp();
-        if (valid && (peers & lt) == 0) warpHist[warp][digit] = before + __popc(peers);
-        __syncwarp();
-        rank[r] = before + __popc(peers & lt);
-    }
-    __syncthreads();
-    {
-        const uint32_t d = threadIdx.x;
-        // Per digit: exclusive prefix over warps, and the tile's count.
-        uint32_t count = 0;
-#pragma unroll
-        for (uint32_t w = 0; w < kWarps; w++) {
-            const uint32_t c = warpHist[w][d];
-            warpHist[w][d] = count;
-            count += c;
-        }
-        uint32_t* mine = status + size_t(tile) * 256 + d;
-        storeRelaxed(mine, (tile == 0 ? kStatusPrefix : kStatusCount) | count);
-        // Decoupled look-back over the tiles before this one.
-        uint32_t before = 0;
-        if (tile > 0) {
-            uint32_t j = tile - 1, polls = 0;
-            while (true) {
-                const uint32_t word = loadRelaxed(status + size_t(j) * 256 + d);
-                if ((word & ~kStatusValue) == 0) {  // tile j has not published yet
-                    if (++polls > kLookbackSpinLimit) {
-                        atomicOr(error, 1u);
-                        break;
-                    }
-                    __nanosleep(32);
-                    continue;
-                }
-                before += word & kStatusValue;
-                if ((word & ~kStatusValue) == kStatusPrefix || j == 0) break;
-                j--;
-            }
-            storeRelaxed(mine, kStatusPrefix | (before + count));
-        }
-        uint32_t total;
-        digitStart[d] = blockExclusiveScan(count, warpSums, total);
-        const uint32_t digitBase = blockExclusiveScan(totals[d], warpSums, total);
-        globalStart[d] = digitBase + before;
-    }
-    __syncthreads();
-#pragma unroll
-    for (uint32_t r = 0; r < kSortItems; r++) {
-        const uint32_t idx = warpBase + r * 32 + lane;
-        if (idx < n) {
-            const uint32_t digit = (key[r] >> shift) & mask;
-            const uint32_t slot = digitStart[digit] + warpHist[warp][digit] + rank[r];
-            sKeys[slot] = key[r];
-            sVals[slot] = val[r];
-        }
-    }
-    __syncthreads();
-    const uint32_t count = n - tileBase < kSortTile ? n - tileBase : kSortTile;
-    for (uint32_t j = threadIdx.x; j < count; j += kSortThreads) {
-        const uint32_t k = sKeys[j];
-        const uint32_t digit = (k >> shift) & mask;
-        const uint32_t out = globalStart[digit] + (j - digitStart[digit]);
-        if (keysOut) keysOut[out] = k;
-        valsOut[out] = sVals[j];
-    }
-}
-
-// The pass as two kernels: sortPassKernel at the registers the compiler
-// picks (86: two blocks an SM), sortPassWideKernel squeezed to 80 so that
-// three fit. The second is faster once the tiles take several waves (20M
-// keys: 27.4 against 23.6 G keys/s), slower within one wave, where each
-// tile's latency is the pass (1M keys: 0.096 against 0.080 ms a sort).
-__global__ void __launch_bounds__(kSortThreads) sortPassKernel(const uint32_t* __restrict__ keysIn,
-                                                               const uint32_t* __restrict__ valsIn, uint32_t n,
-                                                               uint32_t shift, uint32_t mask,
-                                                               const uint32_t* __restrict__ totals,
-                                                               uint32_t* __restrict__ status,
-                                                               uint32_t* __restrict__ ticket,
-                                                               uint32_t* __restrict__ error,
-                                                               uint32_t* __restrict__ keysOut,
-                                                               uint32_t* __restrict__ valsOut) {
-    sortPass(keysIn, valsIn, n, shift, mask, totals, status, ticket, error, keysOut, valsOut);
-}
-
-__global__ void __launch_bounds__(kSortThreads, 3) sortPassWideKernel(const uint32_t* __restrict__ keysIn,
-                                                                      const uint32_t* __restrict__ valsIn,
-                                                                      uint32_t n, uint32_t shift, uint32_t mask,
-                                                                      const uint32_t* __restrict__ totals,
-                                                                      uint32_t* __restrict__ status,
-                                                                      uint32_t* __restrict__ ticket,
-                                                                      uint32_t* __restrict__ error,
-                                                                      uint32_t* __restrict__ keysOut,
-                                                                      uint32_t* __restrict__ valsOut) {
-    sortPass(keysIn, valsIn, n, shift, mask, totals, status, ticket, error, keysOut, valsOut);
+    const uint32_t tile = sh.tile;
+    if (n - tile * (kSortThreads * ITEMS) >= kSortThreads * ITEMS)
+        sortTile<true>(sh, tile, keysIn, valsIn, n, shift, mask, totals, status, error, keysOut, valsOut);
+    else
+        sortTile<false>(sh, tile, keysIn, valsIn, n, shift, mask, totals, status, error, keysOut, valsOut);
 }
 
 namespace {
 // A sort kernel launched with programmatic dependent launch: its blocks may
 // start while the kernel before finishes, and wait (pdlWait) before reading.
 template <class... KArgs, class... Args>
-cudaError_t pdl(void (*kernel)(KArgs...), uint32_t grid, cudaStream_t st, Args... args) {
+cudaError_t pdl(void (*kernel)(KArgs...), uint32_t grid, uint32_t threads, size_t bytes, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kSortThreads);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = bytes;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -477,12 +564,16 @@ cudaError_t pdl(void (*kernel)(KArgs...), uint32_t grid, cudaStream_t st, Args..
 }
 }  // namespace
 
+uint32_t radixSortLaunches(uint32_t n, uint32_t keyBits) {
+    if (n == 0) return 0;
+    return 1 + (keyBits + 7) / 8;  // the digit counts, then one launch per pass
+}
+
 cudaError_t radixSortU32(const uint32_t* keys, uint32_t* order, uint32_t n, uint32_t keyBits, void* temp,
                          size_t tempBytes, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
     if (tempBytes < radixSortTempBytes(n) || n > kStatusValue || keyBits < 1 || keyBits > 32)
         return cudaErrorInvalidValue;
-    const uint32_t tiles = tilesOf(n);
     char* p = static_cast<char*>(temp);
     const size_t vec = align256(size_t(n) * 4);
     uint32_t* keysA = reinterpret_cast<uint32_t*>(p);
@@ -490,18 +581,21 @@ cudaError_t radixSortU32(const uint32_t* keys, uint32_t* order, uint32_t n, uint
     uint32_t* valsA = reinterpret_cast<uint32_t*>(p + 2 * vec);
     uint32_t* valsB = reinterpret_cast<uint32_t*>(p + 3 * vec);
     char* cleared = p + 4 * vec;
-    uint32_t* status = reinterpret_cast<uint32_t*>(cleared);
-    uint32_t* totals = reinterpret_cast<uint32_t*>(cleared + sortStatusBytes(n));
-    uint32_t* tickets = reinterpret_cast<uint32_t*>(cleared + sortStatusBytes(n) + align256(kSortMaxPasses * 256 * 4));
+    uint32_t* totals = reinterpret_cast<uint32_t*>(cleared);
+    uint32_t* tickets = totals + kSortMaxPasses * 256;
     uint32_t* error = tickets + kSortMaxPasses;
+    uint32_t* status = reinterpret_cast<uint32_t*>(cleared + kSortHeadBytes);
     const uint32_t passes = (keyBits + 7) / 8;
     cudaError_t e;
-    if ((e = cudaMemsetAsync(cleared, 0, sortClearedBytes(n), st))) return e;
     int device = 0, sms = 0;
-    if ((e = cudaGetDevice(&device)) || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)))
-        return e;
-    const uint32_t countGrid = std::min<uint32_t>(tiles, 2u * uint32_t(sms));
-    if ((e = pdl(sortDigitCountKernel, countGrid, st, keys, n, keyBits, totals))) return e;
+    if ((e = cudaGetDevice(&device))) return e;
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device))) return e;
+    const bool oneWave = (n + kSortTile - 1) / kSortTile <= 2u * uint32_t(sms);
+    const uint32_t tile = oneWave ? kSortTile : kSortLargeTile, tiles = (n + tile - 1) / tile;
+    if ((e = cudaMemsetAsync(cleared, 0, kSortHeadBytes + size_t(passes) * tiles * 256 * 4, st))) return e;
+    // Eight blocks an SM, all that fit: the counters' round trips bound it.
+    const uint32_t countGrid = std::min<uint32_t>(tiles, 8u * uint32_t(sms));
+    if ((e = pdl(sortDigitCountKernel, countGrid, kCountThreads, 0, st, keys, n, keyBits, totals))) return e;
     const uint32_t* kin = keys;
     const uint32_t* vin = nullptr;
     for (uint32_t pass_ = 0; pass_ < passes; pass_++) {
@@ -511,11 +605,16 @@ cudaError_t radixSortU32(const uint32_t* keys, uint32_t* order, uint32_t n, uint
         const bool last = pass_ + 1 == passes;
         uint32_t* kout = last ? nullptr : (pass_ % 2 == 0 ? keysA : keysB);
         uint32_t* vout = last ? order : (pass_ % 2 == 0 ? valsA : valsB);
-        auto pass = [&](auto kernel) {
-            return pdl(kernel, tiles, st, kin, vin, n, shift, mask, (const uint32_t*)(totals + 256 * pass_),
-                       status + size_t(pass_) * tiles * 256, tickets + pass_, error, kout, vout);
+        auto pass = [&](auto kernel, size_t bytes) {
+            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
+            if (e) return e;
+            return pdl(kernel, tiles, kSortThreads, bytes, st, kin, vin, n, shift, mask,
+                       (const uint32_t*)(totals + 256 * pass_), status + size_t(pass_) * tiles * 256,
+                       tickets + pass_, error, kout, vout);
         };
-        if ((e = tiles > 2u * uint32_t(sms) ? pass(sortPassWideKernel) : pass(sortPassKernel))) return e;
+        e = oneWave ? pass(sortPassKernel<kSortItems>, sizeof(PassShared<kSortItems>))
+                    : pass(sortPassKernel<kSortLargeItems>, sizeof(PassShared<kSortLargeItems>));
+        if (e) return e;
         kin = kout;
         vin = vout;
     }
