@@ -14,10 +14,11 @@
 //      Gaussians whose bracket can hold an extreme;
 //   2. the grid laid out on the host from the bounds (gridForBounds,
 //      voxelize.js:40-67);
-//   3. stamp: a thread per Gaussian marks its centre cell and tests the
-//      cells of its box against the ellipsoid (stampCloud, :138-178), box
-//      edges and samples decided in float unless too close to call; a box
-//      of more than kInlineBoxCells cells is handed to a block instead;
+//   3. stamp: a thread per Gaussian marks its centre cell and looks whether
+//      its box has a cell that is still empty; those that do are tested cell
+//      by cell against the ellipsoid (stampCloud, :138-178), box edges and
+//      samples decided in float unless too close to call; a box that meets
+//      more than two bricks of cells on an axis is walked by warps;
 //   4. seal and fill (:291-306) on the cells packed 32 to a word along x:
 //      6-neighbourhood dilations, the fill, as many erosions, the stamp put
 //      back, the words written out as bytes once. The reference fills by
@@ -60,18 +61,17 @@ namespace {
 
 using bounds::Box;
 using bounds::Ellipsoid;
-using bounds::floatCell;
-using bounds::floatSample;
+using bounds::floatCellAt;
 using bounds::floatTestOf;
 using bounds::FloatTest;
 using bounds::GridView;
+using bounds::quickSample;
 using bounds::sampleInside;
 using bounds::hypotV8;
 using bounds::kReachSlack;
 using bounds::reachEstimate;
 
 constexpr uint32_t kCloudBlock = 256;
-constexpr uint32_t kInlineBoxCells = 64;    // larger boxes are stamped by a block each
 // Caps of the union-find loops. Labels strictly fall along every walk, so
 // the loops end by themselves; the caps, and the shared flag the first
 // thread to reach one raises (every walk polls it), only bound the kernels'
@@ -114,6 +114,17 @@ __device__ void frameOf(const CloudInput& in, uint32_t i, Ellipsoid& e) {
     for (int a = 0; a < 3; a++) e.radius[a] = in.sigma * double(in.scale[3 * size_t(i) + a]);
 }
 
+// The frame's entries as the float32 values frameOf rounds to: in float where
+// every one is certified to equal the double path's rounding
+// (frame_rows.cuh), else in double.
+__device__ __forceinline__ void frameRows(const CloudInput& in, uint32_t i, float col[9]) {
+    const float* q4 = in.rot + 4 * size_t(i);
+    if (frame::rowsInFloat(q4[0], q4[1], q4[2], q4[3], col)) return;
+    Ellipsoid full;
+    frameOf(in, i, full);
+    for (int q = 0; q < 9; q++) col[q] = float(full.col[q]);
+}
+
 // Doubles ordered as unsigned integers: the sign bit flipped on positives,
 // every bit on negatives.
 __device__ __forceinline__ unsigned long long orderedKey(double v) {
@@ -139,12 +150,13 @@ __device__ __forceinline__ unsigned long long warpMax64(unsigned long long v) {
 }
 
 // The float side of the bounds and the stamp. For each Gaussian the bounds
-// pass keeps, per world axis a, frames[3 i + a] = (row a of its frame as the
-// float32 values frameOf rounds to, a float estimate of its reach along a);
-// the estimate is NaN where it cannot be trusted, and only then is V8's
-// hypot evaluated in double (FP64 runs at a small fraction of the float rate
-// on this part: a double division costs about a hundred float operations).
-//
+// pass keeps a float estimate of its reach along each world axis and what the
+// float frame may have put them off by (x, y, z, slack); a reach is NaN where
+// it cannot be trusted, and only then is V8's hypot evaluated in double (FP64
+// runs at a small fraction of the float rate on this part: a double division
+// costs about a hundred float operations). The exact frame waits for the
+// stamp, and for the Gaussians that need one there (2M Gaussians: 71 us with
+// the frames certified and kept here, 41 without).
 
 // The radii float(sigma) * scale for the estimate (within 2^-23 of the
 // double sigma * scale of cloudVolume.js:196-199), NaN where out of its
@@ -163,52 +175,45 @@ __device__ __forceinline__ float fromOrderedKey32(uint32_t k) {
     return __uint_as_float((k >> 31) ? (k & 0x7fffffffu) : ~k);
 }
 
+// The exact reach along axis a (cloudVolume.js:201-209).
+__device__ __noinline__ double exactReach(const CloudInput& in, uint32_t i, int a) {
+    float col[9];
+    frameRows(in, i, col);
+    double v[3];
+    for (int k = 0; k < 3; k++) {
+        const float c = a == 0 ? col[3 * k] : a == 1 ? col[3 * k + 1] : col[3 * k + 2];
+        v[k] = double(c) * (in.sigma * double(in.scale[3 * size_t(i) + k]));
+    }
+    return hypotV8(v[0], v[1], v[2]);
+}
+
 // cloudVolume.js:219-234 (materialBounds), first pass: per axis the smallest
-// float upper bound on position - reach (keys[0..2]) and the largest float
-// lower bound on position + reach (keys[3..5]) over all Gaussians, from the
-// reach estimates with directed roundings (the exact value rounded outwards
-// where a Gaussian has no estimate). A NaN anywhere raises *nan (Math.min
-// and Math.max then give NaN). Fills `frames`.
-__global__ void cloudBoundsKernel(CloudInput in, uint32_t* __restrict__ keys, uint32_t* __restrict__ nan,
-                                  float4* __restrict__ frames) {
+// float upper bound on position - reach (keys[3..5]) and the largest float
+// lower bound on position + reach (keys[0..2]) over all Gaussians, from the
+// reach estimates with directed roundings; a Gaussian without an estimate is
+// passed by, which leaves the bounds wider, not wrong. Fills `reach`. Reads
+// 40 bytes a Gaussian and writes 16.
+__global__ void __launch_bounds__(kCloudBlock) cloudBoundsKernel(CloudInput in, uint32_t* __restrict__ keys,
+                                                                 float4* __restrict__ reach) {
     uint32_t lo[3] = {~0u, ~0u, ~0u}, hi[3] = {0, 0, 0};
-    bool sawNan = false;
+    const bool quads = (reinterpret_cast<uintptr_t>(in.rot) & 15u) == 0;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < in.count; i += gridDim.x * blockDim.x) {
-        // The frame in float where every entry is certified to equal the
-        // double path's float32 rounding (frame_rows.cuh), else in double.
-        float col[9], rf[3];
         const float* q4 = in.rot + 4 * size_t(i);
-        if (!frame::rowsInFloat(q4[0], q4[1], q4[2], q4[3], col)) {
-            Ellipsoid full;
-            frameOf(in, i, full);
-            for (int q = 0; q < 9; q++) col[q] = float(full.col[q]);
-        }
-        // the double frame, when an exact reach is wanted: the float32
-        // entries widened, exactly frameOf's
-        Ellipsoid e;
-        for (int q = 0; q < 9; q++) e.col[q] = col[q];
-        for (int a = 0; a < 3; a++) e.radius[a] = in.sigma * double(in.scale[3 * size_t(i) + a]);
+        const float4 q = quads ? *reinterpret_cast<const float4*>(q4) : make_float4(q4[0], q4[1], q4[2], q4[3]);
+        float col[9], rf[3], hf[3];
+        bounds::frameInFloat(q.x, q.y, q.z, q.w, col);
         radiiOf(in, i, rf);
+        const float slack = bounds::reachSlack(q.x, q.y, q.z, q.w, rf);
         for (int a = 0; a < 3; a++) {
             const float p = in.pos[3 * size_t(i) + a];
-            float hf = reachEstimate(col, rf, a);
-            if (!isfinite(p)) hf = CUDART_NAN_F;
-            frames[3 * size_t(i) + a] = make_float4(col[3 * a], col[3 * a + 1], col[3 * a + 2], hf);
-            float l, u;
-            if (isnan(hf)) {
-                const double half = hypotV8(e.col[a] * e.radius[0], e.col[3 + a] * e.radius[1], e.col[6 + a] * e.radius[2]);
-                const double ld = double(p) - half, ud = double(p) + half;
-                sawNan |= isnan(ld) || isnan(ud);
-                l = __double2float_ru(ld);
-                u = __double2float_rd(ud);
-            } else {
-                const float narrow = __fmul_rd(hf, float(1.0 - kReachSlack));  // <= reach
-                l = __fsub_ru(p, narrow);                                     // >= position - reach
-                u = __fadd_rd(p, narrow);                                     // <= position + reach
-            }
-            lo[a] = min(lo[a], orderedKey32(l));
-            hi[a] = max(hi[a], orderedKey32(u));
+            hf[a] = reachEstimate(col, rf, a);
+            if (!isfinite(p) || !(slack <= 0x1p60f)) hf[a] = CUDART_NAN_F;
+            if (isnan(hf[a])) continue;
+            const float narrow = __fsub_rd(__fmul_rd(hf[a], float(1.0 - kReachSlack)), slack);  // <= reach
+            lo[a] = min(lo[a], orderedKey32(__fsub_ru(p, narrow)));  // >= position - reach
+            hi[a] = max(hi[a], orderedKey32(__fadd_rd(p, narrow)));  // <= position + reach
         }
+        reach[i] = make_float4(hf[0], hf[1], hf[2], slack);
     }
     for (int a = 0; a < 3; a++) {
         for (int o = 16; o > 0; o >>= 1) {
@@ -216,46 +221,43 @@ __global__ void cloudBoundsKernel(CloudInput in, uint32_t* __restrict__ keys, ui
             hi[a] = max(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
         }
     }
-    sawNan = __any_sync(0xffffffffu, sawNan);
     if ((threadIdx.x & 31) == 0) {
+        // Six words that every warp adds to: only where it would change one.
         for (int a = 0; a < 3; a++) {
-            atomicMin(keys + a, lo[a]);
-            atomicMax(keys + 3 + a, hi[a]);
+            if (lo[a] < __ldcg(keys + 3 + a)) atomicMin(keys + 3 + a, lo[a]);
+            if (hi[a] > __ldcg(keys + a)) atomicMax(keys + a, hi[a]);
         }
-        if (sawNan) atomicOr(nan, 1u);
     }
-}
-
-// The exact reach along axis a (cloudVolume.js:201-209).
-__device__ double exactReach(const CloudInput& in, uint32_t i, int a) {
-    Ellipsoid e;
-    frameOf(in, i, e);
-    return hypotV8(e.col[a] * e.radius[0], e.col[3 + a] * e.radius[1], e.col[6 + a] * e.radius[2]);
 }
 
 // Second pass: the exact extremes. Only a Gaussian whose position - reach can
 // lie at or below the first pass's smallest upper bound can hold the minimum
 // (every other one's exceeds it), and likewise for the maximum; those few get
-// the exact reach and their exact bound into exact[0..5]. The test is in
-// float, rounded outwards: position - reach >= RD(position - RU(hf (1 +
-// slack))).
+// the exact reach and their exact bound into exact[0..5], and every Gaussian
+// without an estimate does; a NaN among those raises *nan (Math.min and
+// Math.max then give NaN). The test is in
+// float, rounded outwards: position - reach >= RD(position - RU(RU(hf (1 +
+// kReachSlack)) + slack)).
 __global__ void cloudExtremesKernel(CloudInput in, const uint32_t* __restrict__ keys,
-                                    const float4* __restrict__ frames, unsigned long long* __restrict__ exact) {
+                                    const float4* __restrict__ reach, unsigned long long* __restrict__ exact,
+                                    uint32_t* __restrict__ nan) {
     unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0, 0, 0};
     float bound[6];
     for (int q = 0; q < 6; q++) bound[q] = fromOrderedKey32(keys[q]);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < in.count; i += gridDim.x * blockDim.x) {
+        const float4 r = reach[i];
         for (int a = 0; a < 3; a++) {
             const float p = in.pos[3 * size_t(i) + a];
-            const float hf = frames[3 * size_t(i) + a].w;
+            const float hf = a == 0 ? r.x : a == 1 ? r.y : r.z;
             bool low = true, high = true;
             if (!isnan(hf)) {
-                const float wide = __fmul_ru(hf, float(1.0 + kReachSlack));  // >= reach
-                low = __fsub_rd(p, wide) <= bound[a];
-                high = __fadd_ru(p, wide) >= bound[3 + a];
+                const float wide = __fadd_ru(__fmul_ru(hf, float(1.0 + kReachSlack)), r.w);  // >= reach
+                low = __fsub_rd(p, wide) <= bound[3 + a];
+                high = __fadd_ru(p, wide) >= bound[a];
             }
             if (!(low || high)) continue;
             const double half = exactReach(in, i, a);
+            if (isnan(double(p) - half) || isnan(double(p) + half)) atomicOr(nan, 1u);
             if (low) lo[a] = min(lo[a], orderedKey(double(p) - half));
             if (high) hi[a] = max(hi[a], orderedKey(double(p) + half));
         }
@@ -286,22 +288,78 @@ __device__ bool floatTestInFloat(const CloudInput& in, uint32_t i, const GridVie
     return bounds::floatTestInFloat(g, b, c, cf, col, in.sigma, in.sigmaF, scale, f);
 }
 
-// cloudVolume.js:170-173 for one cell of a box: any sample inside. The index
-// is the reference's cellIndex of the (possibly out-of-grid, when the
-// padding is under two cells) coordinates, and like a typed array the grid
-// ignores an index outside it. The double frame is rebuilt only for a sample
-// the float test cannot call.
+// The stamped cells, a bit each: 64 cells of a 4 x 4 x 4 brick to a word (bit
+// x + 4 y + 16 z), bricks in x, y, z order. A Gaussian's box is a few cells
+// wide, so one or two words (1.95 on average for boxes of two cells a side)
+// hold the state of all of its cells, where bytes took a gather a cell.
+struct Bricks {
+    unsigned long long* bits;
+    uint32_t nx, ny;  // bricks along x and y
+    __device__ __forceinline__ unsigned long long* at(uint32_t bx, uint32_t by, uint32_t bz) const {
+        return bits + (size_t(bz) * ny + by) * nx + bx;
+    }
+    __device__ __forceinline__ void set(uint32_t x, uint32_t y, uint32_t z) const {
+        atomicOr(at(x >> 2, y >> 2, z >> 2), 1ull << ((x & 3) + 4 * (y & 3) + 16 * (z & 3)));
+    }
+};
+
+// A box of cells, all of them in the grid: from lo to hi, hi included.
+struct CellBox {
+    uint32_t lo[3], hi[3];
+    // the box's cells in brick (bx, by, bz), which it meets
+    __device__ __forceinline__ unsigned long long in(uint32_t bx, uint32_t by, uint32_t bz) const {
+        const uint32_t x0 = max(lo[0], 4 * bx) & 3, x1 = min(hi[0] - 4 * bx, 3u);
+        const uint32_t y0 = max(lo[1], 4 * by) & 3, y1 = min(hi[1] - 4 * by, 3u);
+        const uint32_t z0 = max(lo[2], 4 * bz) & 3, z1 = min(hi[2] - 4 * bz, 3u);
+        const uint32_t row = (0xfu << x0) & (0xfu >> (3 - x1));
+        const uint32_t slice = row * ((0x1111u << 4 * y0) & (0xffffu >> 4 * (3 - y1)));
+        return slice * ((0x0001000100010001ull << 16 * z0) & (~0ull >> 16 * (3 - z1)));
+    }
+    // Whether it meets at most two bricks along every axis.
+    __device__ __forceinline__ bool small() const {
+        return (hi[0] >> 2) - (lo[0] >> 2) < 2 && (hi[1] >> 2) - (lo[1] >> 2) < 2 && (hi[2] >> 2) - (lo[2] >> 2) < 2;
+    }
+    // A small box's empty cells: bit x + 4 y + 16 z of word dx + 2 dy + 4 dz
+    // for a cell of the brick that lies (dx, dy, dz) after the box's first.
+    // All of the words are read at once: one after another their round trips
+    // were most of the stamp.
+    __device__ __forceinline__ void empty(const Bricks& bricks, unsigned long long (&m)[8]) const {
+        uint32_t row[2], col[2];       // x and y: the bits of a row, a row's bit in a slice
+        unsigned long long slice[2];
+        bool two[3];
+        for (int a = 0; a < 3; a++) two[a] = (hi[a] >> 2) != (lo[a] >> 2);
+        for (uint32_t d = 0; d < 2; d++) {
+            const uint32_t x0 = d ? 0 : lo[0] & 3, x1 = d || !two[0] ? hi[0] & 3 : 3;
+            const uint32_t y0 = d ? 0 : lo[1] & 3, y1 = d || !two[1] ? hi[1] & 3 : 3;
+            const uint32_t z0 = d ? 0 : lo[2] & 3, z1 = d || !two[2] ? hi[2] & 3 : 3;
+            row[d] = (0xfu << x0) & (0xfu >> (3 - x1));
+            col[d] = (0x1111u << 4 * y0) & (0xffffu >> 4 * (3 - y1));
+            slice[d] = (0x0001000100010001ull << 16 * z0) & (~0ull >> 16 * (3 - z1));
+        }
+        const unsigned long long* first = bricks.at(lo[0] >> 2, lo[1] >> 2, lo[2] >> 2);
+        const size_t plane = size_t(bricks.nx) * bricks.ny;
+#pragma unroll
+        for (uint32_t q = 0; q < 8; q++) {
+            const bool has = (!(q & 1) || two[0]) && (!(q & 2) || two[1]) && (!(q & 4) || two[2]);
+            m[q] = has ? __ldcg(first + (q & 1) + (q & 2 ? bricks.nx : 0u) + (q & 4 ? plane : 0)) : ~0ull;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < 8; q++) m[q] = slice[q >> 2] * (row[q & 1] * col[q >> 1 & 1]) & ~m[q];
+    }
+};
+
+// cloudVolume.js:170-173 for one cell of a box: any sample inside. The double
+// frame is rebuilt only for a sample the float test cannot call.
 //
 // The float path converts nothing from double or 64-bit integers: on this
 // part such conversions run on the FP64 pipe, and nine samples a cell made
 // them the stamp's bottleneck. The cell's place in its box (under 2^20, so
 // exact) is an int32 turned float once; the sample offsets are float
 // constants.
-__device__ void stampCell(const CloudInput& in, uint32_t gaussian, const GridView& g, uint8_t* occ, const int64_t lo[3],
-                          int64_t i, int64_t j, int64_t k, const double c[3], const FloatTest* f) {
-    const int64_t cell = i + int64_t(g.dims[0]) * (j + int64_t(g.dims[1]) * k);
-    if (cell < 0 || cell >= int64_t(g.cells) || occ[cell] != 0) return;
+__device__ bool cellReached(const CloudInput& in, uint32_t gaussian, const GridView& g, const int64_t lo[3], int64_t i,
+                            int64_t j, int64_t k, const FloatTest* f, float quick) {
     Ellipsoid e;
+    double c[3];
     bool haveFrame = false;
     const float fi = float(int32_t(i - lo[0])), fj = float(int32_t(j - lo[1])), fk = float(int32_t(k - lo[2]));
 #pragma unroll
@@ -309,21 +367,19 @@ __device__ void stampCell(const CloudInput& in, uint32_t gaussian, const GridVie
         const float ox = s == 8 ? 0.5f : float(s & 1), oy = s == 8 ? 0.5f : float((s >> 1) & 1);
         const float oz = s == 8 ? 0.5f : float((s >> 2) & 1);
         int inside = -1;
-        if (f) inside = floatSample(*f, fi + ox, fj + oy, fk + oz);
+        if (f) inside = quickSample(*f, quick, fi + ox, fj + oy, fk + oz);
         if (inside < 0) {
             if (!haveFrame) {
                 frameOf(in, gaussian, e);
+                for (int a = 0; a < 3; a++) c[a] = in.pos[3 * size_t(gaussian) + a];
                 haveFrame = true;
             }
             inside = sampleInside(g, i, j, k, s, c, e) ? 1 : 0;
         }
-        if (inside) {
-            occ[cell] = 1;
-            return;
-        }
+        if (inside) return true;
     }
+    return false;
 }
-
 
 // Whether the float cells hold for a position on axis a (ranges that keep
 // every term above a normal float's floor and below overflow).
@@ -331,162 +387,457 @@ __device__ __forceinline__ bool floatCellsHold(const GridView& g, float c, float
     return g.floatBound && g.invH > 0.0f && fabsf(c) <= 0x1p40f && reach <= 0x1p40f;
 }
 
-__device__ __forceinline__ int64_t clampCell(int64_t v, int64_t lo, int64_t hi) { return v < lo ? lo : v > hi ? hi : v; }
+// As clampedCell: where hi < lo (a grid of one or two cells) it is hi.
+__device__ __forceinline__ int64_t clampCell(int64_t v, int64_t lo, int64_t hi) { return min(max(v, lo), hi); }
 
-// cloudVolume.js:384-386 for the centre: in float, else exact.
-__device__ int64_t centreCell(const GridView& g, double c, int a) {
-    const float cf = float(c);  // exact: c is a float position
-    int64_t cell;
-    if (floatCellsHold(g, cf, 0.0f)) {
-        const float co = cf - g.originF[a];
-        const float delta = bounds::cellDelta(g.originMag[a], cf, co, 0.0f, g.invH);
-        if (floatCell(co, 0.0f, 0.0f, g.invH, delta, cell)) return clampCell(cell, 0, int64_t(g.dims[a]) - 1);
-    }
-    return clampedCell(c, g.origin[a], g.h, 0, int64_t(g.dims[a]) - 1);
+// cloudVolume.js:384-386 for the centre: in float (false: not decided), or
+// exact.
+__device__ __forceinline__ bool floatCentre(const GridView& g, float c, int a, uint32_t& cell) {
+    if (!floatCellsHold(g, c, 0.0f)) return false;
+    const float co = c - g.originF[a];
+    const float delta = bounds::cellDelta(g.originMag[a], c, co, 0.0f, g.invH);
+    float at;
+    if (!floatCellAt(co, 0.0f, 0.0f, g.invH, delta, at)) return false;
+    cell = uint32_t(clampCell(int32_t(at), 0, int64_t(g.dims[a]) - 1));  // under 2^22, so an int32
+    return true;
 }
 
-// cloudVolume.js:147-160: the cells from position - reach to position +
-// reach, within one cell of the faces. With a reach estimate hf the exact
-// reach lies in [hf (1 - kReachSlack), hf (1 + kReachSlack)], also after
-// those bounds are rounded to float (slack 2^-18 against the estimate's
-// 2^-21), so each edge is the float cell of that interval; only an edge
-// within delta of a cell boundary (or a Gaussian without an estimate)
-// takes the exact reach and the double division.
-__device__ Box boxOf(const CloudInput& in, uint32_t i, const GridView& g, const double c[3], const float hf[3]) {
+__device__ __forceinline__ uint32_t exactCentre(const GridView& g, float c, int a) {
+    return uint32_t(clampedCell(double(c), g.origin[a], g.h, 0, int64_t(g.dims[a]) - 1));
+}
+
+// cloudVolume.js:147-160 along one axis: the cells from position - reach to
+// position + reach, within one cell of the faces. With a reach estimate hf
+// the exact reach lies in [hf (1 - kReachSlack) - slack, hf (1 + kReachSlack)
+// + slack], also after those bounds are rounded to float (kReachSlack 2^-18
+// against the estimate's 2^-21, slack twice what it must be), so each edge is
+// the float cell of that interval; only an edge within delta of a cell
+// boundary (or a Gaussian without an estimate) takes the exact reach and the
+// double division.
+__device__ __forceinline__ bool floatEdges(const GridView& g, int a, float c, const float4& reach, int32_t& lo,
+                                           int32_t& hi) {
+    const float hf = a == 0 ? reach.x : a == 1 ? reach.y : reach.z;
+    const float narrow = hf * float(1.0 - kReachSlack) - reach.w, wide = hf * float(1.0 + kReachSlack) + reach.w;
+    if (isnan(hf) || !floatCellsHold(g, c, wide)) return false;
+    const float co = c - g.originF[a];
+    const float delta = bounds::cellDelta(g.originMag[a], c, co, wide, g.invH);
+    float l, u;
+    const bool below = floatCellAt(co, -wide, -narrow, g.invH, delta, l);
+    const bool above = floatCellAt(co, narrow, wide, g.invH, delta, u);
+    if (!below || !above) return false;
+    lo = int32_t(l);  // under 2^22; before the clamp to the faces
+    hi = int32_t(u);
+    return true;
+}
+
+__device__ __noinline__ void exactEdges(const CloudInput& in, uint32_t i, const GridView& g, int a, int64_t* edges) {
+    const int64_t lo = 1, hi = int64_t(g.dims[a]) - 2;
+    const double c = in.pos[3 * size_t(i) + a], half = exactReach(in, i, a);
+    edges[0] = clampedCell(c - half, g.origin[a], g.h, lo, hi);
+    edges[1] = clampedCell(c + half, g.origin[a], g.h, lo, hi);
+}
+
+__device__ __forceinline__ Box boxOf(const CloudInput& in, uint32_t i, const GridView& g,
+                                     const float4* __restrict__ reach) {
     Box b;
+    const float4 r = reach[i];
     for (int a = 0; a < 3; a++) {
-        const int64_t lo = 1, hi = int64_t(g.dims[a]) - 2;
-        const float cf = float(c[a]);  // exact: c is a float position
-        if (!isnan(hf[a]) && floatCellsHold(g, cf, hf[a])) {
-            const float narrow = hf[a] * float(1.0 - kReachSlack), wide = hf[a] * float(1.0 + kReachSlack);
-            const float co = cf - g.originF[a];
-            const float delta = bounds::cellDelta(g.originMag[a], cf, co, wide, g.invH);
-            int64_t l, u;
-            if (floatCell(co, -wide, -narrow, g.invH, delta, l) && floatCell(co, narrow, wide, g.invH, delta, u)) {
-                b.lo[a] = clampCell(l, lo, hi);
-                b.hi[a] = clampCell(u, lo, hi);
-                continue;
-            }
+        int32_t l, u;
+        if (floatEdges(g, a, in.pos[3 * size_t(i) + a], r, l, u)) {
+            b.lo[a] = clampCell(l, 1, int64_t(g.dims[a]) - 2);
+            b.hi[a] = clampCell(u, 1, int64_t(g.dims[a]) - 2);
+            continue;
         }
-        const double half = exactReach(in, i, a);
-        b.lo[a] = clampedCell(c[a] - half, g.origin[a], g.h, lo, hi);
-        b.hi[a] = clampedCell(c[a] + half, g.origin[a], g.h, lo, hi);
+        int64_t edges[2];
+        exactEdges(in, i, g, a, edges);
+        b.lo[a] = edges[0];
+        b.hi[a] = edges[1];
     }
     return b;
 }
 
-// The Gaussian's box and its float test (false: test in double), from the
-// frame rows and reach estimates the bounds pass kept; the frame's double
-// values are the float rows widened, exactly frameOf's.
-__device__ bool prepareStamp(const CloudInput& in, uint32_t i, const GridView& g, const float4* __restrict__ frames,
-                             const double c[3], Box& b, FloatTest& f) {
-    float col[9], hf[3], cf[3];
+// The box where every edge is decided in float, of a grid with three cells
+// or more on every axis.
+__device__ __forceinline__ bool floatBox(const CloudInput& in, uint32_t i, const GridView& g,
+                                         const float4* __restrict__ reach, CellBox& b) {
+    bool ok = true;
+    const float4 r = reach[i];
+#pragma unroll
     for (int a = 0; a < 3; a++) {
-        const float4 row = frames[3 * size_t(i) + a];
-        col[3 * a] = row.x;
-        col[3 * a + 1] = row.y;
-        col[3 * a + 2] = row.z;
-        hf[a] = row.w;
-        cf[a] = in.pos[3 * size_t(i) + a];
+        int32_t l = 0, u = 0;
+        ok = floatEdges(g, a, in.pos[3 * size_t(i) + a], r, l, u) && ok;
+        const int32_t top = int32_t(min(g.dims[a] - 2, 1u << 30));
+        b.lo[a] = uint32_t(max(1, min(l, top)));
+        b.hi[a] = uint32_t(max(1, min(u, top)));
     }
-    b = boxOf(in, i, g, c, hf);
+    return ok;
+}
+
+__device__ __forceinline__ CellBox cellBox(const Box& b) {
+    CellBox c;
+    for (int a = 0; a < 3; a++) {
+        c.lo[a] = uint32_t(b.lo[a]);
+        c.hi[a] = uint32_t(b.hi[a]);
+    }
+    return c;
+}
+
+// Gaussians left for the pass that decides in double.
+struct HardList {
+    uint32_t* items;
+    unsigned long long* count;
+    __device__ __forceinline__ void add(uint32_t i) const { items[atomicAdd(count, 1ull)] = i; }
+};
+
+// One Gaussian's stamp as a walk over its box needs it, in shared memory.
+struct StampEntry {
+    FloatTest f;
+    float quick;     // quickBound(f)
+    uint32_t gaussian;
+    uint32_t fast;   // the float test holds; else test in double
+    CellBox box;
+};
+
+// The Gaussian's float test, from the frame formed again.
+__device__ __forceinline__ bool testOf(const CloudInput& in, uint32_t i, const GridView& g, const Box& b,
+                                       FloatTest& f) {
+    float col[9], cf[3];
+    double c[3];
+    frameRows(in, i, col);
+    for (int a = 0; a < 3; a++) {
+        cf[a] = in.pos[3 * size_t(i) + a];
+        c[a] = cf[a];
+    }
     return floatTestInFloat(in, i, g, b, c, cf, col, f);
 }
 
-// One Gaussian's stamp as the walk below needs it, in shared memory.
-struct StampEntry {
-    FloatTest f;
-    int64_t lo[3];
-    uint32_t ex, exy;  // the box's extent along x, and x times y
-    uint32_t gaussian;
-    uint32_t fast;
-};
+__device__ __forceinline__ void setUp(const CloudInput& in, uint32_t i, const GridView& g, const CellBox& box,
+                                      StampEntry& e) {
+    Box b;
+    for (int a = 0; a < 3; a++) {
+        b.lo[a] = box.lo[a];
+        b.hi[a] = box.hi[a];
+    }
+    e.fast = testOf(in, i, g, b, e.f) ? 1u : 0u;
+    e.quick = bounds::quickBound(e.f);
+    e.gaussian = i;
+    e.box = box;
+}
+
+__device__ __forceinline__ void markCell(const Bricks& bricks, const uint32_t at[3]) {
+    unsigned long long* word = bricks.at(at[0] >> 2, at[1] >> 2, at[2] >> 2);
+    const unsigned long long bit = 1ull << ((at[0] & 3) + 4 * (at[1] & 3) + 16 * (at[2] & 3));
+    if ((__ldcg(word) & bit) == 0) atomicOr(word, bit);
+}
 
 constexpr uint32_t kStampBlock = 128;
+constexpr uint32_t kStampBlocks = 7;  // an SM
 
-// cloudVolume.js:147-177. Each thread sets up one Gaussian: its centre's cell
-// unconditionally, its box and float test; a box of more than
-// kInlineBoxCells cells is listed for cloudStampBoxKernel. Then each warp
-// walks its 32 Gaussians' boxes as one list of cells dealt to its lanes 32
-// at a time (a lane finds the Gaussian owning its cell by a binary search
-// over the warp's running offsets), so lanes are not idle while one
-// Gaussian's box is longer than its neighbours'. Marking is an OR: which
-// lane tests a cell, and when, changes nothing.
-__global__ void __launch_bounds__(kStampBlock) cloudStampKernel(CloudInput in, GridView g,
-                                                                const float4* __restrict__ frames,
-                                                                uint8_t* __restrict__ occ, uint32_t* __restrict__ big,
-                                                                uint32_t* __restrict__ bigCount) {
+// The place of the n-th set bit of a word that has more than n.
+__device__ __forceinline__ uint32_t setBit(unsigned long long word, uint32_t n) {
+    uint32_t w = uint32_t(word), at = 0;
+    const uint32_t low = __popc(w);
+    if (n >= low) {
+        n -= low;
+        w = uint32_t(word >> 32);
+        at = 32;
+    }
+#pragma unroll
+    for (uint32_t half = 16; half >= 1; half >>= 1) {
+        const uint32_t here = __popc(w & ((1u << half) - 1u));
+        if (n >= here) {
+            n -= here;
+            w >>= half;
+            at += half;
+        }
+    }
+    return at;
+}
+
+// cloudVolume.js:147-177 for boxes that meet at most two bricks on an axis;
+// larger ones are listed for cloudStampBoxKernel. A block takes `rounds` times
+// its threads of Gaussians and marks their centres. A Gaussian whose box then
+// has no empty cell left is done (of 2M Gaussians on a surface of 418,000
+// cells' centres 61 % at least); the others wait in shared memory until a
+// block's worth of them can be set up together, since the set-up (the frame,
+// the float test's bounds, some of them in double) costs more than finding
+// that nothing is left to do. Then each warp walks the empty cells of its 32
+// boxes as one list dealt to its lanes 32 at a time (a lane finds the Gaussian
+// owning its cell by a binary search over the warp's running offsets).
+// Marking is an OR: which lane tests a cell, and when, changes nothing; a cell
+// that another marks meanwhile is tested for nothing.
+//
+// Instructions bound it, 985 a warp of Gaussians (2M at 231 x 223 x 243 cells:
+// 142 us, where setting every Gaussian up and walking bytes of all its cells
+// took 405; with a brick's words read one after another 258). One wave of
+// blocks: two of half as many rounds each take 20 us more, since the first
+// rounds know the fewest marks.
+//
+// An edge or centre that float cannot decide (one of 250 Gaussians at 230 cells
+// across) would hold its whole warp up for the exact reach and divisions, some
+// four hundred double operations at 16 cycles a warp: such Gaussians are
+// listed, and a second launch, HARD, takes
+// them together.
+template <bool HARD>
+__global__ void __launch_bounds__(kStampBlock, HARD ? 4 : kStampBlocks) cloudStampKernel(CloudInput in, GridView g,
+                                                                const float4* __restrict__ reach, Bricks bricks,
+                                                                uint32_t rounds, HardList hard,
+                                                                uint32_t* __restrict__ big,
+                                                                unsigned long long* __restrict__ bigCount) {
     constexpr unsigned kAll = 0xffffffffu;
     __shared__ StampEntry entries[kStampBlock];
-    const uint32_t lane = threadIdx.x & 31;
-    const StampEntry* warpEntries = entries + (threadIdx.x & ~31u);
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t n = 0;
-    if (i < in.count) {
-        const double c[3] = {in.pos[3 * size_t(i)], in.pos[3 * size_t(i) + 1], in.pos[3 * size_t(i) + 2]};
-        int64_t at[3];
-        for (int a = 0; a < 3; a++) at[a] = centreCell(g, c[a], a);
-        occ[at[0] + int64_t(g.dims[0]) * (at[1] + int64_t(g.dims[1]) * at[2])] = 1;
-        Box b;
-        StampEntry& mine = entries[threadIdx.x];
-        const bool fast = prepareStamp(in, i, g, frames, c, b, mine.f);
-        if (b.cells() > kInlineBoxCells) {
-            big[atomicAdd(bigCount, 1u)] = i;  // at most one slot per Gaussian: `big` holds count
-        } else {
-            n = uint32_t(b.cells());
-            for (int a = 0; a < 3; a++) mine.lo[a] = b.lo[a];
-            mine.ex = uint32_t(b.extent(0));
-            mine.exy = mine.ex * uint32_t(b.extent(1));
-            mine.gaussian = i;
-            mine.fast = fast ? 1u : 0u;
-        }
-    }
-    // The warp's running offsets: lane l's cells are [off, off + n).
-    uint32_t incl = n;
+    __shared__ unsigned long long empties[8][kStampBlock];
+    __shared__ uint32_t queue[2 * kStampBlock];
+    __shared__ uint32_t queued;
+    const uint32_t t = threadIdx.x, lane = t & 31, warpBase = t & ~31u;
+    // Sets up a Gaussian a lane and walks the warp's empty cells.
+    auto stamp = [&](bool active, uint32_t i, const CellBox& box) {
+        uint32_t n = 0;
+        if (active) {
+            unsigned long long m[8];
+            box.empty(bricks, m);
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t v = __shfl_up_sync(kAll, incl, d);
-        if (lane >= uint32_t(d)) incl += v;
-    }
-    const uint32_t off = incl - n;
-    const uint32_t total = __shfl_sync(kAll, incl, 31);
-    __syncwarp();
-    for (uint32_t base = 0; base < total; base += 32) {
-        const uint32_t t = base + lane;
-        // the last lane whose offset is at or below t (offsets never fall)
-        uint32_t owner = 0;
-#pragma unroll
-        for (uint32_t step = 16; step >= 1; step >>= 1) {
-            const uint32_t probe = __shfl_sync(kAll, off, owner + step);
-            if (probe <= t) owner += step;
+            for (uint32_t q = 0; q < 8; q++) {
+                n += __popcll(m[q]);
+                empties[q][t] = m[q];
+            }
+            if (n) setUp(in, i, g, box, entries[t]);
         }
-        const uint32_t first = __shfl_sync(kAll, off, owner);
-        if (t >= total) continue;
-        const StampEntry& e = warpEntries[owner];
-        const uint32_t r = t - first, ex = e.ex, exy = e.exy;
-        const uint32_t k = r / exy, rem = r - k * exy, j = rem / ex, i2 = rem - j * ex;
-        const uint32_t gi = e.gaussian;
-        const double c[3] = {in.pos[3 * size_t(gi)], in.pos[3 * size_t(gi) + 1], in.pos[3 * size_t(gi) + 2]};
-        const int64_t lo[3] = {e.lo[0], e.lo[1], e.lo[2]};
-        stampCell(in, gi, g, occ, lo, lo[0] + i2, lo[1] + j, lo[2] + k, c, e.fast ? &e.f : nullptr);
+        // The warp's running offsets: lane l's cells are [off, off + n).
+        uint32_t incl = n;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t v = __shfl_up_sync(kAll, incl, d);
+            if (lane >= uint32_t(d)) incl += v;
+        }
+        const uint32_t off = incl - n;
+        const uint32_t total = __shfl_sync(kAll, incl, 31);
+        __syncwarp();
+        for (uint32_t base = 0; base < total; base += 32) {
+            const uint32_t c = base + lane;
+            // the last lane whose offset is at or below c (offsets never fall)
+            uint32_t owner = 0;
+#pragma unroll
+            for (uint32_t step = 16; step >= 1; step >>= 1) {
+                const uint32_t probe = __shfl_sync(kAll, off, owner + step);
+                if (probe <= c) owner += step;
+            }
+            const uint32_t start = __shfl_sync(kAll, off, owner);
+            if (c >= total) continue;
+            const StampEntry& e = entries[warpBase + owner];
+            // the cell: the (c - start)-th of the owner's empty ones
+            uint32_t at = c - start, q = 0;
+            unsigned long long m = empties[0][warpBase + owner];
+            for (uint32_t here = __popcll(m); at >= here && q < 7; here = __popcll(m)) {
+                at -= here;
+                m = empties[++q][warpBase + owner];
+            }
+            const uint32_t bit = setBit(m, at);
+            const uint32_t x = 4 * ((e.box.lo[0] >> 2) + (q & 1)) + (bit & 3);
+            const uint32_t y = 4 * ((e.box.lo[1] >> 2) + (q >> 1 & 1)) + (bit >> 2 & 3);
+            const uint32_t z = 4 * ((e.box.lo[2] >> 2) + (q >> 2)) + (bit >> 4);
+            const int64_t lo[3] = {e.box.lo[0], e.box.lo[1], e.box.lo[2]};
+            if (cellReached(in, e.gaussian, g, lo, x, y, z, e.fast ? &e.f : nullptr, e.quick)) bricks.set(x, y, z);
+        }
+        __syncwarp();  // the warp's entries have been read
+    };
+    if (HARD) {
+        // Few, and the double chain of one axis is the time: a lane for each
+        // axis, ten Gaussians a warp, the warps spread over the grid's blocks
+        // first (2M Gaussians list about 8,000: 36 us with full warps, 23 so).
+        constexpr uint32_t kTen = 10;
+        const uint64_t listed = *hard.count;
+        const uint32_t mine = lane / 3, axis = lane % 3;
+        for (uint64_t base = ((t >> 5) * uint64_t(gridDim.x) + blockIdx.x) * kTen; base < listed;
+             base += uint64_t(gridDim.x) * (kStampBlock / 32) * kTen) {
+            uint32_t i = 0, centreAt = 0, l = 0, u = 0;
+            if (mine < kTen && base + mine < listed) {
+                i = hard.items[base + mine];
+                const float c = in.pos[3 * size_t(i) + axis];
+                if (!floatCentre(g, c, axis, centreAt)) centreAt = exactCentre(g, c, axis);
+                int32_t lf, uf;
+                int64_t edges[2];
+                if (floatEdges(g, axis, c, reach[i], lf, uf)) {
+                    edges[0] = clampCell(lf, 1, int64_t(g.dims[axis]) - 2);
+                    edges[1] = clampCell(uf, 1, int64_t(g.dims[axis]) - 2);
+                } else {
+                    exactEdges(in, i, g, axis, edges);
+                }
+                l = uint32_t(edges[0]);
+                u = uint32_t(edges[1]);
+            }
+            // gathered to a lane a Gaussian
+            CellBox b;
+            uint32_t centre[3];
+#pragma unroll
+            for (uint32_t a = 0; a < 3; a++) {
+                centre[a] = __shfl_sync(kAll, centreAt, 3 * lane + a);
+                b.lo[a] = __shfl_sync(kAll, l, 3 * lane + a);
+                b.hi[a] = __shfl_sync(kAll, u, 3 * lane + a);
+            }
+            i = __shfl_sync(kAll, i, 3 * lane);
+            bool small = false;
+            if (lane < kTen && base + lane < listed) {
+                markCell(bricks, centre);
+                small = b.small();
+                if (!small) big[atomicAdd(bigCount, 1ull)] = i;
+            }
+            stamp(small, i, b);
+        }
+        return;
+    }
+    if (t == 0) queued = 0;
+    __syncthreads();
+    const uint64_t first = uint64_t(blockIdx.x) * rounds * kStampBlock;
+    for (uint32_t round = 0; round < rounds; round++) {
+        const uint64_t at = first + uint64_t(round) * kStampBlock + t;
+        bool left = false;
+        if (at < in.count) {
+            // cloudVolume.js:161: the centre's cell, unconditionally
+            uint32_t centre[3];
+            bool known = true;
+#pragma unroll
+            for (int a = 0; a < 3; a++) known = floatCentre(g, in.pos[3 * size_t(at) + a], a, centre[a]) && known;
+            if (known) markCell(bricks, centre);
+            CellBox b;
+            if (!floatBox(in, uint32_t(at), g, reach, b) || !known) {
+                hard.add(uint32_t(at));
+            } else if (!b.small()) {
+                big[atomicAdd(bigCount, 1ull)] = uint32_t(at);
+            } else {
+                unsigned long long m[8], any = 0;
+                b.empty(bricks, m);
+#pragma unroll
+                for (uint32_t q = 0; q < 8; q++) any |= m[q];
+                left = any != 0;
+            }
+        }
+        const uint32_t keep = __ballot_sync(kAll, left);
+        uint32_t slot = 0;
+        if (lane == 0 && keep) slot = atomicAdd(&queued, uint32_t(__popc(keep)));
+        slot = __shfl_sync(kAll, slot, 0) + __popc(keep & ((1u << lane) - 1u));
+        if (left) queue[slot] = uint32_t(at);  // under kStampBlock wait from the round before
+        __syncthreads();
+        const uint32_t waiting = queued;
+        __syncthreads();  // every thread has read it before the next round adds to it
+        // The queue's last block's worth (in the last round all there is).
+        uint32_t end = waiting;
+        while (end >= kStampBlock || (end > 0 && round + 1 == rounds)) {
+            const uint32_t take = min(end, kStampBlock);
+            uint32_t i = 0;
+            CellBox b;
+            if (t < take) {
+                i = queue[end - take + t];
+                floatBox(in, i, g, reach, b);  // decided before
+            }
+            stamp(t < take, i, b);
+            end -= take;
+        }
+        if (end != waiting) {
+            __syncthreads();  // the queue's end has been read
+            if (t == 0) queued = end;
+            __syncthreads();
+        }
     }
 }
 
-// The listed large boxes, a block each, its threads over the box's cells.
-__global__ void cloudStampBoxKernel(CloudInput in, GridView g, const float4* __restrict__ frames,
-                                    uint8_t* __restrict__ occ, const uint32_t* __restrict__ big,
-                                    const uint32_t* __restrict__ bigCount) {
-    const uint32_t listed = *bigCount;
-    for (uint32_t n = blockIdx.x; n < listed; n += gridDim.x) {
-        const uint32_t i = big[n];
-        const double c[3] = {in.pos[3 * size_t(i)], in.pos[3 * size_t(i) + 1], in.pos[3 * size_t(i) + 2]};
-        Box b;
+// The listed larger boxes, several to a block: one thread sets each up, then
+// the block's warps walk the bricks of all of them, a brick's 64 cells two to
+// a lane, and mark a brick by one OR. A brick with no empty cell of the box
+// costs one read.
+constexpr uint32_t kBoxThreads = 256;
+constexpr uint32_t kBoxBatch = kBoxThreads / 32;
+
+__global__ void __launch_bounds__(kBoxThreads) cloudStampBoxKernel(CloudInput in, GridView g,
+                                                                   const float4* __restrict__ reach, Bricks bricks,
+                                                                   const uint32_t* __restrict__ big,
+                                                                   const unsigned long long* __restrict__ bigCount) {
+    __shared__ StampEntry entries[kBoxBatch];
+    __shared__ unsigned long long ends[kBoxBatch];
+    const uint64_t listed = *bigCount;
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    // as many a block as spreads the list over the grid
+    const uint64_t even = (listed + gridDim.x - 1) / gridDim.x;
+    const uint32_t batch = even < 1 ? 1 : even > kBoxBatch ? kBoxBatch : uint32_t(even);
+    for (uint64_t base = uint64_t(blockIdx.x) * batch; base < listed; base += uint64_t(gridDim.x) * batch) {
+        const uint32_t held = listed - base < batch ? uint32_t(listed - base) : batch;
+        __syncthreads();
+        if (t < held) {
+            const uint32_t i = big[base + t];
+            const CellBox box = cellBox(boxOf(in, i, g, reach));
+            setUp(in, i, g, box, entries[t]);
+            unsigned long long all = 1;
+            for (int a = 0; a < 3; a++) all *= (box.hi[a] >> 2) - (box.lo[a] >> 2) + 1;
+            ends[t] = all;
+        }
+        __syncthreads();
+        unsigned long long total = 0;
+        for (uint32_t q = 0; q < held; q++) total += ends[q];
+        for (unsigned long long task = warp; task < total; task += kBoxThreads / 32) {
+            uint32_t q = 0;
+            unsigned long long r = task;
+            while (r >= ends[q]) r -= ends[q++];
+            const StampEntry& e = entries[q];
+            const uint32_t bx0 = e.box.lo[0] >> 2, by0 = e.box.lo[1] >> 2, bz0 = e.box.lo[2] >> 2;
+            const uint32_t ex = (e.box.hi[0] >> 2) - bx0 + 1, ey = (e.box.hi[1] >> 2) - by0 + 1;
+            uint32_t bx, by, bz;
+            if (r >> 32) {
+                const unsigned long long row = r / ex;
+                bx = uint32_t(r - row * ex);
+                bz = uint32_t(row / ey);
+                by = uint32_t(row - (unsigned long long)bz * ey);
+            } else {
+                const uint32_t row = uint32_t(r) / ex;
+                bx = uint32_t(r) - row * ex;
+                bz = row / ey;
+                by = row - bz * ey;
+            }
+            bx += bx0;
+            by += by0;
+            bz += bz0;
+            unsigned long long* word = bricks.at(bx, by, bz);
+            const unsigned long long empty = e.box.in(bx, by, bz) & ~__ldcg(word);  // the warp's, by one address
+            if (empty == 0) continue;
+            const int64_t lo[3] = {e.box.lo[0], e.box.lo[1], e.box.lo[2]};
+            unsigned long long mark = 0;
+#pragma unroll
+            for (uint32_t half = 0; half < 2; half++) {
+                const uint32_t bit = lane + 32 * half;
+                bool in_ = (empty >> bit & 1) != 0;
+                if (in_)
+                    in_ = cellReached(in, e.gaussian, g, lo, 4 * bx + (bit & 3), 4 * by + (bit >> 2 & 3),
+                                      4 * bz + (bit >> 4), e.fast ? &e.f : nullptr, e.quick);
+                mark |= static_cast<unsigned long long>(__ballot_sync(0xffffffffu, in_)) << 32 * half;
+            }
+            if (lane == 0 && mark) atomicOr(word, mark);
+        }
+    }
+}
+
+// The stamp of a grid with fewer than three cells on an axis, where "within
+// one cell of the faces" leaves the grid: the index is the reference's
+// cellIndex of the (possibly out-of-grid) coordinates, and like a typed array
+// the grid ignores an index outside it. A block a Gaussian.
+__global__ void cloudStampLooseKernel(CloudInput in, GridView g, const float4* __restrict__ reach, Bricks bricks) {
+    for (uint32_t i = blockIdx.x; i < in.count; i += gridDim.x) {
+        if (threadIdx.x == 0) {
+            uint32_t centre[3];
+            for (int a = 0; a < 3; a++) centre[a] = exactCentre(g, in.pos[3 * size_t(i) + a], a);
+            markCell(bricks, centre);
+        }
+        const Box b = boxOf(in, i, g, reach);
         FloatTest f;
-        const bool fast = prepareStamp(in, i, g, frames, c, b, f);
-        const int64_t ex = b.extent(0), exy = ex * b.extent(1), total = b.cells();
-        for (int64_t t = threadIdx.x; t < total; t += blockDim.x) {
-            const int64_t k = b.lo[2] + t / exy, r = t % exy;
-            stampCell(in, i, g, occ, b.lo, b.lo[0] + r % ex, b.lo[1] + r / ex, k, c, fast ? &f : nullptr);
+        const bool fast = testOf(in, i, g, b, f);
+        const int64_t ex = b.extent(0), ey = b.extent(1), ez = b.extent(2);
+        if (ex <= 0 || ey <= 0 || ez <= 0) continue;
+        for (int64_t t = threadIdx.x; t < ex * ey * ez; t += blockDim.x) {
+            const int64_t x = b.lo[0] + t % ex, y = b.lo[1] + t / ex % ey, z = b.lo[2] + t / (ex * ey);
+            const int64_t cell = x + int64_t(g.dims[0]) * (y + int64_t(g.dims[1]) * z);
+            if (cell < 0 || cell >= int64_t(g.cells)) continue;
+            const int64_t row = cell / g.dims[0];
+            const uint32_t cx = uint32_t(cell % g.dims[0]), cy = uint32_t(row % g.dims[1]), cz = uint32_t(row / g.dims[1]);
+            if (*bricks.at(cx >> 2, cy >> 2, cz >> 2) >> ((cx & 3) + 4 * (cy & 3) + 16 * (cz & 3)) & 1) continue;
+            if (cellReached(in, i, g, b.lo, x, y, z, fast ? &f : nullptr, bounds::quickBound(f))) bricks.set(cx, cy, cz);
         }
     }
 }
@@ -617,14 +968,6 @@ __global__ void fillEnclosedKernel(uint8_t* __restrict__ occ, uint32_t* L, const
     if (threadIdx.x == 0 && total) atomicAdd(filled, total);
 }
 
-__global__ void countKernel(const uint8_t* __restrict__ occ, uint32_t cells, unsigned long long* __restrict__ count) {
-    unsigned long long mine = 0;
-    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < cells; idx += gridDim.x * blockDim.x)
-        mine += occ[idx];
-    const unsigned long long total = blockSum(mine);
-    if (threadIdx.x == 0 && total) atomicAdd(count, total);
-}
-
 // Small device words of one run.
 // ---------------------------------------------------------------- flood --
 // The same set fillEnclosed's flood reaches (cloudVolume.js:321-375): the
@@ -675,6 +1018,22 @@ __device__ __forceinline__ uint32_t fillDown(uint32_t g, uint32_t p) {
 __device__ __forceinline__ uint32_t validBits(const Dims& d, uint32_t word) {
     const uint32_t count = min(32u, d.nx - word * 32);
     return count == 32 ? 0xffffffffu : (1u << count) - 1u;
+}
+
+// The stamp's bricks as words along x: a word is four cells each of eight
+// bricks.
+__global__ void brickWordsKernel(Bricks bricks, Dims d, Words w, uint32_t* __restrict__ bits) {
+    const uint32_t total = w.rows * w.nw;
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+        const uint32_t row = t / w.nw, word = t - row * w.nw, z = row / w.ny, y = row - z * w.ny;
+        const unsigned long long* brick = bricks.at(8 * word, y >> 2, z >> 2);
+        const uint32_t shift = 4 * (y & 3) + 16 * (z & 3);
+        uint32_t m = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < 8; q++)
+            if (8 * word + q < bricks.nx) m |= uint32_t(brick[q] >> shift & 0xf) << 4 * q;
+        bits[t] = m;
+    }
 }
 
 // A thread per word: bit b of word w of a row set where cell 32 w + b is.
@@ -894,14 +1253,15 @@ __global__ void unpackCellsKernel(const uint32_t* __restrict__ a, const uint32_t
 }
 
 struct CloudScalars {
-    unsigned long long exact[6];  // the exact extremes
-    uint32_t keys[6];             // the bounds' first pass, float keys
+    uint32_t keys[6];             // the bounds' first pass, float keys: largest, then smallest
+    unsigned long long exact[6];  // the exact extremes: smallest, then largest
     unsigned long long filled;
     unsigned long long occupied;
+    unsigned long long bigCount;
+    unsigned long long hardCount;
     uint32_t nan;
     uint32_t err;
-    uint32_t bigCount;
-    uint32_t changed;  // a flood round added cells
+    uint32_t changed[2];  // whether a flood round added cells, two rounds at a time
 };
 
 // Scratch comes from a stream-ordered memory pool of this library's own, one
@@ -957,17 +1317,15 @@ int voxelizeCloud(vsim_cloud_volume* v, const CloudInput& in, const vsim_cloud_o
     DeviceBuffer scalarsBuf;
     POOL_ALLOC(scalarsBuf, sizeof(CloudScalars), pool, st, "cloud scratch");
     auto* sc = static_cast<CloudScalars*>(scalarsBuf.p);
-    CloudScalars init{};
-    for (int a = 0; a < 3; a++) {
-        init.keys[a] = ~0u;
-        init.exact[a] = ~0ull;
-    }
-    CK(cudaMemcpyAsync(sc, &init, sizeof init, cudaMemcpyHostToDevice, st), "cloud scratch");
-    DeviceBuffer framesBuf;
-    POOL_ALLOC(framesBuf, size_t(in.count) * 3 * sizeof(float4), pool, st, "cloud scratch");
-    auto* frames = static_cast<float4*>(framesBuf.p);
-    cloudBoundsKernel<<<streamGrid(in.count, sms), kCloudBlock, 0, st>>>(in, sc->keys, &sc->nan, frames);
-    cloudExtremesKernel<<<streamGrid(in.count, sms), kCloudBlock, 0, st>>>(in, sc->keys, frames, sc->exact);
+    CK(cudaMemsetAsync(sc, 0, sizeof(CloudScalars), st), "cloud scratch");
+    // of none the largest is 0, the smallest all ones
+    CK(cudaMemsetAsync(sc->keys + 3, 0xff, sizeof(uint32_t) * 3 + sizeof(unsigned long long) * 3, st), "cloud scratch");
+    DeviceBuffer reachBuf;
+    POOL_ALLOC(reachBuf, size_t(in.count) * sizeof(float4), pool, st, "cloud scratch");
+    auto* reach = static_cast<float4*>(reachBuf.p);
+    cloudBoundsKernel<<<streamGrid(in.count, sms), kCloudBlock, 0, st>>>(in, sc->keys, reach);
+    cloudExtremesKernel<<<streamGrid(in.count, sms), kCloudBlock, 0, st>>>(in, sc->keys, reach, sc->exact,
+                                                                              &sc->nan);
     CK(cudaGetLastError(), "cloud bounds");
     CloudScalars got{};
     CK(cudaMemcpyAsync(&got, sc, sizeof got, cudaMemcpyDeviceToHost, st), "cloud bounds");
@@ -1020,35 +1378,49 @@ int voxelizeCloud(vsim_cloud_volume* v, const CloudInput& in, const vsim_cloud_o
     g.cells = n;
 
     CK(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&v->occupancy), n, pool, st), "cloud occupancy");
-    CK(cudaMemsetAsync(v->occupancy, 0, n, st), "cloud occupancy");
 
     // 3. stamp
-    DeviceBuffer bigBuf;
-    POOL_ALLOC(bigBuf, size_t(in.count) * 4, pool, st, "cloud scratch");
-    cloudStampKernel<<<(in.count + kStampBlock - 1) / kStampBlock, kStampBlock, 0, st>>>(
-        in, g, frames, v->occupancy, static_cast<uint32_t*>(bigBuf.p), &sc->bigCount);
-    cloudStampBoxKernel<<<uint32_t(sms) * 4, kCloudBlock, 0, st>>>(
-        in, g, frames, v->occupancy, static_cast<const uint32_t*>(bigBuf.p), &sc->bigCount);
+    const Words W{(d.nx + 31) / 32, d.ny * d.nz, d.ny, d.nz};
+    const size_t words = size_t(W.rows) * W.nw;
+    const uint32_t wordGrid = streamGrid(words, sms);
+    DeviceBuffer listsBuf, bricksBuf, wordsBuf;
+    // a Gaussian is listed as hard at most once, and as large at most once
+    POOL_ALLOC(listsBuf, size_t(in.count) * 2 * 4, pool, st, "cloud scratch");
+    const HardList hard{static_cast<uint32_t*>(listsBuf.p), &sc->hardCount};
+    uint32_t* big = hard.items + in.count;
+    const size_t brickBytes = size_t((d.nx + 3) / 4) * ((d.ny + 3) / 4) * ((d.nz + 3) / 4) * 8;
+    POOL_ALLOC(bricksBuf, brickBytes, pool, st, "cloud scratch");
+    const Bricks bricks{static_cast<unsigned long long*>(bricksBuf.p), (d.nx + 3) / 4, (d.ny + 3) / 4};
+    CK(cudaMemsetAsync(bricksBuf.p, 0, brickBytes, st), "cloud stamp");
+    if (d.nx < 3 || d.ny < 3 || d.nz < 3) {
+        cloudStampLooseKernel<<<std::min(in.count, uint32_t(sms) * 8), kCloudBlock, 0, st>>>(in, g, reach, bricks);
+    } else {
+        // As many rounds as make the blocks one wave.
+        const uint64_t wave = uint64_t(sms) * kStampBlocks * kStampBlock;
+        const uint32_t rounds = uint32_t((in.count + wave - 1) / wave);
+        const uint64_t each = uint64_t(rounds) * kStampBlock;
+        cloudStampKernel<false><<<uint32_t((in.count + each - 1) / each), kStampBlock, 0, st>>>(
+            in, g, reach, bricks, rounds, hard, big, &sc->bigCount);
+        cloudStampKernel<true><<<uint32_t(sms) * 8, kStampBlock, 0, st>>>(in, g, reach, bricks, 0, hard, big,
+                                                                           &sc->bigCount);
+        cloudStampBoxKernel<<<uint32_t(sms) * 8, kBoxThreads, 0, st>>>(in, g, reach, bricks, big, &sc->bigCount);
+    }
+    POOL_ALLOC(wordsBuf, words * (o.fill ? 5 : 1) * sizeof(uint32_t), pool, st, "cloud scratch");
+    uint32_t* stampW = static_cast<uint32_t*>(wordsBuf.p);
+    brickWordsKernel<<<wordGrid, kCloudBlock, 0, st>>>(bricks, d, W, stampW);
     CK(cudaGetLastError(), "cloud stamp");
 
     // 4. seal and fill
     const uint32_t grid = streamGrid(n, sms);
     if (o.fill) {
-        // The seal and fill on the cells packed 32 to a word along x: the
-        // stamp packed once, `seal` dilations, the flood, the enclosed cells
+        // The seal and fill on the cells packed 32 to a word along x: `seal`
+        // dilations of the stamp, the flood, the enclosed cells
         // set, `seal` erosions, the stamp put back as the words are written
         // out as bytes once.
-        const Words W{(d.nx + 31) / 32, d.ny * d.nz, d.ny, d.nz};
-        const size_t words = size_t(W.rows) * W.nw;
-        DeviceBuffer wordsBuf;
-        POOL_ALLOC(wordsBuf, words * 5 * sizeof(uint32_t), pool, st, "cloud fill scratch");
-        uint32_t* stampW = static_cast<uint32_t*>(wordsBuf.p);
         uint32_t* cur = stampW + words;
         uint32_t* other = cur + words;
         uint32_t* emptyW = other + words;
         uint32_t* reachedW = emptyW + words;
-        const uint32_t wordGrid = streamGrid(words, sms);
-        packCellsKernel<<<wordGrid, kCloudBlock, 0, st>>>(v->occupancy, d, W, stampW);
         const uint32_t* src = stampW;
         for (uint32_t p = 0; p < o.seal; p++) {
             neighbourhoodWordsKernel<true><<<wordGrid, kCloudBlock, 0, st>>>(src, cur, d, W);
@@ -1062,20 +1434,26 @@ int voxelizeCloud(vsim_cloud_volume* v, const CloudInput& in, const vsim_cloud_o
         seedFloodKernel<<<wordGrid, kCloudBlock, 0, st>>>(cur, d, W, emptyW, reachedW);
         // a warp per line, four to a block
         auto lineBlocks = [](uint64_t lines) { return uint32_t(std::max<uint64_t>(1, (lines + 3) / 4)); };
+        // Two rounds a look at the device: a grid seldom floods in one, and the
+        // look costs as much as half a round.
         bool converged = false;
         const uint32_t rounds = floodRounds.load();
-        for (uint32_t round = 0; round < rounds && !converged; round++) {
-            CK(cudaMemsetAsync(&sc->changed, 0, sizeof(uint32_t), st), "cloud flood");
-            sweepXKernel<<<uint32_t((W.rows + 127) / 128), 128, 0, st>>>(W, emptyW, reachedW, &sc->changed);
-            sweepLineKernel<<<lineBlocks(uint64_t(d.nz) * W.nw), 128, 0, st>>>(W, d.nz, d.ny, W.nw, W.nw * d.ny,
-                                                                                emptyW, reachedW, &sc->changed);
-            sweepLineKernel<<<lineBlocks(uint64_t(d.ny) * W.nw), 128, 0, st>>>(W, d.ny, d.nz, W.nw * d.ny, W.nw,
-                                                                                emptyW, reachedW, &sc->changed);
+        for (uint32_t round = 0; round < rounds && !converged; round += 2) {
+            const uint32_t now = std::min(2u, rounds - round);
+            CK(cudaMemsetAsync(sc->changed, 0, sizeof sc->changed, st), "cloud flood");
+            for (uint32_t r = 0; r < now; r++) {
+                sweepXKernel<<<uint32_t((W.rows + 127) / 128), 128, 0, st>>>(W, emptyW, reachedW, sc->changed + r);
+                sweepLineKernel<<<lineBlocks(uint64_t(d.nz) * W.nw), 128, 0, st>>>(
+                    W, d.nz, d.ny, W.nw, W.nw * d.ny, emptyW, reachedW, sc->changed + r);
+                sweepLineKernel<<<lineBlocks(uint64_t(d.ny) * W.nw), 128, 0, st>>>(
+                    W, d.ny, d.nz, W.nw * d.ny, W.nw, emptyW, reachedW, sc->changed + r);
+            }
             CK(cudaGetLastError(), "cloud flood");
-            uint32_t changed = 1;
-            CK(cudaMemcpyAsync(&changed, &sc->changed, sizeof changed, cudaMemcpyDeviceToHost, st), "cloud flood");
+            uint32_t changed[2] = {1, 1};
+            CK(cudaMemcpyAsync(changed, sc->changed, now * sizeof(uint32_t), cudaMemcpyDeviceToHost, st),
+               "cloud flood");
             CK(cudaStreamSynchronize(st), "cloud flood");
-            converged = changed == 0;
+            for (uint32_t r = 0; r < now; r++) converged |= changed[r] == 0;
         }
         if (converged) {
             encloseWordsKernel<<<wordGrid, kCloudBlock, 0, st>>>(cur, W, emptyW, reachedW, &sc->filled);
@@ -1107,7 +1485,9 @@ int voxelizeCloud(vsim_cloud_volume* v, const CloudInput& in, const vsim_cloud_o
         CK(cudaMemcpyAsync(&got, sc, sizeof got, cudaMemcpyDeviceToHost, st), "cloud fill");
         CK(cudaStreamSynchronize(st), "cloud fill");  // before the words are freed
     } else {
-        countKernel<<<grid, kCloudBlock, 0, st>>>(v->occupancy, n, &sc->occupied);
+        unpackCellsKernel<<<streamGrid((n + 15) / 16, sms), kCloudBlock, 0, st>>>(stampW, nullptr, d, W, v->occupancy,
+                                                                                   &sc->occupied);
+        CK(cudaGetLastError(), "cloud stamp");
         CK(cudaMemcpyAsync(&got, sc, sizeof got, cudaMemcpyDeviceToHost, st), "cloud stamp");
         CK(cudaStreamSynchronize(st), "cloud stamp");
     }

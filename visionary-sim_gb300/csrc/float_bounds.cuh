@@ -69,6 +69,32 @@ VSIM_BOUNDS_HD float reachEstimate(const float col[9], const float r[3], int a) 
     return std::sqrt(sum);
 }
 
+// The frame's entries in plain float, and what they may put a reach off by.
+// Off the diagonal 2 (a b +- c d) is three roundings of terms that sum to at
+// most Q / 2, Q = |q|^2; on it 1 - 2 (a a + b b) is one more, of at most 1 +
+// 2 Q; the reference's own float32 rounding adds 2^-24 of the entry: within
+// 2^-21 (1 + Q) of the entries it holds in all. A reach is the length of
+// (c_k r_k), so it moves by at most 2^-21 (1 + Q) (|r_0| + |r_1| + |r_2|);
+// reachSlack is twice that, its own roundings included. With an estimate hf
+// from such a frame
+//   hf (1 - kReachSlack) - slack <= reach <= hf (1 + kReachSlack) + slack.
+VSIM_BOUNDS_HD void frameInFloat(float x, float y, float z, float w, float col[9]) {
+    col[0] = 1.0f - 2.0f * (y * y + z * z);
+    col[1] = 2.0f * (x * y + z * w);
+    col[2] = 2.0f * (x * z - y * w);
+    col[3] = 2.0f * (x * y - z * w);
+    col[4] = 1.0f - 2.0f * (x * x + z * z);
+    col[5] = 2.0f * (y * z + x * w);
+    col[6] = 2.0f * (x * z + y * w);
+    col[7] = 2.0f * (y * z - x * w);
+    col[8] = 1.0f - 2.0f * (x * x + y * y);
+}
+
+VSIM_BOUNDS_HD float reachSlack(float x, float y, float z, float w, const float r[3]) {
+    const float q = x * x + y * y + z * z + w * w;
+    return 0x1p-20f * (1.0f + q) * (std::fabs(r[0]) + std::fabs(r[1]) + std::fabs(r[2]));
+}
+
 // A radius float(sigma) * scale for the estimate, NaN where out of its
 // range.
 VSIM_BOUNDS_HD float radiusEstimate(float sigmaF, float scale) {
@@ -85,21 +111,28 @@ VSIM_BOUNDS_HD float radiusEstimate(float sigmaF, float scale) {
 // magnitude, invH within 2^-24 of 1 / h, so e is within 5 2^-24 M of (c +
 // s - origin) / h, M = (|origin| + |c| + |co| + |s|) / h bounding every
 // magnitude in cells; the double path's quotient is within 3 2^-53 M of it
-// too. delta = 2^-20 M (plus 2^-100 for subnormal roundings) covers both,
-// and e and the double quotient are monotone in s, so one floor of e(s1) -
-// delta and e(s2) + delta is the floor of every x's quotient. False when
-// they differ or leave float's exact integers.
-VSIM_BOUNDS_HD bool floatCell(float co, float s1, float s2, float invH, float delta, int64_t& cell) {
+// too, and taking delta off rounds within 2^-24 M once more. delta = 2^-21 M
+// (plus 2^-100 for subnormal roundings) covers the 6 2^-24 M, its own
+// roundings included, and e and the double quotient are monotone in s, so
+// one floor of e(s1) - delta and e(s2) + delta is the floor of every x's
+// quotient. False when they differ or leave float's exact integers.
+VSIM_BOUNDS_HD bool floatCellAt(float co, float s1, float s2, float invH, float delta, float& cell) {
     const float a = std::floor((co + s1) * invH - delta), b = std::floor((co + s2) * invH + delta);
-    if (a != b || !(std::fabs(a) < 0x1p22f)) return false;
-    cell = int64_t(a);
+    cell = a;
+    return a == b && std::fabs(a) < 0x1p22f;
+}
+
+VSIM_BOUNDS_HD bool floatCell(float co, float s1, float s2, float invH, float delta, int64_t& cell) {
+    float at;
+    if (!floatCellAt(co, s1, s2, invH, delta, at)) return false;
+    cell = int64_t(at);
     return true;
 }
 
 // delta of floatCell for a position c and half-reach bound `wide` (0 for the
 // centre), with originMag = max(|float(origin)|, 2^-100).
 VSIM_BOUNDS_HD float cellDelta(float originMag, float c, float co, float wide, float invH) {
-    return 0x1p-20f * (originMag + std::fabs(c) + std::fabs(co) + wide) * invH + 0x1p-100f;
+    return 0x1p-21f * (originMag + std::fabs(c) + std::fabs(co) + wide) * invH + 0x1p-100f;
 }
 
 
@@ -292,6 +325,32 @@ VSIM_BOUNDS_HD int floatSample(const FloatTest& f, float ox, float oy, float oz)
     if (sum > 1.0f + bound) return 0;
     if (sum < 1.0f - bound) return 1;
     return -1;
+}
+
+// floatSample's answer where a bound that holds for every sample with a sum
+// of at most 4 decides it, else floatSample's own. Each of the bound's float
+// operations is monotone in |t|, so at |t| = 2 and a sum of 4 it is at least
+// floatSample's there; past 4, floatSample's bound (err is under 1e-3) is far
+// under the sum less 1.
+VSIM_BOUNDS_HD float quickBound(const FloatTest& f) {
+    float bound = 0.0f;
+    for (int a = 0; a < 3; a++) {
+        const float et = f.err[a] + 0x1p-21f * 2.0f;
+        bound += (2.0f * 2.0f + et) * et;
+    }
+    return bound + (0x1p-20f * 4.0f + 0x1p-20f);
+}
+
+VSIM_BOUNDS_HD int quickSample(const FloatTest& f, float quick, float ox, float oy, float oz) {
+    const float dx = f.base[0] + ox * f.h, dy = f.base[1] + oy * f.h, dz = f.base[2] + oz * f.h;
+    float sum = 0.0f;
+    for (int a = 0; a < 3; a++) {
+        const float t = (f.col[3 * a] * dx + f.col[3 * a + 1] * dy + f.col[3 * a + 2] * dz) * f.inv[a];
+        sum += t * t;
+    }
+    if (sum > 4.0f || sum > 1.0f + quick) return 0;
+    if (sum < 1.0f - quick) return 1;
+    return floatSample(f, ox, oy, oz);
 }
 
 }  // namespace bounds
