@@ -110,3 +110,27 @@ def test_chains_take_turns_and_bodies_sit_out(lib):
             assert np.array_equal(g, o), f"frame {frame}"
     mixed.destroy()
     plain.destroy()
+
+
+@pytest.mark.parametrize("factor", [0.3, 0.1, 0.02])
+def test_crowded_buckets_in_order(lib, factor):
+    """The five-launch chain's order of a crowded bucket: hundreds and
+    thousands of records in one, starting at any place of the order."""
+    import vsim.scenes as sc
+
+    scene = sc.noise_blob(n=20, seed=5, splats=0)
+    sim, orc = make(scene)
+    sim.set_gather_mapping("thread")
+    pos = orc.state()[0]
+    inside = orc.inv_mass() > 0
+    centre = pos[inside, :3].mean(axis=0)
+    squeezed = pos.copy()
+    squeezed[:, :3] = centre + (squeezed[:, :3] - centre) * np.float32(factor)
+    # some where they were, so that the crowd's run starts at an odd place
+    squeezed[::17] = pos[::17]
+    start(sim, orc, squeezed)
+    for frame in range(2):
+        sim.dispatch(scene.substeps)
+        orc.dispatch(scene.substeps)
+        same(sim, orc, f"factor {factor} frame {frame}")
+    sim.destroy()

@@ -185,7 +185,7 @@ __device__ __forceinline__ void runJob(const SessionJob& job, const SessionLaunc
                 sync();
                 ok = !failed();
                 for (uint32_t i = tid; ok && i < records; i += threads)
-                    canonRecord(first + i, ca, a.entries, a.sorted, a.pos, a.prev);
+                    canonRecord<false>(first + i, ca, a.entries, a.sorted, a.pos, a.prev);
                 sync();
                 // The gather over the session's entries in bucket order.
                 if (ok && records <= L.warpRecords * (threads >> 5)) {

@@ -377,7 +377,7 @@ __global__ void canonKernel(const FrameParams* __restrict__ fp, Work work, const
     const SortedEntries out{sMeta, sPos, sMoved, sRec, sKey};
     forEachItem(work, [&](uint32_t r) {
         if (key[r] == kIdle) return;
-        canonRecord(r, arrays, entries, out, pos, prevState);
+        canonRecord<true>(r, arrays, entries, out, pos, prevState);
     });
 }
 
