@@ -179,10 +179,11 @@ def replica_throughput(local_seconds: float, units_per_rank: int, device):
 
 
 def colour_pass_rate(sim, sweeps: int = 10):
-    """The elastic colour pass timed as the frame runs it: `sweeps` x 8
-    passes back to back in one graph (programmatic dependent launch), events
-    at the two ends only (vsim_time_colour_passes; state restored). Returns
-    (algorithmic bytes per launch, average launch seconds)."""
+    """The elastic passes timed as the frame runs them: `sweeps` sweeps of the
+    eight colours (two to a launch where rows are packed) back to back in one
+    graph (programmatic dependent launch), events at the two ends only
+    (vsim_time_colour_passes; state restored). Returns (algorithmic bytes per
+    colour, average seconds a colour)."""
     counts = sim.color_counts()
     passes = sweeps * int(np.count_nonzero(counts))
     ms = sim.time_colour_passes(sweeps)
@@ -190,10 +191,11 @@ def colour_pass_rate(sim, sweeps: int = 10):
 
 
 def roofline(sim, scene, hbm):
-    """The dominant kernel's roofline: the elastic colour pass. `achieved` is
-    algorithmic bytes per launch over the average launch time with the passes
-    back to back as in the frame; `isolated_launch_us` is one launch
-    bracketed by events on its own (no overlap with its neighbours)."""
+    """The dominant kernel's roofline: the elastic passes, per colour.
+    `achieved` is algorithmic bytes per colour over the average time a colour
+    with the passes back to back as in the frame; `isolated_launch_us` is a
+    colour's share of launches bracketed by events on their own (no overlap
+    with their neighbours)."""
     prof = sim.profile_frame(scene.substeps, splats=True, view_dir=VIEW)
     ms, launches = prof["elastic"]
     per_launch_bytes, per_launch_s = colour_pass_rate(sim)
@@ -206,7 +208,7 @@ def roofline(sim, scene, hbm):
     share = {k: round(v[0] / sum(x[0] for x in prof.values()), 4) for k, v in prof.items()}
     return {
         "bound": "hbm",
-        "kernel": "elasticKernel (one colour pass)",
+        "kernel": "elasticRowKernel (two colours a launch; figures are per colour)",
         "achieved": round(achieved, 1),
         "peak": hbm,
         "unit": "GB/s",
@@ -216,7 +218,7 @@ def roofline(sim, scene, hbm):
         "avg_launch_us": round(per_launch_s * 1e6, 3),
         "isolated_launch_us": round(1e3 * ms / (scene.substeps * scene.iterations *
                                                  int(np.count_nonzero(sim.color_counts()))), 3),
-        "method": "10 sweeps x 8 colour passes back to back in one graph, CUDA events at its ends",
+        "method": "10 sweeps of the 8 colours back to back in one graph, CUDA events at its ends",
         "four_lanes_a_cell_launch_us": round(quad_s * 1e6, 3),
     }, {k: {"ms": round(v[0], 4), "launches": v[1]} for k, v in prof.items()}, share
 
@@ -530,7 +532,7 @@ def stress(quick: bool, hbm: float, frames: int = 3):
            "elastic_pass": {"achieved_gbs": round(achieved, 1), "frac_of_measured_hbm": round(achieved / hbm, 4),
                             "bytes_per_launch": round(per_launch), "avg_launch_us": round(per_launch_s * 1e6, 2),
                             "isolated_launch_us": round(1e3 * ms / launches, 2),
-                            "method": "10 sweeps x 8 colour passes back to back in one graph"},
+                            "method": "10 sweeps of the 8 colours back to back in one graph"},
            "single_body_elastic_pass": single_body_pass(quick, hbm),
            "splat_deform_gbs": round(92 * n_splats / (splat_ms / 1e3) / 1e9, 1) if splat_ms else None,
            "sort_keys_per_s": round(n_splats / (sort_ms / 1e3)) if sort_ms else None,

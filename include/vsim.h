@@ -263,7 +263,10 @@ int vsim_set_iterations(vsim_sim* sim, uint32_t iterations);
 int vsim_set_graph(vsim_sim* sim, int enabled);
 /* Threads per block of the elastic colour pass (128, 256 or 512) and the
    cell order inside each colour (0: lattice order, 4 or 8: bricks of that
-   many cells per axis). Chosen by vsim_tune; settable for sweeps. */
+   many cells per axis). Chosen by vsim_tune; settable for sweeps. Frames
+   whose cells are solved row by row, two colours a launch (scenes with no
+   run of cells along x over 256 long, none of the forms below asked for),
+   read neither. */
 int vsim_set_launch_shape(vsim_sim* sim, uint32_t block, uint32_t brick);
 /* The large colour passes (a dense pass of at least two cells per resident
    thread) through tensor-memory-accelerator brick tiles: each block takes
@@ -289,11 +292,14 @@ int vsim_tune(vsim_sim* sim, uint32_t frames, uint32_t* block, uint32_t* brick);
    on): the next kernel's launch overlaps the tail of the one before it. */
 int vsim_set_pdl(vsim_sim* sim, int enabled);
 
-/* How the contact gather maps surface records to GPU threads: AUTO (default)
-   gives each record a warp while the substep has fewer than 2048 records
-   per SM and a thread otherwise; WARP and THREAD force one mapping. All three
-   give the same results (each record's hits are summed in the reference's
-   order); the setting exists for tests and sweeps. No reference counterpart. */
+/* How the contact gather maps surface records to GPU threads. AUTO (default)
+   bins a whole scene's records into bucket slots and gives each record nine
+   lanes; where bodies are isolated it orders the records by bucket and gives
+   each a warp while the substep has fewer than 2048 records per SM and a
+   thread otherwise. WARP and THREAD order them by bucket and force one
+   mapping. All give the same results (each record's hits are summed in the
+   reference's order); the setting exists for tests and sweeps. No reference
+   counterpart. */
 #define VSIM_GATHER_AUTO 0
 #define VSIM_GATHER_WARP 1
 #define VSIM_GATHER_THREAD 2
@@ -344,9 +350,9 @@ int vsim_contact_surface(vsim_sim* sim, uint32_t* nodes, uint32_t* bodies, size_
 /* Kernel groups a frame is made of. */
 #define VSIM_KIND_PREDICT 0
 #define VSIM_KIND_DRIVE 1     /* unused: the drive runs inside the pass that predicts each substep */
-#define VSIM_KIND_ELASTIC 2   /* the colour passes */
+#define VSIM_KIND_ELASTIC 2   /* the colour passes, or the row passes (two colours each) */
 #define VSIM_KIND_LIMIT 3     /* limit-only stretch sweeps */
-#define VSIM_KIND_CONTACT 4   /* bin, segment, scatter, order, collide, settle */
+#define VSIM_KIND_CONTACT 4   /* bin and gather; or bin, segment, scatter, order, collide, settle */
 #define VSIM_KIND_FINALIZE 5
 #define VSIM_KIND_SPLAT 6     /* splat deformation */
 #define VSIM_KIND_SORT 7      /* splat depth sort */
@@ -363,8 +369,9 @@ typedef struct vsim_profile {
    kernel group. The frame advances the simulation like vsim_dispatch. */
 int vsim_profile_frame(vsim_sim* sim, uint32_t steps, int with_splats, const float view_dir[3],
                        vsim_profile* out);
-/* Time `sweeps` Gauss-Seidel sweeps of the elastic colour passes (8 passes
-   each, the frame's launch shapes) run back to back as one captured graph,
+/* Time `sweeps` Gauss-Seidel sweeps of the elastic colour passes (each all
+   eight colours, in the frame's own launches: four row passes or eight colour
+   passes) run back to back as one captured graph,
    with events only at its two ends; *ms receives the total. The positions
    the passes move are saved first and restored after, so the state is
    unchanged. For roofline measurement: the bracketed launches in

@@ -103,3 +103,37 @@ def test_many_groups(lib, rows, stretch):
     scene = scene_of(rows, 0.15, seed=8, stretch=stretch)
     scene.substeps = 2
     run(scene, strained(scene, amount=0.1), frames=1)
+
+
+@pytest.mark.parametrize("longest", [40, 256, 257])
+@pytest.mark.parametrize("stretch", [0.0, 1.05])
+def test_rows_of_sessions_in_ticks(lib, longest, stretch):
+    """Sessions stepped in shared frames, some of them at a time: each body's
+    groups are its own, and a body with a run of 257 cells sends all of them
+    the colours' way."""
+    import pyoracle
+    import vsim.scenes as sc
+    from vsim.server import Server
+
+    rng = np.random.default_rng(longest)
+    bodies = []
+    for dims in ((1, 1, 1), (3, 2, 1), (longest, 2, 3), (9, 7, 5), (130, 3, 2), (2, 40, 3)):
+        occ = (rng.random(np.prod(dims)) >= 0.15).astype(np.uint8)
+        occ[: dims[0]] = 1
+        bodies.append(sc.Body(dims, (0.0, 0.02, 0.0), sc.H, occ, dict(sc.DEFAULT_MATERIAL, max_stretch=stretch)))
+    tank = ((-1.0, 0.0, -1.0), (6.0, 3.0, 6.0))
+    server = Server(bodies, tank)
+    frames = [2, 1, 3, 2, 0, 3]
+    for b, n in enumerate(frames):
+        if n:
+            server.submit(b, n, None)
+    while server.stats()["pending"]:
+        server.tick()
+        server.poll()
+    for b, n in enumerate(frames):
+        orc = pyoracle.Oracle(sc.Scene([bodies[b]], tank, step_duration=1 / 600, substeps=10, contact=True,
+                                       self_contact=True, isolated=True), 32)
+        for _ in range(n):
+            orc.dispatch(10)
+        assert np.array_equal(server.read_positions(b), orc.state()[0]), f"session {b}"
+    server.destroy()

@@ -68,10 +68,11 @@ struct Work {
 };
 
 // Spans of a frame: the active nodes, the eight colours' cells, the surface
-// records.
-constexpr uint32_t kSpans = 10;
+// records, the four row passes' groups (a chunk each).
+constexpr uint32_t kSpans = 14;
 constexpr uint32_t kNodeSpan = 0, kRecordSpan = 9;
 constexpr uint32_t colourSpan(int c) { return 1 + uint32_t(c); }
+constexpr uint32_t rowSpan(uint32_t pass) { return 10 + pass; }
 
 // Calls f(item) for each item of `w` this thread owns.
 template <class F>
@@ -210,6 +211,10 @@ constexpr uint32_t rowFields(uint32_t stride, uint32_t nearOdd, uint32_t farOdd)
 enum class RowWork { kProject, kBoth, kLimit };
 cudaError_t launchElasticRows(const LaunchCtx& c, const DeviceState& s, const uint4* groups, uint32_t count,
                               RowWork work, const StretchLengths& lens);
+// The groups a chunked frame's table lists for one row pass.
+cudaError_t launchElasticRowChunks(const LaunchCtx& c, const DeviceState& s, const Span& span, RowWork work,
+                                   const StretchLengths& lens);
+constexpr uint32_t kRowChunksPerSm = 3;  // blocks of it an SM holds
 
 // A whole frame of a small scene without contact in one launch (small_frame.cu):
 // every row pass at most one group, at most kSmallNodes nodes.

@@ -208,7 +208,8 @@ int uploadCells(vsim_sim* s, bool again) {
 }
 
 // The row passes' groups (kRowBlock), pass by pass (y and z parity), bodies in
-// order and rows in lattice order inside each. False when some run of cells
+// order and rows in lattice order inside each; a group of isolated bodies
+// holds one body's. False when some run of cells
 // does not fit a group.
 bool buildRows(vsim_sim* s, std::vector<uint4>& out) {
     out.clear();
@@ -216,9 +217,14 @@ bool buildRows(vsim_sim* s, std::vector<uint4>& out) {
     for (uint32_t pass = 0; pass < kRowPasses; pass++) {
         s->rowStart[pass] = uint32_t(out.size() / kRowGroup);
         uint32_t evens = kRowBlock, odds = kRowBlock;  // cells in the open group; full: none open
+        s->rowBodyStart[pass].clear();
         for (size_t b = 0; b < s->lat.size(); b++) {
             const Lattice& L = s->lat[b];
             const uint32_t nx = L.nodeDims[0], nxy = nx * L.nodeDims[1], cx = L.cellDims[0];
+            if (s->isolated) {
+                s->rowBodyStart[pass].push_back(uint32_t(out.size() / kRowGroup));
+                evens = odds = kRowBlock;
+            }
             for (uint32_t k = pass >> 1; k < L.cellDims[2]; k += 2)
                 for (uint32_t j = pass & 1; j < L.cellDims[1]; j += 2) {
                     const uint8_t* row = L.occupancy.data() + size_t(cx) * (j + size_t(L.cellDims[1]) * k);
@@ -251,10 +257,14 @@ bool buildRows(vsim_sim* s, std::vector<uint4>& out) {
                     }
                 }
         }
+        if (s->isolated) s->rowBodyStart[pass].push_back(uint32_t(out.size() / kRowGroup));
     }
     s->rowStart[kRowPasses] = uint32_t(out.size() / kRowGroup);
     return true;
 }
+
+// Whether the frame's elastic passes run as row passes (two colours each).
+bool inRows(const vsim_sim* s) { return s->rowPasses && !s->tma.enabled && !s->quadCells; }
 
 // Spans over every body.
 void buildDensePlan(vsim_sim* s) {
@@ -288,7 +298,21 @@ int planBodies(vsim_sim* s, const std::vector<uint32_t>& bodies) {
     // The staging may still feed the previous frame's upload.
     CK(cudaStreamSynchronize(s->stream), "upload work chunks");
     bool ok = emit(kNodeSpan, s->nodeBodyStart);
-    for (int c = 0; c < 8 && ok; c++) ok = emit(colourSpan(c), s->colourBodyStart[c]);
+    const bool rows = inRows(s);
+    for (int c = 0; c < 8 && ok; c++) {
+        if (rows) table[colourSpan(c)] = make_uint2(0, 0);
+        else ok = emit(colourSpan(c), s->colourBodyStart[c]);
+    }
+    for (uint32_t q = 0; q < kRowPasses && ok; q++) {
+        const size_t first = at;
+        if (rows)
+            for (uint32_t b : bodies)
+                for (uint32_t g = s->rowBodyStart[q][b]; ok && g < s->rowBodyStart[q][b + 1]; g++) {
+                    ok = at < s->chunkCapacity;
+                    if (ok) chunks[at++] = make_uint2(g, 1);
+                }
+        table[rowSpan(q)] = make_uint2(uint32_t(first), uint32_t(at - first));
+    }
     ok = ok && emit(kRecordSpan, s->recordBodyStart);
     if (!ok) return fail(VSIM_ERR_CAPACITY, "chunk table too small (a body listed twice?)");
     CK(cudaMemcpyAsync(s->chunkDev, table, (kSpans + at) * sizeof(uint2), cudaMemcpyHostToDevice, s->stream),
@@ -352,9 +376,6 @@ cudaError_t launchColourPass(const LaunchCtx& c, const vsim_sim* s, int col, boo
     return launchElastic(c, s->d, s->d.cells + s->colorStart[col], sp, limitOnly, lens);
 }
 
-// Whether the frame's elastic passes run as row passes (two colours each).
-bool inRows(const vsim_sim* s) { return s->rowPasses && !s->plan.chunked && !s->tma.enabled && !s->quadCells; }
-
 // One sweep over the eight colours, as four row passes or eight colour
 // passes; each(launch) is called for every pass that has cells.
 template <class Each>
@@ -364,7 +385,9 @@ cudaError_t forEachPass(const LaunchCtx& c, const vsim_sim* s, bool limitOnly, c
         const RowWork work = limitOnly ? RowWork::kLimit : anyStretch(s) ? RowWork::kBoth : RowWork::kProject;
         for (uint32_t q = 0; q < kRowPasses && !e; q++) {
             const uint32_t groups = s->rowStart[q + 1] - s->rowStart[q];
-            if (groups)
+            if (s->plan.chunked && groups)
+                e = each([&] { return launchElasticRowChunks(c, s->d, s->plan.rows[q], work, lens); });
+            else if (groups)
                 e = each([&] {
                     return launchElasticRows(c, s->d, s->d.rows + size_t(s->rowStart[q]) * kRowGroup, groups, work, lens);
                 });
@@ -384,7 +407,7 @@ bool contactMatters(const vsim_sim* s) {
 
 // Whether the frame runs in one launch (small_frame.cu).
 bool inOneLaunch(const vsim_sim* s) {
-    if (!inRows(s) || contactMatters(s) || s->nodeCount > kSmallNodes) return false;
+    if (!inRows(s) || s->isolated || contactMatters(s) || s->nodeCount > kSmallNodes) return false;
     for (uint32_t q = 0; q < kRowPasses; q++)
         if (s->rowStart[q + 1] - s->rowStart[q] > 1) return false;
     return true;
@@ -747,8 +770,15 @@ int createSim(const vsim_body_desc* bodies, uint32_t n, const vsim_tank* tank, v
     countCells(s);
     buildDensePlan(s);
     useDensePlan(s);
-    // Isolated bodies step in chunked frames, which take the colours one by one.
-    if (!isolated && buildRows(s, rows)) {
+    // Isolated bodies' cells go to the session kernel too, and their pool is
+    // sized without the groups: those are built where they take little of
+    // what memory is left.
+    size_t freeBytes = ~size_t(0), allBytes = 0;
+    if (isolated) {
+        if (int rc = uploadCells(s, false)) return rc;
+        CK(cudaMemGetInfo(&freeBytes, &allBytes), "memory left");
+    }
+    if (buildRows(s, rows) && rows.size() * 16 <= freeBytes / 8) {
         s->rowPasses = true;
         CK(allocN(&d.rows, rows.size()), "allocate rows");
         CK(cudaMemcpyAsync(d.rows, rows.data(), rows.size() * 16, cudaMemcpyHostToDevice, s->stream), "upload rows");
@@ -772,11 +802,17 @@ int createSim(const vsim_body_desc* bodies, uint32_t n, const vsim_tank* tank, v
         p.nodes = span(kNodeSpan, s->nodeBodyStart, 16);
         for (int c = 0; c < 8; c++) p.colour[c] = span(colourSpan(c), s->colourBodyStart[c], 4);
         p.records = span(kRecordSpan, s->recordBodyStart, 16);
+        for (uint32_t q = 0; s->rowPasses && q < kRowPasses; q++) {
+            const uint32_t most = s->rowStart[q + 1] - s->rowStart[q];
+            chunks += most;
+            p.rows[q] = Span{Work{nullptr, rowSpan(q), 0}, std::min(most, kRowChunksPerSm * uint32_t(s->sms)), kRowBlock};
+        }
         s->chunkCapacity = chunks;
         CK(allocN(&s->chunkDev, kSpans + chunks), "allocate work chunks");
         CK(cudaMallocHost(&s->chunkPinned, (kSpans + chunks) * sizeof(uint2)), "allocate staging");
         p.nodes.work.table = s->chunkDev;
         for (int c = 0; c < 8; c++) p.colour[c].work.table = s->chunkDev;
+        for (Span& r : p.rows) r.work.table = s->chunkDev;
         p.records.work.table = s->chunkDev;
     }
     std::vector<int32_t> nodeRecord(N, -1);

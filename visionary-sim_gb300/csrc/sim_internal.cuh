@@ -51,6 +51,7 @@ struct FramePlan {
     Span nodes{};
     Span colour[8]{};
     Span records{};
+    Span rows[kRowPasses]{};  // chunked frames: the row passes' groups
 };
 
 }  // namespace vsim
@@ -74,6 +75,9 @@ struct vsim_sim {
     uint32_t colorStart[9] = {};
     bool rowPasses = false;  // the row passes' groups are built (every run of cells fits one)
     uint32_t rowStart[vsim::kRowPasses + 1] = {};  // first group of each row pass
+    // isolated bodies: the first group of each body in each pass (groups hold
+    // one body's cells)
+    std::vector<uint32_t> rowBodyStart[vsim::kRowPasses];
     std::vector<uint4> surfHost;
     vsim_tank tank{};
     // Contact grids: one shared by all bodies, or one per body when the

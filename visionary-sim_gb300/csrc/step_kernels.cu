@@ -158,6 +158,33 @@ __global__ void __launch_bounds__(kRowBlock, EARLY ? 3 : 2) elasticRowKernel(con
         });
 }
 
+// The row pass over the groups a chunked frame's table lists, blocks taking
+// them in turn: a frame of a few sessions is a chain of short launches, and
+// this halves the elastic ones. Ten sessions of 5,000 to 40,000 cells: 8.4 us
+// for two colours, 6.5 each one by one; a one-frame request of a 5,364-cell
+// session 0.46 ms against 0.55.
+template <RowWork WORK>
+__global__ void __launch_bounds__(kRowBlock, kRowChunksPerSm) elasticRowChunksKernel(
+    const uint4* __restrict__ groups, Work work, const DevBody* __restrict__ bodies,
+    const uint32_t* __restrict__ bodyActive, float4* __restrict__ pos, const float4* __restrict__ prevState,
+    StretchLengths lens) {
+    __shared__ RowShared shared;
+    const uint2 d = work.table[work.span];
+    bool waited = false;
+    auto ready = [&] {
+        if (waited) return;
+        waited = true;
+        pdlWait();
+        pdlLaunchNext();
+    };
+    for (uint32_t c = blockIdx.x; c < d.y; c += gridDim.x) {
+        if (c != blockIdx.x) __syncthreads();  // the group before is out of shared memory
+        rowGroup(groups + size_t(work.table[kSpans + d.x + c].x) * kRowGroup, bodies, bodyActive, pos, prevState, lens,
+                 WORK != RowWork::kLimit, WORK != RowWork::kProject, shared, ready, [] {});
+    }
+    ready();  // a block without a group still follows the kernel before
+}
+
 // The colour pass for passes much larger than the GPU: each thread solves
 // cells in turn (grid-stride) and copies the next cell's eight positions and
 // eight previous positions into its slots of shared memory (cp.async) while
@@ -873,6 +900,17 @@ cudaError_t launchElasticRows(const LaunchCtx& c, const DeviceState& s, const ui
         default:
             return early ? go(elasticRowKernel<RowWork::kLimit, true>) : go(elasticRowKernel<RowWork::kLimit, false>);
     }
+}
+
+cudaError_t launchElasticRowChunks(const LaunchCtx& c, const DeviceState& s, const Span& span, RowWork work,
+                                   const StretchLengths& lens) {
+    auto go = [&](auto kernel) {
+        return launch(c, kernel, span.grid, span.block, (const uint4*)s.rows, span.work, (const DevBody*)s.bodies,
+                      (const uint32_t*)s.bodyActive, s.pos, (const float4*)s.prev, lens);
+    };
+    return work == RowWork::kProject ? go(elasticRowChunksKernel<RowWork::kProject>)
+           : work == RowWork::kBoth  ? go(elasticRowChunksKernel<RowWork::kBoth>)
+                                     : go(elasticRowChunksKernel<RowWork::kLimit>);
 }
 
 cudaError_t launchFinalize(const LaunchCtx& c, const DeviceState& s, const Span& n, bool contact, bool predictNext,

@@ -349,7 +349,7 @@ class Simulator:
         return {k: (prof.ms[i], prof.launches[i]) for i, k in enumerate(_ffi.KINDS) if prof.launches[i]}
 
     def time_colour_passes(self, sweeps: int) -> float:
-        """Milliseconds for `sweeps` x 8 colour passes run back to back
+        """Milliseconds for `sweeps` sweeps of the eight colours run back to back
         (vsim_time_colour_passes); the state is left unchanged."""
         ms = C.c_float()
         check(lib().vsim_time_colour_passes(self._h, int(sweeps), C.byref(ms)))
