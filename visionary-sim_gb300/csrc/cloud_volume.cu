@@ -348,38 +348,58 @@ struct CellBox {
     }
 };
 
-// cloudVolume.js:170-173 for one cell of a box: any sample inside. The double
-// frame is rebuilt only for a sample the float test cannot call.
+// A cell's sample, number s of nine, in its box's cells.
+__device__ __forceinline__ int floatSampleOf(const FloatTest& f, float quick, float fi, float fj, float fk, int s) {
+    const float ox = s == 8 ? 0.5f : float(s & 1), oy = s == 8 ? 0.5f : float((s >> 1) & 1);
+    const float oz = s == 8 ? 0.5f : float((s >> 2) & 1);
+    return quickSample(f, quick, fi + ox, fj + oy, fk + oz);
+}
+
+// Whether any sample of a cell from number s on is inside: s in double, and
+// those after it that the float test (null: none) cannot call.
+__device__ __noinline__ bool exactFrom(const CloudInput& in, uint32_t gaussian, const GridView& g, const int64_t* lo,
+                                       int64_t i, int64_t j, int64_t k, int s, const FloatTest* f, float quick) {
+    Ellipsoid e;
+    frameOf(in, gaussian, e);
+    double c[3];
+    for (int a = 0; a < 3; a++) c[a] = in.pos[3 * size_t(gaussian) + a];
+    const float fi = float(int32_t(i - lo[0])), fj = float(int32_t(j - lo[1])), fk = float(int32_t(k - lo[2]));
+    if (sampleInside(g, i, j, k, s, c, e)) return true;
+    for (s++; s < 9; s++) {
+        int inside = f ? floatSampleOf(*f, quick, fi, fj, fk, s) : -1;
+        if (inside < 0) inside = sampleInside(g, i, j, k, s, c, e) ? 1 : 0;
+        if (inside) return true;
+    }
+    return false;
+}
+
+// cloudVolume.js:170-173 for one cell of a box: any sample inside. What the
+// float test cannot call (one sample in 10^5) is decided out of line: the
+// double code would take the registers of half the warps.
 //
 // The float path converts nothing from double or 64-bit integers: on this
 // part such conversions run on the FP64 pipe, and nine samples a cell made
 // them the stamp's bottleneck. The cell's place in its box (under 2^20, so
 // exact) is an int32 turned float once; the sample offsets are float
 // constants.
-__device__ bool cellReached(const CloudInput& in, uint32_t gaussian, const GridView& g, const int64_t lo[3], int64_t i,
-                            int64_t j, int64_t k, const FloatTest* f, float quick) {
-    Ellipsoid e;
-    double c[3];
-    bool haveFrame = false;
+__device__ __forceinline__ bool cellReached(const CloudInput& in, uint32_t gaussian, const GridView& g,
+                                            const int64_t lo[3], int64_t i, int64_t j, int64_t k, const FloatTest* f,
+                                            float quick) {
+    if (!f) return exactFrom(in, gaussian, g, lo, i, j, k, 0, nullptr, quick);
     const float fi = float(int32_t(i - lo[0])), fj = float(int32_t(j - lo[1])), fk = float(int32_t(k - lo[2]));
+    int undecided = -1;
+    bool reached = false;
 #pragma unroll
     for (int s = 0; s < 9; s++) {
-        const float ox = s == 8 ? 0.5f : float(s & 1), oy = s == 8 ? 0.5f : float((s >> 1) & 1);
-        const float oz = s == 8 ? 0.5f : float((s >> 2) & 1);
-        int inside = -1;
-        if (f) inside = quickSample(*f, quick, fi + ox, fj + oy, fk + oz);
-        if (inside < 0) {
-            if (!haveFrame) {
-                frameOf(in, gaussian, e);
-                for (int a = 0; a < 3; a++) c[a] = in.pos[3 * size_t(gaussian) + a];
-                haveFrame = true;
-            }
-            inside = sampleInside(g, i, j, k, s, c, e) ? 1 : 0;
-        }
-        if (inside) return true;
+        const int inside = floatSampleOf(*f, quick, fi, fj, fk, s);
+        if (inside == 0) continue;
+        reached = inside > 0;
+        if (inside < 0) undecided = s;
+        break;
     }
-    return false;
+    return undecided < 0 ? reached : exactFrom(in, gaussian, g, lo, i, j, k, undecided, f, quick);
 }
+
 
 // Whether the float cells hold for a position on axis a (ranges that keep
 // every term above a normal float's floor and below overflow).
@@ -567,9 +587,11 @@ __device__ __forceinline__ uint32_t setBit(unsigned long long word, uint32_t n) 
 // Marking is an OR: which lane tests a cell, and when, changes nothing; a cell
 // that another marks meanwhile is tested for nothing.
 //
-// Instructions bound it, 985 a warp of Gaussians (2M at 231 x 223 x 243 cells:
-// 142 us, where setting every Gaussian up and walking bytes of all its cells
-// took 405; with a brick's words read one after another 258). One wave of
+// Its schedulers issue 0.56 of the time with the 26 warps an SM that its
+// registers allow, waiting for the bricks' words (L2, at no two lanes' same
+// place) the rest (2M Gaussians at 231 x 223 x 243 cells: 142 us, where setting
+// every Gaussian up and walking bytes of all its cells took 405; with a
+// brick's words read one after another 258). One wave of
 // blocks: two of half as many rounds each take 20 us more, since the first
 // rounds know the fewest marks.
 //
@@ -579,7 +601,8 @@ __device__ __forceinline__ uint32_t setBit(unsigned long long word, uint32_t n) 
 // listed, and a second launch, HARD, takes
 // them together.
 template <bool HARD>
-__global__ void __launch_bounds__(kStampBlock, HARD ? 4 : kStampBlocks) cloudStampKernel(CloudInput in, GridView g,
+__global__ void __launch_bounds__(kStampBlock, HARD ? 4 : kStampBlocks) cloudStampKernel(const __grid_constant__ CloudInput in,
+                                                                const __grid_constant__ GridView g,
                                                                 const float4* __restrict__ reach, Bricks bricks,
                                                                 uint32_t rounds, HardList hard,
                                                                 uint32_t* __restrict__ big,
@@ -744,11 +767,16 @@ __global__ void __launch_bounds__(kStampBlock, HARD ? 4 : kStampBlocks) cloudSta
 // The listed larger boxes, several to a block: one thread sets each up, then
 // the block's warps walk the bricks of all of them, a brick's 64 cells two to
 // a lane, and mark a brick by one OR. A brick with no empty cell of the box
-// costs one read.
+// costs one read. Four blocks an SM (64 registers) against two with the exact
+// samples inline (110): 20,000 Gaussians of 1,300 cells' boxes, a whole
+// voxelisation 1,125 us with a block a box and byte cells, 1,175 with bricks
+// at two blocks, 908 at four.
 constexpr uint32_t kBoxThreads = 256;
+constexpr uint32_t kBoxBlocks = 4;  // an SM
 constexpr uint32_t kBoxBatch = kBoxThreads / 32;
 
-__global__ void __launch_bounds__(kBoxThreads) cloudStampBoxKernel(CloudInput in, GridView g,
+__global__ void __launch_bounds__(kBoxThreads, kBoxBlocks) cloudStampBoxKernel(const __grid_constant__ CloudInput in,
+                                                                   const __grid_constant__ GridView g,
                                                                    const float4* __restrict__ reach, Bricks bricks,
                                                                    const uint32_t* __restrict__ big,
                                                                    const unsigned long long* __restrict__ bigCount) {
@@ -1401,9 +1429,10 @@ int voxelizeCloud(vsim_cloud_volume* v, const CloudInput& in, const vsim_cloud_o
         const uint64_t each = uint64_t(rounds) * kStampBlock;
         cloudStampKernel<false><<<uint32_t((in.count + each - 1) / each), kStampBlock, 0, st>>>(
             in, g, reach, bricks, rounds, hard, big, &sc->bigCount);
-        cloudStampKernel<true><<<uint32_t(sms) * 8, kStampBlock, 0, st>>>(in, g, reach, bricks, 0, hard, big,
+        // The last two on as many blocks as fit at their registers: they loop.
+        cloudStampKernel<true><<<uint32_t(sms) * 4, kStampBlock, 0, st>>>(in, g, reach, bricks, 0, hard, big,
                                                                            &sc->bigCount);
-        cloudStampBoxKernel<<<uint32_t(sms) * 8, kBoxThreads, 0, st>>>(in, g, reach, bricks, big, &sc->bigCount);
+        cloudStampBoxKernel<<<uint32_t(sms) * kBoxBlocks, kBoxThreads, 0, st>>>(in, g, reach, bricks, big, &sc->bigCount);
     }
     POOL_ALLOC(wordsBuf, words * (o.fill ? 5 : 1) * sizeof(uint32_t), pool, st, "cloud scratch");
     uint32_t* stampW = static_cast<uint32_t*>(wordsBuf.p);
