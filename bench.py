@@ -243,6 +243,7 @@ def contact_roofline(sim, hbm):
     the per-surface-node formula (key 8 B, an 8 B read+write per sort pass --
     here 4 passes: bin, segment, scatter, order -- the 27 buckets' 8 B, 36 B
     per candidate, 32 B to apply)."""
+    sim.contact_census()  # the chain's kernels loaded: frames run another
     c = sim.contact_census()
     r, b, k = c["records"], c["occupied_buckets"], c["candidates"]
     per = {}
