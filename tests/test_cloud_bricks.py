@@ -66,6 +66,16 @@ def test_out_of_float_range(vz, cells):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("thin", [0.0, 1e-7, 1e-5])
+@pytest.mark.parametrize("cells", [1.0, 7.0])
+def test_surfels(vz, cells, thin):
+    # an axis of no or next to no thickness: every sample goes to double
+    pos, rot, scale = _cloud(300, 0.05, 0.004 * cells, seed=12)
+    scale[::2, 1] = thin
+    _same(vz, (pos, rot, scale), 0.004)
+
+
+@pytest.mark.gpu
 def test_rotations_off_a_boundary(vz):
     import torch
 

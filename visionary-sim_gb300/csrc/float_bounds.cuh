@@ -170,9 +170,10 @@ struct Ellipsoid {
 // order, then its centre) tested against the ellipsoid in the reference's
 // double arithmetic and order (cloudVolume.js:255-273).
 VSIM_BOUNDS_HD void sampleOffset(int s, double& ox, double& oy, double& oz) {
-    ox = s == 8 ? 0.5 : double(s & 1);
-    oy = s == 8 ? 0.5 : double((s >> 1) & 1);
-    oz = s == 8 ? 0.5 : double((s >> 2) & 1);
+    // by selects: a conversion runs on the double pipe
+    ox = s == 8 ? 0.5 : (s & 1) ? 1.0 : 0.0;
+    oy = s == 8 ? 0.5 : (s & 2) ? 1.0 : 0.0;
+    oz = s == 8 ? 0.5 : (s & 4) ? 1.0 : 0.0;
 }
 
 VSIM_BOUNDS_HD bool sampleInside(const GridView& g, int64_t i, int64_t j, int64_t k, int s, const double c[3],
