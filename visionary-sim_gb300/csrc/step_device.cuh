@@ -203,7 +203,8 @@ __device__ __forceinline__ float2 weighted4(float w0, float w1, float w2, float 
 // again and again, misses on every line (two inlined projections in a loop:
 // 4,340 cycles each). The reference's two
 // early outs need no branch: a weightless tetrahedron moves nothing, and a
-// determinant under 1e-20 is outside the ranges. Corner 0's gradients are
+// determinant under 1e-20, a negative one with it (stiff bodies near rest,
+// where the gradients are parallel but for roundings), is outside the ranges. Corner 0's gradients are
 // minus the sum of the others'; the sum is kept and the sign moved to where
 // it is used, which rounds the same.
 template <int t, class Prev>
@@ -239,7 +240,7 @@ __device__ __forceinline__ void projectTetInRange(V (&p)[8], Prev&& prev, const 
     const float r = rounded::reciprocal(k.det, rounded::approxReciprocal(k.det));
     const float lx = rounded::quotient(k.nx, k.det, r);
     const float ly = rounded::quotient(k.ny, k.det, r);
-    ranges.arguments(square, k.det);
+    ranges.argumentAndPositive(square, k.det);
     ranges.quotients(lx, ly);
     p[i0] = moved(p[i0], minus0.dev(), minus0.hyd(), lx, ly, -w0);
     p[i1] = moved(p[i1], g1.dev(), g1.hyd(), lx, ly, w1);
