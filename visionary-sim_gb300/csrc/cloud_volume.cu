@@ -858,7 +858,11 @@ __global__ void __launch_bounds__(kBoxThreads, kBoxBlocks) cloudStampBoxKernel(c
             by += by0;
             bz += bz0;
             unsigned long long* word = bricks.at(bx, by, bz);
-            const unsigned long long empty = e.box.in(bx, by, bz) & ~__ldcg(word);  // the warp's, by one address
+            // One lane's look for all: the ballots below are the whole warp's, and
+            // lanes that read the word apart, other warps marking it meanwhile,
+            // could part here.
+            unsigned long long empty = lane == 0 ? e.box.in(bx, by, bz) & ~__ldcg(word) : 0ull;
+            empty = __shfl_sync(0xffffffffu, empty, 0);
             if (empty == 0) continue;
             unsigned long long mark = 0;
 #pragma unroll
