@@ -8,6 +8,18 @@
 
 namespace vsim {
 
+// The buckets that more than 32 records reached in a substep, by hash of the
+// bucket (step_kernels.cu joinCrowd); all idle between substeps.
+struct Crowds {
+    uint32_t* bucket = nullptr;    // per place: the bucket whose crowd it holds
+    uint32_t* lowest = nullptr;    //   ... the 32 lowest of its records past the first 32, ascending
+    uint32_t* ordered = nullptr;   //   ... the 32 lowest of all of them, once a warp has put them in order
+    uint32_t* used = nullptr;      // the places taken
+    uint32_t* count = nullptr;     //   ... how many by bin
+    uint32_t* gathered = nullptr;  //   ... how many for the closing pass to empty
+    uint32_t mask = 0;             // places - 1
+};
+
 // Device buffers of one simulator, as the kernels see them.
 struct DeviceState {
     float4* pos = nullptr;        // xyz position, w = inverse mass the solver uses
@@ -40,7 +52,8 @@ struct DeviceState {
     // the two-launch chain (launchContactSlots; null where it is not used)
     uint4* slots = nullptr;       // per bucket: its first kSlots arrivals
     uint32_t* over = nullptr;     // per bucket: the last arrival past those
-    uint32_t* next = nullptr;     // per record past its bucket's slots: the one that arrived before it
+    uint32_t* next = nullptr;     // per record past its bucket's slots, up to the 32nd: the one that arrived before it
+    Crowds crowds;                // the records past that
     float4* recPos = nullptr;     // per record: its node's position and weight
     // drive
     uint32_t* driven = nullptr;

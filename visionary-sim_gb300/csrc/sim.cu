@@ -559,7 +559,7 @@ void freeSim(vsim_sim* s) {
     DeviceState& d = s->d;
     void* ptrs[] = {d.pos, d.prev, d.vel, d.baseW, d.active, d.activeBody, d.cells, d.bodies, d.fp,
                     d.surf, d.key, d.rank, d.entries, d.count, d.start, d.cursor, d.delta, d.driven,
-                    d.drivenOffset, d.drivenOf, d.rows, d.slots, d.over, d.next, d.recPos, d.nodeRecord, d.sMeta, d.sPos, d.sMoved, d.sRec, d.sKey, d.bodyActive, d.grabs,
+                    d.drivenOffset, d.drivenOf, d.rows, d.slots, d.over, d.next, d.recPos, d.crowds.lowest, d.nodeRecord, d.sMeta, d.sPos, d.sMoved, d.sRec, d.sKey, d.bodyActive, d.grabs,
                     s->chunkDev, s->staging, s->pairs, s->pairCount, s->sp.embed, s->sp.quat,
                     s->sp.scaleBody, s->sp.bodies, s->sp.means, s->sp.cov, s->sp.keys, s->sp.order,
                     s->sp.sortTemp, s->sp.axesRotation, s->sp.axesScale};
@@ -597,6 +597,25 @@ Grid bodyGrid(const Lattice& L, const vsim_tank& tank) {
     }
     const double zero[3] = {0, 0, 0};
     return contactGrid(box, L.h * kContactRadiusCells, zero, zero);
+}
+
+// Whether a bucket of the shared grid holds at most two surface records at rest,
+// by the mean over the records: of the nodes that fill a bucket of the largest
+// cell's edge, the share that is surface. The two-launch contact orders a
+// bucket's records for every record beside it, the five-launch chain once: in
+// scenes of a 90x30x90 body under one of coarser cells its frames' contact took,
+// two launches against five, 255 and 404 us at twice the cell's edge (0.97 by
+// this measure), 600 and 465 at three times (3.0), 3.5 and 3.2 ms at twice with
+// 35 % of the cells out (7.8), 10.7 and 8.9 at four times (62).
+bool sparseAtRest(const vsim_sim* s) {
+    constexpr double kMost = 2.0;
+    double sum = 0;
+    for (size_t b = 0; b < s->lat.size(); b++) {
+        const double nodes = s->nodeBodyStart[b + 1] - s->nodeBodyStart[b];
+        const double records = s->recordBodyStart[b + 1] - s->recordBodyStart[b];
+        if (records > 0) sum += records * (records / nodes) * std::pow(s->grids[0].bucket / s->lat[b].h, 3.0);
+    }
+    return sum <= kMost * s->surfaceCount;
 }
 
 int createSim(const vsim_body_desc* bodies, uint32_t n, const vsim_tank* tank, void* stream, bool isolated,
@@ -738,11 +757,24 @@ int createSim(const vsim_body_desc* bodies, uint32_t n, const vsim_tank* tank, v
     CK(allocN(&d.nodeRecord, N), "allocate node records");
     CK(allocN(&d.count, s->bucketTotal), "allocate contact grid");
     CK(allocN(&d.start, s->bucketTotal), "allocate contact grid");
-    if (!s->isolated && s->bucketTotal <= kSlotBuckets) {
+    if (!s->isolated && s->bucketTotal <= kSlotBuckets && sparseAtRest(s)) {
         CK(allocN(&d.slots, s->bucketTotal), "allocate contact slots");
         CK(allocN(&d.over, s->bucketTotal), "allocate contact slots");
         CK(allocN(&d.next, s->surfaceCount), "allocate contact slots");
         CK(allocN(&d.recPos, s->surfaceCount), "allocate contact slots");
+        // twice as many places as there can be crowds
+        uint32_t places = 2;
+        while (places < 2 * (s->surfaceCount / (kBucketSlots + 1) + 1)) places *= 2;
+        const size_t words = size_t(places) * (2 * kBucketSlots + 2) + 2;
+        CK(allocN(&d.crowds.lowest, words), "allocate contact slots");
+        d.crowds.ordered = d.crowds.lowest + size_t(places) * kBucketSlots;
+        d.crowds.bucket = d.crowds.ordered + size_t(places) * kBucketSlots;
+        d.crowds.used = d.crowds.bucket + places;
+        d.crowds.count = d.crowds.used + places;
+        d.crowds.gathered = d.crowds.count + 1;
+        d.crowds.mask = places - 1;
+        CK(cudaMemsetAsync(d.crowds.lowest, 0xff, (words - 2) * 4, s->stream), "allocate contact slots");
+        CK(cudaMemsetAsync(d.crowds.count, 0, 8, s->stream), "allocate contact slots");
     }
     CK(allocN(&d.bodyActive, s->activeHost.size()), "allocate body activity");
     CK(allocN(&d.grabs, s->grabsHost.size()), "allocate drive targets");

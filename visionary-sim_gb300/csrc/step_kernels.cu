@@ -269,7 +269,7 @@ __global__ void finalizeKernel(const FrameParams* __restrict__ fp, Work work, co
                                const int32_t* __restrict__ nodeRecord, const float4* __restrict__ delta,
                                const uint32_t* __restrict__ key, uint32_t* __restrict__ count,
                                uint32_t* __restrict__ cursor, const uint32_t* __restrict__ bodyActive,
-                               DriveTables drive) {
+                               DriveTables drive, const __grid_constant__ Crowds crowds) {
     struct Pre {
         uint32_t n, live;
         int32_t record, driven;
@@ -291,7 +291,19 @@ __global__ void finalizeKernel(const FrameParams* __restrict__ fp, Work work, co
                                        });
     });
     // After the wait (inside the loop above): the gather has read it.
-    if (CONTACT && blockIdx.x == 0 && threadIdx.x == 0) *cursor = 0;
+    const uint32_t thread = blockIdx.x * blockDim.x + threadIdx.x;
+    if (CONTACT && thread == 0) *cursor = 0;
+    if (CONTACT && crowds.bucket) {
+        constexpr uint32_t kParts = kBucketSlots / 4;
+        const uint32_t parts = *crowds.gathered * kParts;
+        for (uint32_t i = thread; i < parts; i += gridDim.x * blockDim.x) {
+            const uint32_t at = crowds.used[i / kParts];
+            const uint4 idle = make_uint4(kIdle, kIdle, kIdle, kIdle);
+            reinterpret_cast<uint4*>(crowds.lowest)[size_t(at) * kParts + i % kParts] = idle;
+            reinterpret_cast<uint4*>(crowds.ordered)[size_t(at) * kParts + i % kParts] = idle;
+            if (i % kParts == 0) crowds.bucket[at] = kIdle;
+        }
+    }
 }
 
 // ------------------------------------------------------------- contact --
@@ -483,14 +495,51 @@ __global__ void __launch_bounds__(kCollideBlock, 5) collideKernel(
 // Nothing is reset but the counts (by the closing pass): slots past a
 // bucket's count and the list past its overflow are never read.
 //
+// A bucket that more than 32 records reach (bodies dragged past the tank's
+// faces share its outermost buckets, a scene that has gone NaN its first one)
+// is a crowd: later arrivals leave the list alone and put themselves among the
+// crowd's 32 lowest, found in a hash table by their bucket. Each of its words
+// takes the lower of itself and what comes and passes the other on to the next
+// (atomicMin), which leaves the lowest in ascending order whatever the order of
+// arrival; a record above the last of them, as nearly all of thousands are,
+// looks once and leaves. So a crowd of n costs about n looks, and the gather
+// reads at most 64 of it. The closing pass empties the crowds of the substep.
+//
 // The bodies share one grid of at most kSlotBuckets buckets, so a record's
 // bucket and which faces of the grid it lies on fit one word.
+
+// Where bucket b's crowd is looked for first.
+__device__ __forceinline__ uint32_t crowdAt(uint32_t b, const Crowds& crowds) {
+    return (b * 0x9e3779b1u >> 7) & crowds.mask;
+}
+
+// Record r among the 32 lowest of bucket b's crowd. The table has more places
+// than there can be crowds, so the search ends.
+__device__ __noinline__ void joinCrowd(uint32_t r, uint32_t b, const Crowds& crowds) {
+    uint32_t at = crowdAt(b, crowds);
+    for (uint32_t probe = 0; probe <= crowds.mask; probe++, at = (at + 1) & crowds.mask) {
+        uint32_t holder = __ldcg(crowds.bucket + at);
+        if (holder == kIdle) {
+            holder = atomicCAS(crowds.bucket + at, kIdle, b);
+            if (holder == kIdle) {
+                crowds.used[atomicAdd(crowds.count, 1u)] = at;
+                holder = b;
+            }
+        }
+        if (holder == b) break;
+    }
+    uint32_t* lowest = crowds.lowest + size_t(at) * kBucketSlots;
+    // The words only fall: one below the record now stays below it.
+    if (__ldcg(lowest + kBucketSlots - 1) < r) return;
+    for (uint32_t i = 0; i < kBucketSlots && r != kIdle; i++)
+        if (__ldcg(lowest + i) > r) r = max(atomicMin(lowest + i, r), r);
+}
 
 __global__ void binSlotsKernel(Work work, const uint4* __restrict__ surf, const DevBody* __restrict__ bodies,
                                const uint32_t* __restrict__ bodyActive, const float4* __restrict__ pos,
                                uint32_t* __restrict__ key, uint32_t* __restrict__ place, uint32_t* __restrict__ count,
                                uint32_t* __restrict__ slots, uint32_t* __restrict__ over, uint32_t* __restrict__ next,
-                               float4* __restrict__ recPos) {
+                               float4* __restrict__ recPos, const __grid_constant__ Crowds crowds) {
     struct Pre {
         uint4 rec;
         uint32_t live;
@@ -519,8 +568,10 @@ __global__ void binSlotsKernel(Work work, const uint4* __restrict__ surf, const 
         recPos[r] = P;
         if (rank < kSlots)
             slots[kSlots * size_t(b) + rank] = r;
-        else
+        else if (rank < kBucketSlots)
             next[r] = atomicExch(&over[b], r);
+        else
+            joinCrowd(r, b, crowds);
     });
 }
 
@@ -528,21 +579,193 @@ constexpr uint32_t kSlotsBlock = 128;   // threads of a gather block
 constexpr uint32_t kGatherLanes = 9;    // lanes a record: one per row of three buckets along x
 constexpr uint32_t kGatherRecords = 3;  // records a warp
 constexpr uint32_t kGatherList = 96;    // candidates of a record its lanes go through together
+static_assert(kGatherRecords * kGatherList == 9 * kBucketSlots, "a warp's lists hold what nine buckets show");
 
-// The smallest record of bucket b above `last` (kIdle: none), for the records
-// with more candidates than the list holds.
-__device__ uint32_t nextInBucket(uint32_t b, uint32_t n, uint32_t last, bool any, const uint4* slots,
-                                 const uint32_t* over, const uint32_t* next) {
-    uint32_t best = kIdle;
-    uint32_t e = 0;
-    for (uint32_t i = 0; i < n; i++) {
-        if (i < kSlots)
-            e = reinterpret_cast<const uint32_t*>(slots + b)[i];
-        else
-            e = i == kSlots ? over[b] : next[e];
-        if ((any || e > last) && e < best) best = e;
+// collide.wgsl:16-125 for record r by a whole warp (every lane calls it with the
+// same r): a record with more candidates than its own list holds, or next to a
+// crowd. Lane q < 27 lays the early records of neighbour bucket q into `list`
+// (the warp's three lists together; `owner` names the bucket of each), and the
+// warp merges each crowd's lowest with them, unless another has left them in
+// order. The lanes look at the candidates as they come, 32 at a time; only those
+// in reach are then put in order, each ranked against its bucket's others, and
+// corrected for. Where the 27 buckets show more than the list holds they are
+// gone through nine by nine. Returns the corrections' sum and the number of
+// hits, added in candidate order.
+//
+// Instructions and the walk along a bucket's list bound it (3,100 a record when
+// every candidate was put in order, 2,000 here, as the longer chain's warp takes
+// on buckets ordered before). Contact of a frame of ten substeps, microseconds,
+// longer chain by a warp a record and here: 64^3 blob (51k records) squeezed to
+// 0.45, 0.3 and 0.12: 708, 1273, 3350 and 751, 1525, 4821; past a tank's corner
+// 3877 and 2912 (24k records 2238 and 2252), gone NaN 7722 and 3803.
+__device__ __forceinline__ float4 collideFull(uint32_t r, uint32_t selfContact, uint32_t rowStride, uint32_t planeStride,
+                                              const uint4* surf, const DevBody* bodies, const uint32_t* place,
+                                              const uint32_t* count, const uint4* slots, const uint32_t* over,
+                                              const uint32_t* next, const float4* recPos, const float4* prevState,
+                                              const Crowds& crowds, uint32_t* list, uint8_t* owner) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t home = place[r], faces = home / kSlotBuckets;
+    const uint32_t dx = lane % 3, dy = lane / 3 % 3, dz = lane / 9;  // offsets + 1
+    const uint32_t outside = (dx == 0 ? 1u : dx == 2 ? 2u : 0u) | (dy == 0 ? 4u : dy == 2 ? 8u : 0u) |
+                             (dz == 0 ? 16u : dz == 2 ? 32u : 0u);
+    const uint32_t b = (home & (kSlotBuckets - 1)) + (dx - 1) + (dy - 1) * rowStride + (dz - 1) * planeStride;
+    const uint32_t n = lane < 27 && !(faces & outside) ? count[b] : 0;
+    const uint32_t held = min(n, kBucketSlots);
+    uint32_t end = held;
+#pragma unroll
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(kAll, end, d);
+        if (lane >= d) end += v;
     }
-    return best;
+    const uint32_t total = __shfl_sync(kAll, end, 31);
+    const uint32_t each = total <= 9 * kBucketSlots ? 27 : 9;  // buckets at a time
+    uint32_t crowd = 0;                                        // the bucket's, where it has one
+    if (n > kBucketSlots) {
+        crowd = crowdAt(b, crowds);
+        for (uint32_t probe = 0; probe < crowds.mask && crowds.bucket[crowd] != b; probe++)
+            crowd = (crowd + 1) & crowds.mask;
+    }
+    Contactor c;
+    c.me = surf[r];
+    c.node = c.me.x;
+    c.radius = __uint_as_float(c.me.w);
+    const float4 P = recPos[r];
+    c.pi = xyz(P);
+    c.wi = P.w;
+    V sum = mk(0.0f, 0.0f, 0.0f);
+    float hits = 0.0f;
+#pragma unroll 1
+    for (uint32_t first = 0; first < 27; first += each) {
+        const uint32_t before = first ? __shfl_sync(kAll, end, first - 1) : 0u;
+        const uint32_t candidates = __shfl_sync(kAll, end, first + each - 1) - before;
+        const bool mine = lane >= first && lane < first + each && held > 0;
+        const uint32_t at = end - held - before;  // of the lane's bucket in the list
+        __syncwarp();                             // the list's readers are done with it
+        // The crowds that some warp has ordered before (a word of theirs is idle
+        // or final, so a whole row speaks for itself).
+        uint32_t unordered = 0;
+        uint32_t some = __ballot_sync(kAll, mine && n > kBucketSlots);
+        const uint32_t* ordered = crowds.ordered + lane;
+        uint32_t ahead = kIdle;
+        if (some) ahead = __ldcg(ordered + size_t(__shfl_sync(kAll, crowd, __ffs(some) - 1)) * kBucketSlots);
+        while (some) {
+            const uint32_t q = __ffs(some) - 1, row = ahead;
+            some &= some - 1;
+            if (some) ahead = __ldcg(ordered + size_t(__shfl_sync(kAll, crowd, __ffs(some) - 1)) * kBucketSlots);
+            const uint32_t base = __shfl_sync(kAll, at, q);
+            if (__any_sync(kAll, row == kIdle)) {
+                unordered |= 1u << q;
+            } else {
+                list[base + lane] = row;
+                owner[base + lane] = uint8_t(q);
+            }
+        }
+        if (mine && (n <= kBucketSlots || (unordered >> lane & 1))) {
+            const uint4 s = slots[b];
+            list[at] = s.x;
+            if (held > 1) list[at + 1] = s.y;
+            if (held > 2) list[at + 2] = s.z;
+            if (held > 3) list[at + 3] = s.w;
+            uint32_t e = held > kSlots ? over[b] : 0;
+            for (uint32_t i = kSlots; i < held; i++) {
+                list[at + i] = e;
+                if (i + 1 < held) e = next[e];
+            }
+            for (uint32_t i = 0; i < held; i++) owner[at + i] = uint8_t(lane);
+        }
+        __syncwarp();
+        // The others: the lowest of their early records, put in order, and of the
+        // rest, which ascend. The lower of the one from below and the other from
+        // above are the lowest of both, falling and rising once: five exchanges
+        // order them.
+        for (; unordered; unordered &= unordered - 1) {
+            const uint32_t q = __ffs(unordered) - 1, base = __shfl_sync(kAll, at, q);
+            const size_t row = size_t(__shfl_sync(kAll, crowd, q)) * kBucketSlots + lane;
+            uint32_t e = list[base + lane];
+            const uint32_t late = crowds.lowest[row];
+            auto exchange = [&](uint32_t distance, bool up) {
+                const uint32_t other = __shfl_xor_sync(kAll, e, distance);
+                e = up == ((lane & distance) == 0) ? min(e, other) : max(e, other);
+            };
+#pragma unroll
+            for (uint32_t size = 2; size <= 32; size *= 2)
+#pragma unroll
+                for (uint32_t distance = size / 2; distance > 0; distance /= 2)
+                    exchange(distance, (lane & size) == 0 || size == 32);
+            e = min(late, __shfl_sync(kAll, e, 31 - lane));
+#pragma unroll
+            for (uint32_t distance = 16; distance > 0; distance /= 2) exchange(distance, true);
+            list[base + lane] = e;
+            __stcg(crowds.ordered + row, e);
+        }
+        __syncwarp();
+        // The records in reach, moved to the list's front as they are found.
+        uint32_t found = 0;
+        for (uint32_t from = 0; from < candidates; from += 32) {
+            bool hit = false;
+            uint32_t e = 0, of = 0;
+            if (from + lane < candidates) {
+                e = list[from + lane];
+                of = owner[from + lane];
+                float dist2;
+                hit = contactHit(c, surf[e], recPos[e], selfContact, dist2);
+            }
+            const uint32_t bits = __ballot_sync(kAll, hit);
+            if (hit) {
+                const uint32_t to = found + __popc(bits & ((1u << lane) - 1u));
+                list[to] = e;
+                owner[to] = uint8_t(of);
+            }
+            found += __popc(bits);
+        }
+        __syncwarp();
+        // As many whole buckets' at a time as 32 lanes hold, one a lane.
+        for (uint32_t from = 0; from < found;) {
+            uint32_t here = min(32u, found - from);
+            uint32_t e = lane < here ? list[from + lane] : 0;
+            const uint32_t of = lane < here ? owner[from + lane] : 0xffu;
+            const uint32_t left = __shfl_up_sync(kAll, of, 1);
+            // bit l: a bucket's start at lane l
+            uint32_t starts = __ballot_sync(kAll, lane < here && (lane == 0 || of != left));
+            if (from + here < found && owner[from + here] == __shfl_sync(kAll, of, 31)) {
+                here = 31 - __clz(starts);  // the last goes on
+                starts &= (1u << here) - 1u;
+            }
+            const uint32_t upTo = starts & (0xffffffffu >> (31 - lane)), above = starts & ~(0xffffffffu >> (31 - lane));
+            const uint32_t run = 31 - __clz(upTo | 1u);  // where the lane's bucket starts, and how many it has
+            const uint32_t holds = lane < here ? (above ? __ffs(above) - 1 : here) - run : 0;
+            const uint32_t most = __reduce_max_sync(kAll, holds);
+            if (most > 1) {
+                uint32_t rank = 0;
+                for (uint32_t j = 0; j < most; j++) {
+                    const uint32_t other = __shfl_sync(kAll, e, run + j);
+                    rank += j < holds && other < e ? 1u : 0u;
+                }
+                if (lane < here) list[from + run + rank] = e;
+                __syncwarp();
+                if (lane < here) e = list[from + lane];
+            }
+            V correction = mk(0.0f, 0.0f, 0.0f);
+            if (lane < here) {
+                const uint4 them = surf[e];
+                const float4 Q = recPos[e];
+                const V d = c.pi - xyz(Q);
+                c.movedI = c.pi - xyz(prevState[c.node]);
+                c.frictionI = bodies[c.me.y].friction;
+                const V moved = xyz(Q) - xyz(prevState[them.x]);
+                correction = contactCorrection(c, them, Q, withW(moved, bodies[them.y].friction), dot(d, d));
+            }
+            for (uint32_t at = 0; at < here; at++) {
+                const V add = mk(__shfl_sync(kAll, correction.x, at), __shfl_sync(kAll, correction.y, at),
+                                 __shfl_sync(kAll, correction.z, at));
+                sum = sum + add;
+                hits = hits + 1.0f;
+            }
+            from += here;
+        }
+    }
+    return withW(sum, hits);
 }
 
 // collide.wgsl:16-125 for every live record. Nine lanes share a record, three
@@ -557,17 +780,18 @@ __device__ uint32_t nextInBucket(uint32_t b, uint32_t n, uint32_t last, bool any
 // and 64 registers, eight blocks an SM, measured best (the 64^3 blob's frame
 // 465 us; with ten blocks, which spill, 484).
 //
-// A record with more than kGatherList candidates, or next to a bucket of
-// more than 32, is gone through by its first lane alone.
+// A record with more than kGatherList candidates, or next to a crowd, is gone
+// through by its whole warp after that (collideFull).
 __global__ void __launch_bounds__(kSlotsBlock, 8) collideSlotsKernel(
     const FrameParams* __restrict__ fp, uint32_t records, uint32_t rowStride, uint32_t planeStride,
     const uint4* __restrict__ surf, const DevBody* __restrict__ bodies, const uint32_t* __restrict__ place,
     const uint32_t* __restrict__ count, const uint4* __restrict__ slots, const uint32_t* __restrict__ over,
     const uint32_t* __restrict__ next, const float4* __restrict__ recPos, const float4* __restrict__ prevState,
-    float4* __restrict__ delta) {
+    const __grid_constant__ Crowds crowds, float4* __restrict__ delta) {
     constexpr unsigned kAll = 0xffffffffu;
     constexpr uint32_t kGroup = (1u << kGatherLanes) - 1u;
     __shared__ uint32_t lists[kSlotsBlock / 32][kGatherRecords][kGatherList];
+    __shared__ uint8_t owners[kSlotsBlock / 32][kGatherRecords * kGatherList];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t group = lane / kGatherLanes, q = lane - group * kGatherLanes;
     const uint32_t r = (blockIdx.x * (kSlotsBlock / 32) + warp) * kGatherRecords + group;
@@ -696,26 +920,17 @@ __global__ void __launch_bounds__(kSlotsBlock, 8) collideSlotsKernel(
             }
         }
     }
-    if (live && !listed && q == 0) {
-        for (uint32_t row = 0; row < kGatherLanes; row++) {
-            if (!rowOf(row, middle)) continue;
-            for (uint32_t d = 0; d < 3; d++) {
-                if (!inRow(d)) continue;
-                const uint32_t b = middle + d - 1, n = count[b];
-                uint32_t last = 0;
-                for (uint32_t i = 0; i < min(n, kBucketSlots); i++) {
-                    last = nextInBucket(b, n, last, i == 0, slots, over, next);
-                    const uint4 them = surf[last];
-                    const float4 Q = recPos[last];
-                    float dist2;
-                    if (!contactHit(c, them, Q, selfContact, dist2)) continue;
-                    sum = sum + correct(them, Q, dist2);
-                    hits = hits + 1.0f;
-                }
-            }
-        }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *crowds.gathered = *crowds.count;
+        *crowds.count = 0;
     }
-    if (live && q == 0) delta[r] = withW(sum, hits);
+    if (listed && q == 0) delta[r] = withW(sum, hits);
+    for (uint32_t full = __ballot_sync(kAll, live && !listed && q == 0); full; full &= full - 1) {
+        const uint32_t at = __shfl_sync(kAll, r, __ffs(full) - 1);
+        const float4 d = collideFull(at, selfContact, rowStride, planeStride, surf, bodies, place, count, slots, over,
+                                     next, recPos, prevState, crowds, reinterpret_cast<uint32_t*>(&lists[warp]), owners[warp]);
+        if (lane == 0) delta[at] = d;
+    }
     pdlLaunchNext();
 }
 
@@ -918,7 +1133,7 @@ cudaError_t launchFinalize(const LaunchCtx& c, const DeviceState& s, const Span&
     auto go = [&](auto kernel) {
         return launch(c, kernel, n.grid, n.block, s.fp, n.work, s.active, s.activeBody, s.bodies, s.pos, s.prev,
                       s.vel, (const int32_t*)s.nodeRecord, (const float4*)s.delta, (const uint32_t*)s.key, s.count,
-                      s.cursor, (const uint32_t*)s.bodyActive, driveTables(s));
+                      s.cursor, (const uint32_t*)s.bodyActive, driveTables(s), s.crowds);
     };
     if (predictNext && drive)
         return contact ? go(finalizeKernel<true, true, true>) : go(finalizeKernel<false, true, true>);
@@ -990,12 +1205,12 @@ cudaError_t launchContactSlots(const LaunchCtx& c, const DeviceState& s, const S
     cudaError_t e;
     if ((e = launch(c, binSlotsKernel, r.grid, r.block, r.work, s.surf, (const DevBody*)s.bodies,
                     (const uint32_t*)s.bodyActive, (const float4*)s.pos, s.key, s.rank, s.count,
-                    reinterpret_cast<uint32_t*>(s.slots), s.over, s.next, s.recPos)))
+                    reinterpret_cast<uint32_t*>(s.slots), s.over, s.next, s.recPos, s.crowds)))
         return e;
     return launch(c, collideSlotsKernel, blocks(r.work.count, kGatherRecords * (kSlotsBlock / 32)), kSlotsBlock, s.fp,
                   r.work.count, rowStride, planeStride, s.surf, (const DevBody*)s.bodies, (const uint32_t*)s.rank,
                   (const uint32_t*)s.count, (const uint4*)s.slots, (const uint32_t*)s.over, (const uint32_t*)s.next,
-                  (const float4*)s.recPos, (const float4*)s.prev, s.delta);
+                  (const float4*)s.recPos, (const float4*)s.prev, s.crowds, s.delta);
 }
 
 cudaError_t launchCensus(const LaunchCtx& c, const DeviceState& s, const Span& r, unsigned long long* out) {
