@@ -879,30 +879,130 @@ __global__ void __launch_bounds__(kBoxThreads, kBoxBlocks) cloudStampBoxKernel(c
     }
 }
 
-// The stamp of a grid with fewer than three cells on an axis, where "within
-// one cell of the faces" leaves the grid: the index is the reference's
-// cellIndex of the (possibly out-of-grid) coordinates, and like a typed array
-// the grid ignores an index outside it. A block a Gaussian.
-__global__ void cloudStampLooseKernel(CloudInput in, GridView g, const float4* __restrict__ reach, Bricks bricks) {
-    for (uint32_t i = blockIdx.x; i < in.count; i += gridDim.x) {
-        if (threadIdx.x == 0) {
-            uint32_t centre[3];
-            for (int a = 0; a < 3; a++) centre[a] = exactCentre(g, in.pos[3 * size_t(i) + a], a);
-            markCell(bricks, centre);
+// The stamp of a grid with fewer than three cells on an axis (a flat cloud, no
+// padding), where "within one cell of the faces" leaves the grid: the index is
+// the reference's cellIndex of the (possibly out-of-grid) coordinates, and like a
+// typed array the grid ignores an index outside it.
+
+// The cell that (x, y, z) index, false where none.
+__device__ __forceinline__ bool looseCell(const GridView& g, int64_t x, int64_t y, int64_t z, uint32_t at[3]) {
+    const int64_t cell = x + int64_t(g.dims[0]) * (y + int64_t(g.dims[1]) * z);
+    if (cell < 0 || cell >= int64_t(g.cells)) return false;
+    const uint32_t row = uint32_t(cell) / g.dims[0];
+    at[2] = row / g.dims[1];
+    at[1] = row - at[2] * g.dims[1];
+    at[0] = uint32_t(cell) - row * g.dims[0];
+    return true;
+}
+
+__device__ __forceinline__ bool isMarked(const Bricks& bricks, const uint32_t at[3]) {
+    const uint32_t bit = (at[0] & 3) + 4 * (at[1] & 3) + 16 * (at[2] & 3);
+    return __ldcg(bricks.at(at[0] >> 2, at[1] >> 2, at[2] >> 2)) >> bit & 1;
+}
+
+struct LooseEntry {
+    FloatTest f;
+    float quick;
+    int64_t lo[3];
+    uint32_t ex, ey, gaussian, fast;
+};
+
+// A thread a Gaussian: its centre, its box, and whether the box has a cell that
+// is still empty; larger boxes are listed for the kernel below. Each warp then
+// deals the cells of those that do to its lanes, 32 at a time, as
+// cloudStampKernel does (2M Gaussians on 501 x 1 x 501 cells, a whole
+// voxelisation: 75 ms with a block a Gaussian, 0.46 so).
+constexpr int64_t kLooseCells = 64;  // of a box that a warp's lanes share
+__global__ void __launch_bounds__(kStampBlock) cloudStampLooseKernel(const __grid_constant__ CloudInput in,
+                                                                     const __grid_constant__ GridView g,
+                                                                     const float4* __restrict__ reach, Bricks bricks,
+                                                                     uint32_t* __restrict__ big,
+                                                                     unsigned long long* __restrict__ bigCount) {
+    constexpr unsigned kAll = 0xffffffffu;
+    __shared__ LooseEntry entries[kStampBlock];
+    const uint32_t t = threadIdx.x, lane = t & 31, warpBase = t & ~31u;
+    const uint64_t i = uint64_t(blockIdx.x) * kStampBlock + t;
+    uint32_t n = 0;
+    if (i < in.count) {
+        uint32_t at[3];
+        for (int a = 0; a < 3; a++) {
+            const float c = in.pos[3 * size_t(i) + a];
+            if (!floatCentre(g, c, a, at[a])) at[a] = exactCentre(g, c, a);
         }
-        const Box b = boxOf(in, i, g, reach);
-        FloatTest f;
-        const bool fast = testOf(in, i, g, b, f);
+        markCell(bricks, at);
+        const Box b = boxOf(in, uint32_t(i), g, reach);
         const int64_t ex = b.extent(0), ey = b.extent(1), ez = b.extent(2);
-        if (ex <= 0 || ey <= 0 || ez <= 0) continue;
-        for (int64_t t = threadIdx.x; t < ex * ey * ez; t += blockDim.x) {
+        if (ex > kLooseCells || ey > kLooseCells || ez > kLooseCells || ex * ey * ez > kLooseCells) {
+            big[atomicAdd(bigCount, 1ull)] = uint32_t(i);
+        } else {
+            bool empty = false;
+            for (int64_t z = b.lo[2]; z <= b.hi[2]; z++)
+                for (int64_t y = b.lo[1]; y <= b.hi[1]; y++)
+                    for (int64_t x = b.lo[0]; x <= b.hi[0]; x++)
+                        if (looseCell(g, x, y, z, at) && !isMarked(bricks, at)) empty = true;
+            if (empty) {
+                LooseEntry& e = entries[t];
+                e.fast = testOf(in, uint32_t(i), g, b, e.f) ? 1u : 0u;
+                e.quick = bounds::quickBound(e.f);
+                for (int a = 0; a < 3; a++) e.lo[a] = b.lo[a];
+                e.ex = uint32_t(ex);
+                e.ey = uint32_t(ey);
+                e.gaussian = uint32_t(i);
+                n = uint32_t(ex * ey * ez);
+            }
+        }
+    }
+    uint32_t incl = n;  // the warp's running offsets: lane l's cells are [off, off + n)
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(kAll, incl, d);
+        if (lane >= uint32_t(d)) incl += v;
+    }
+    const uint32_t off = incl - n, total = __shfl_sync(kAll, incl, 31);
+    __syncwarp();
+    for (uint32_t base = 0; base < total; base += 32) {
+        const uint32_t c = base + lane;
+        uint32_t owner = 0;  // the last lane whose offset is at or below c
+#pragma unroll
+        for (uint32_t step = 16; step >= 1; step >>= 1) {
+            const uint32_t probe = __shfl_sync(kAll, off, owner + step);
+            if (probe <= c) owner += step;
+        }
+        const uint32_t first = __shfl_sync(kAll, off, owner);
+        if (c >= total) continue;
+        const LooseEntry& e = entries[warpBase + owner];
+        const uint32_t row = (c - first) / e.ex, plane = row / e.ey;
+        const int64_t x = e.lo[0] + (c - first - row * e.ex), y = e.lo[1] + (row - plane * e.ey), z = e.lo[2] + plane;
+        uint32_t at[3];
+        if (!looseCell(g, x, y, z, at) || isMarked(bricks, at)) continue;
+        if (cellReached(in, e.gaussian, g, e.lo, x, y, z, e.fast ? &e.f : nullptr, e.quick)) markCell(bricks, at);
+    }
+}
+
+// The larger boxes, a block each.
+__global__ void __launch_bounds__(kCloudBlock) cloudStampLooseBoxKernel(const __grid_constant__ CloudInput in,
+                                                                        const __grid_constant__ GridView g,
+                                                                        const float4* __restrict__ reach, Bricks bricks,
+                                                                        const uint32_t* __restrict__ big,
+                                                                        const unsigned long long* __restrict__ bigCount) {
+    __shared__ LooseEntry e;
+    __shared__ Box b;
+    const uint64_t listed = *bigCount;
+    for (uint64_t n = blockIdx.x; n < listed; n += gridDim.x) {
+        __syncthreads();  // the box before is done
+        if (threadIdx.x == 0) {
+            e.gaussian = big[n];
+            b = boxOf(in, e.gaussian, g, reach);
+            e.fast = testOf(in, e.gaussian, g, b, e.f) ? 1u : 0u;
+            e.quick = bounds::quickBound(e.f);
+        }
+        __syncthreads();
+        const int64_t ex = b.extent(0), ey = b.extent(1), cells = b.cells();
+        for (int64_t t = threadIdx.x; t < cells; t += kCloudBlock) {
             const int64_t x = b.lo[0] + t % ex, y = b.lo[1] + t / ex % ey, z = b.lo[2] + t / (ex * ey);
-            const int64_t cell = x + int64_t(g.dims[0]) * (y + int64_t(g.dims[1]) * z);
-            if (cell < 0 || cell >= int64_t(g.cells)) continue;
-            const int64_t row = cell / g.dims[0];
-            const uint32_t cx = uint32_t(cell % g.dims[0]), cy = uint32_t(row % g.dims[1]), cz = uint32_t(row / g.dims[1]);
-            if (*bricks.at(cx >> 2, cy >> 2, cz >> 2) >> ((cx & 3) + 4 * (cy & 3) + 16 * (cz & 3)) & 1) continue;
-            if (cellReached(in, i, g, b.lo, x, y, z, fast ? &f : nullptr, bounds::quickBound(f))) bricks.set(cx, cy, cz);
+            uint32_t at[3];
+            if (!looseCell(g, x, y, z, at) || isMarked(bricks, at)) continue;
+            if (cellReached(in, e.gaussian, g, b.lo, x, y, z, e.fast ? &e.f : nullptr, e.quick)) markCell(bricks, at);
         }
     }
 }
@@ -1458,7 +1558,9 @@ int voxelizeCloud(vsim_cloud_volume* v, const CloudInput& in, const vsim_cloud_o
     const Bricks bricks{static_cast<unsigned long long*>(bricksBuf.p), (d.nx + 3) / 4, (d.ny + 3) / 4};
     CK(cudaMemsetAsync(bricksBuf.p, 0, brickBytes, st), "cloud stamp");
     if (d.nx < 3 || d.ny < 3 || d.nz < 3) {
-        cloudStampLooseKernel<<<std::min(in.count, uint32_t(sms) * 8), kCloudBlock, 0, st>>>(in, g, reach, bricks);
+        cloudStampLooseKernel<<<uint32_t((uint64_t(in.count) + kStampBlock - 1) / kStampBlock), kStampBlock, 0, st>>>(
+            in, g, reach, bricks, big, &sc->bigCount);
+        cloudStampLooseBoxKernel<<<uint32_t(sms) * 4, kCloudBlock, 0, st>>>(in, g, reach, bricks, big, &sc->bigCount);
     } else {
         // As many rounds as make the blocks one wave.
         const uint64_t wave = uint64_t(sms) * kStampBlocks * kStampBlock;
