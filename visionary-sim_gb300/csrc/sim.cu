@@ -207,6 +207,27 @@ int uploadCells(vsim_sim* s, bool again) {
     return VSIM_OK;
 }
 
+// Whether row passes are worth their groups. A group of isolated bodies holds one
+// body's cells, and a block takes about as long for a few as for many: a pool of
+// 10,000 bodies of 2x2x2 cells took 374 us a sweep in rows where its colours take
+// 31, and was twice as long in the making. Rows, where a pass is at most a wave of
+// blocks (400 such bodies 17 us, the colours 27; 500, two waves: 31 and 27), or
+// the groups are three eighths full (rows and colours: 10,000 of 2x2x16, an
+// eighth, 390 and 107; 3,000 of 7x7x7, a third, 158 and 97; 1,000 of 8x8x8, a
+// half, 62, where the colours took 64 before the branch-free arithmetic).
+bool rowsPay(const vsim_sim* s) {
+    if (!s->isolated) return true;
+    uint64_t groups[kRowPasses] = {}, all = 0, most = 0;
+    for (const Lattice& L : s->lat)
+        for (uint32_t q = 0; q < kRowPasses; q++)
+            groups[q] += (std::max(L.cellsByColor[2 * q].size(), L.cellsByColor[2 * q + 1].size()) + kRowBlock - 1) / kRowBlock;
+    for (uint64_t g : groups) {
+        all += g;
+        most = std::max(most, g);
+    }
+    return most <= kRowChunksPerSm * s->sms || uint64_t(s->cellCount) * 8 >= all * kRowGroup * 3;
+}
+
 // The row passes' groups (kRowBlock), pass by pass (y and z parity), bodies in
 // order and rows in lattice order inside each; a group of isolated bodies
 // holds one body's. False when some run of cells
@@ -810,7 +831,7 @@ int createSim(const vsim_body_desc* bodies, uint32_t n, const vsim_tank* tank, v
         if (int rc = uploadCells(s, false)) return rc;
         CK(cudaMemGetInfo(&freeBytes, &allBytes), "memory left");
     }
-    if (buildRows(s, rows) && rows.size() * 16 <= freeBytes / 8) {
+    if (rowsPay(s) && buildRows(s, rows) && rows.size() * 16 <= freeBytes / 8) {
         s->rowPasses = true;
         CK(allocN(&d.rows, rows.size()), "allocate rows");
         CK(cudaMemcpyAsync(d.rows, rows.data(), rows.size() * 16, cudaMemcpyHostToDevice, s->stream), "upload rows");
