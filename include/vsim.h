@@ -294,9 +294,10 @@ int vsim_set_pdl(vsim_sim* sim, int enabled);
 
 /* How the contact gather maps surface records to GPU threads. AUTO (default)
    bins a whole scene's records into bucket slots and gives each record nine
-   lanes; where bodies are isolated it orders the records by bucket and gives
-   each a warp while the substep has fewer than 2048 records per SM and a
-   thread otherwise. WARP and THREAD order them by bucket and force one
+   lanes; where bodies are isolated, the scene has more than 3200 records per SM,
+   or a bucket holds more than two at rest (cells of different size), it orders
+   the records by bucket and gives each a warp while the substep has fewer than
+   2048 records per SM and a thread otherwise. WARP and THREAD order them by bucket and force one
    mapping. All give the same results (each record's hits are summed in the
    reference's order); the setting exists for tests and sweeps. No reference
    counterpart. */

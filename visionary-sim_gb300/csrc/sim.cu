@@ -639,6 +639,14 @@ bool sparseAtRest(const vsim_sim* s) {
     return sum <= kMost * s->surfaceCount;
 }
 
+// The most records the two-launch contact takes, an SM. It spends nine lanes on a
+// record where the five-launch chain, once the GPU is full, spends one thread, and
+// saves that chain's ordering: contact of a frame, two launches against five, of a
+// blob and a sheet at rest and sagged: 422k records 2.17 against 2.18 and 2.19
+// against 2.40 ms, 502k 2.59 against 2.50 and 2.62 against 2.68, 571k 2.92 against
+// 2.62 and 2.98 against 2.91, 820k 4.69 against 3.70 and 4.72 against 4.06.
+constexpr uint32_t kSlotRecordsPerSm = 3200;
+
 int createSim(const vsim_body_desc* bodies, uint32_t n, const vsim_tank* tank, void* stream, bool isolated,
               vsim_sim* s) {
     s->isolated = isolated;
@@ -778,7 +786,8 @@ int createSim(const vsim_body_desc* bodies, uint32_t n, const vsim_tank* tank, v
     CK(allocN(&d.nodeRecord, N), "allocate node records");
     CK(allocN(&d.count, s->bucketTotal), "allocate contact grid");
     CK(allocN(&d.start, s->bucketTotal), "allocate contact grid");
-    if (!s->isolated && s->bucketTotal <= kSlotBuckets && sparseAtRest(s)) {
+    if (!s->isolated && s->bucketTotal <= kSlotBuckets && s->surfaceCount <= kSlotRecordsPerSm * s->sms &&
+        sparseAtRest(s)) {
         CK(allocN(&d.slots, s->bucketTotal), "allocate contact slots");
         CK(allocN(&d.over, s->bucketTotal), "allocate contact slots");
         CK(allocN(&d.next, s->surfaceCount), "allocate contact slots");
