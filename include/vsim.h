@@ -297,7 +297,9 @@ int vsim_set_pdl(vsim_sim* sim, int enabled);
    lanes; where bodies are isolated, the scene has more than 3200 records per SM,
    or a bucket holds more than two at rest (cells of different size), it orders
    the records by bucket and gives each a warp while the substep has fewer than
-   2048 records per SM and a thread otherwise. WARP and THREAD order them by bucket and force one
+   2048 records per SM and a thread otherwise. The slots, 20 bytes a bucket, are
+   made once contact can touch anything; where the device has no room for them
+   the records are ordered. WARP and THREAD order them by bucket and force one
    mapping. All give the same results (each record's hits are summed in the
    reference's order); the setting exists for tests and sweeps. No reference
    counterpart. */

@@ -515,6 +515,7 @@ uint64_t graphKey(const vsim_sim* s, uint32_t steps) {
     k = k * 31 + (s->tma.enabled ? 1 : 0);
     k = k * 31 + (s->quadCells ? 1 : 0);
     k = k * 31 + (inRows(s) ? 1 : 0);
+    k = k * 31 + (inSlots(s) ? 1 : 0);
     k = k * 131 + s->plan.records.gatherPerSm;
     return k;
 }
@@ -646,6 +647,51 @@ bool sparseAtRest(const vsim_sim* s) {
 // against 2.40 ms, 502k 2.59 against 2.50 and 2.62 against 2.68, 571k 2.92 against
 // 2.62 and 2.98 against 2.91, 820k 4.69 against 3.70 and 4.72 against 4.06.
 constexpr uint32_t kSlotRecordsPerSm = 3200;
+
+// The two-launch contact's buffers, once contact can touch anything and the scene
+// is one for it: up to 20 bytes a bucket. Where the device has no room for them
+// the frames take the five-launch chain, which needs none. A caller may be
+// capturing a stream, so the calls are made as ones that may be.
+void makeSlots(vsim_sim* s) {
+    DeviceState& d = s->d;
+    if (d.slots || s->isolated || !contactMatters(s) || s->bucketTotal > kSlotBuckets ||
+        s->surfaceCount > kSlotRecordsPerSm * s->sms || !sparseAtRest(s))
+        return;
+    // twice as many places as there can be crowds
+    uint32_t places = 2;
+    while (places < 2 * (s->surfaceCount / (kBucketSlots + 1) + 1)) places *= 2;
+    const size_t words = size_t(places) * (2 * kBucketSlots + 2) + 2;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    uint4* slots = nullptr;
+    Crowds& c = d.crowds;
+    cudaError_t e = allocN(&slots, s->bucketTotal);
+    if (!e) e = allocN(&d.over, s->bucketTotal);
+    if (!e) e = allocN(&d.next, s->surfaceCount);
+    if (!e) e = allocN(&d.recPos, s->surfaceCount);
+    if (!e) e = allocN(&c.lowest, words);
+    if (!e) e = cudaMemsetAsync(c.lowest, 0xff, (words - 2) * 4, s->capture);
+    if (!e) e = cudaMemsetAsync(c.lowest + words - 2, 0, 8, s->capture);
+    if (!e) e = cudaStreamSynchronize(s->capture);
+    if (!e) {
+        c.ordered = c.lowest + size_t(places) * kBucketSlots;
+        c.bucket = c.ordered + size_t(places) * kBucketSlots;
+        c.used = c.bucket + places;
+        c.count = c.used + places;
+        c.gathered = c.count + 1;
+        c.mask = places - 1;
+        d.slots = slots;
+    } else {
+        for (void* p : {static_cast<void*>(slots), static_cast<void*>(d.over), static_cast<void*>(d.next),
+                        static_cast<void*>(d.recPos), static_cast<void*>(c.lowest)})
+            if (p) cudaFree(p);
+        d.over = d.next = nullptr;
+        d.recPos = nullptr;
+        c = Crowds{};
+        cudaGetLastError();
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+}
 
 int createSim(const vsim_body_desc* bodies, uint32_t n, const vsim_tank* tank, void* stream, bool isolated,
               vsim_sim* s) {
@@ -786,26 +832,6 @@ int createSim(const vsim_body_desc* bodies, uint32_t n, const vsim_tank* tank, v
     CK(allocN(&d.nodeRecord, N), "allocate node records");
     CK(allocN(&d.count, s->bucketTotal), "allocate contact grid");
     CK(allocN(&d.start, s->bucketTotal), "allocate contact grid");
-    if (!s->isolated && s->bucketTotal <= kSlotBuckets && s->surfaceCount <= kSlotRecordsPerSm * s->sms &&
-        sparseAtRest(s)) {
-        CK(allocN(&d.slots, s->bucketTotal), "allocate contact slots");
-        CK(allocN(&d.over, s->bucketTotal), "allocate contact slots");
-        CK(allocN(&d.next, s->surfaceCount), "allocate contact slots");
-        CK(allocN(&d.recPos, s->surfaceCount), "allocate contact slots");
-        // twice as many places as there can be crowds
-        uint32_t places = 2;
-        while (places < 2 * (s->surfaceCount / (kBucketSlots + 1) + 1)) places *= 2;
-        const size_t words = size_t(places) * (2 * kBucketSlots + 2) + 2;
-        CK(allocN(&d.crowds.lowest, words), "allocate contact slots");
-        d.crowds.ordered = d.crowds.lowest + size_t(places) * kBucketSlots;
-        d.crowds.bucket = d.crowds.ordered + size_t(places) * kBucketSlots;
-        d.crowds.used = d.crowds.bucket + places;
-        d.crowds.count = d.crowds.used + places;
-        d.crowds.gathered = d.crowds.count + 1;
-        d.crowds.mask = places - 1;
-        CK(cudaMemsetAsync(d.crowds.lowest, 0xff, (words - 2) * 4, s->stream), "allocate contact slots");
-        CK(cudaMemsetAsync(d.crowds.count, 0, 8, s->stream), "allocate contact slots");
-    }
     CK(allocN(&d.bodyActive, s->activeHost.size()), "allocate body activity");
     CK(allocN(&d.grabs, s->grabsHost.size()), "allocate drive targets");
     CK(allocN(&d.cursor, 1), "allocate contact cursor");
@@ -899,6 +925,7 @@ int createSim(const vsim_body_desc* bodies, uint32_t n, const vsim_tank* tank, v
     s->splatMeans.resize(n);
     s->splatQuats.resize(n);
     s->splatScales.resize(n);
+    makeSlots(s);
     return VSIM_OK;
 }
 
@@ -1223,6 +1250,7 @@ int vsim_set_material(vsim_sim* s, uint32_t body, const vsim_material* m, uint32
 int vsim_set_contact(vsim_sim* s, int enabled) {
     SIM_GUARD(s);
     s->contact = enabled != 0;
+    makeSlots(s);
     return VSIM_OK;
 }
 
@@ -1233,6 +1261,7 @@ int vsim_set_self_contact(vsim_sim* s, int enabled) {
             if (enabled && L.nodeDims[a] > 1024) return fail(VSIM_ERR_RANGE, "self contact needs bodies of at most 1023 cells per axis");
     s->selfContact = enabled != 0;
     s->frameDirty = true;
+    makeSlots(s);
     return VSIM_OK;
 }
 
