@@ -284,7 +284,9 @@ int vsim_set_tma_pass(vsim_sim* sim, int enabled);
    (else VSIM_ERR_RANGE). */
 int vsim_set_cell_lanes(vsim_sim* sim, uint32_t lanes);
 /* Time every {brick 0,4,8} x {block 128,256,512} shape on `frames` frames of
-   the live state (which is saved and restored) and keep the fastest.
+   the live state (which is saved and restored) and keep the fastest. Frames
+   that solve their cells row by row read no shape (vsim_set_launch_shape):
+   theirs stays as it is and nothing is timed.
    Writes the chosen shape to *block and *brick when non-NULL. */
 int vsim_tune(vsim_sim* sim, uint32_t frames, uint32_t* block, uint32_t* brick);
 

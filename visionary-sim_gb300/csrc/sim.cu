@@ -1318,6 +1318,11 @@ int vsim_set_launch_shape(vsim_sim* s, uint32_t block, uint32_t brick) {
 
 int vsim_tune(vsim_sim* s, uint32_t frames, uint32_t* block, uint32_t* brick) {
     SIM_GUARD(s);
+    if (inRows(s)) {  // frames read neither: the caller's stay
+        if (block) *block = s->block;
+        if (brick) *brick = s->brick;
+        return VSIM_OK;
+    }
     if (frames < 1) frames = 1;
     const size_t N = s->nodeCount;
     std::vector<float> saved(12 * N);
