@@ -49,7 +49,7 @@ struct DeviceState {
     float4* sMoved = nullptr;     //   ... its motion over the substep, its body's friction
     uint32_t* sRec = nullptr;     //   ... its record index
     uint32_t* sKey = nullptr;     //   ... its bucket
-    // the two-launch chain (launchContactSlots; null where it is not used)
+    // the two-launch chain (launchContactSlots; null where it is not used; one allocation)
     uint4* slots = nullptr;       // per bucket: its first kSlots arrivals
     uint32_t* over = nullptr;     // per bucket: the last arrival past those
     uint32_t* next = nullptr;     // per record past its bucket's slots, up to the 32nd: the one that arrived before it

@@ -168,28 +168,41 @@ void countCells(vsim_sim* s) {
 // colour and body the cells run in lattice order, or brick by brick when
 // `brick` is 4 or 8 (bricks of that many cells per axis).
 void buildCells(const vsim_sim* s, std::vector<uint4>& out) {
-    out.clear();
-    out.reserve(s->cellCount);
+    out.resize(s->cellCount);
+    uint4* at = out.data();
     for (int c = 0; c < 8; c++)
         for (size_t b = 0; b < s->lat.size(); b++) {
             const Lattice& L = s->lat[b];
-            std::vector<uint32_t> order(L.cellsByColor[c]);
+            const uint32_t cx = L.cellDims[0], cy = L.cellDims[1];
+            const uint32_t nx = L.nodeDims[0], nxy = L.nodeDims[0] * L.nodeDims[1];
             if (s->brick > 1) {
+                std::vector<uint32_t> order(L.cellsByColor[c]);
                 const uint32_t B = s->brick;
                 auto brickKey = [&](uint32_t cell) {
-                    const uint32_t i = cell % L.cellDims[0], j = (cell / L.cellDims[0]) % L.cellDims[1],
-                                   k = cell / (L.cellDims[0] * L.cellDims[1]);
-                    const uint32_t bx = (L.cellDims[0] + B - 1) / B, by = (L.cellDims[1] + B - 1) / B;
+                    const uint32_t i = cell % cx, j = (cell / cx) % cy, k = cell / (cx * cy);
+                    const uint32_t bx = (cx + B - 1) / B, by = (cy + B - 1) / B;
                     return uint64_t((i / B) + bx * ((j / B) + by * (k / B))) << 32 | cell;
                 };
                 std::sort(order.begin(), order.end(),
                           [&](uint32_t a, uint32_t bb) { return brickKey(a) < brickKey(bb); });
+                for (uint32_t cell : order) {
+                    const uint32_t i = cell % cx, j = (cell / cx) % cy, k = cell / (cx * cy);
+                    *at++ = make_uint4(s->offsets[b] + i + nx * j + nxy * k, uint32_t(b), nx, nxy);
+                }
+                continue;
             }
-            for (uint32_t cell : order) {
-                const uint32_t i = cell % L.cellDims[0], j = (cell / L.cellDims[0]) % L.cellDims[1],
-                               k = cell / (L.cellDims[0] * L.cellDims[1]);
-                out.push_back(make_uint4(s->offsets[b] + i + L.nodeDims[0] * (j + L.nodeDims[1] * k), uint32_t(b),
-                                         L.nodeDims[0], L.nodeDims[0] * L.nodeDims[1]));
+            // Lattice order: rows come one after the other, no division a cell.
+            uint32_t j = 0, rowFirst = 0, node = s->offsets[b];  // the row's first cell, and that cell's node
+            for (uint32_t cell : L.cellsByColor[c]) {
+                while (cell - rowFirst >= cx) {
+                    rowFirst += cx;
+                    node += nx;
+                    if (++j == cy) {
+                        j = 0;
+                        node += nx;  // a slice has one row of nodes more than of cells
+                    }
+                }
+                *at++ = make_uint4(node + (cell - rowFirst), uint32_t(b), nx, nxy);
             }
         }
 }
@@ -581,7 +594,7 @@ void freeSim(vsim_sim* s) {
     DeviceState& d = s->d;
     void* ptrs[] = {d.pos, d.prev, d.vel, d.baseW, d.active, d.activeBody, d.cells, d.bodies, d.fp,
                     d.surf, d.key, d.rank, d.entries, d.count, d.start, d.cursor, d.delta, d.driven,
-                    d.drivenOffset, d.drivenOf, d.rows, d.slots, d.over, d.next, d.recPos, d.crowds.lowest, d.nodeRecord, d.sMeta, d.sPos, d.sMoved, d.sRec, d.sKey, d.bodyActive, d.grabs,
+                    d.drivenOffset, d.drivenOf, d.rows, d.slots, d.nodeRecord, d.sMeta, d.sPos, d.sMoved, d.sRec, d.sKey, d.bodyActive, d.grabs,
                     s->chunkDev, s->staging, s->pairs, s->pairCount, s->sp.embed, s->sp.quat,
                     s->sp.scaleBody, s->sp.bodies, s->sp.means, s->sp.cov, s->sp.keys, s->sp.order,
                     s->sp.sortTemp, s->sp.axesRotation, s->sp.axesScale};
@@ -660,34 +673,36 @@ void makeSlots(vsim_sim* s) {
     // twice as many places as there can be crowds
     uint32_t places = 2;
     while (places < 2 * (s->surfaceCount / (kBucketSlots + 1) + 1)) places *= 2;
-    const size_t words = size_t(places) * (2 * kBucketSlots + 2) + 2;
+    // one block: a vector a bucket and a record, the crowds' rows, then words
+    const size_t vectors = s->bucketTotal + s->surfaceCount + size_t(places) * (2 * kBucketSlots / 4);
+    const size_t words = s->bucketTotal + s->surfaceCount + 2 * size_t(places) + 2;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     cudaThreadExchangeStreamCaptureMode(&mode);
-    uint4* slots = nullptr;
-    Crowds& c = d.crowds;
-    cudaError_t e = allocN(&slots, s->bucketTotal);
-    if (!e) e = allocN(&d.over, s->bucketTotal);
-    if (!e) e = allocN(&d.next, s->surfaceCount);
-    if (!e) e = allocN(&d.recPos, s->surfaceCount);
-    if (!e) e = allocN(&c.lowest, words);
-    if (!e) e = cudaMemsetAsync(c.lowest, 0xff, (words - 2) * 4, s->capture);
-    if (!e) e = cudaMemsetAsync(c.lowest + words - 2, 0, 8, s->capture);
-    if (!e) e = cudaStreamSynchronize(s->capture);
+    uint4* block = nullptr;
+    cudaError_t e = allocN(&block, vectors + (words + 3) / 4);
     if (!e) {
+        d.recPos = reinterpret_cast<float4*>(block + s->bucketTotal);
+        Crowds& c = d.crowds;
+        c.lowest = reinterpret_cast<uint32_t*>(d.recPos + s->surfaceCount);
         c.ordered = c.lowest + size_t(places) * kBucketSlots;
         c.bucket = c.ordered + size_t(places) * kBucketSlots;
         c.used = c.bucket + places;
         c.count = c.used + places;
         c.gathered = c.count + 1;
         c.mask = places - 1;
-        d.slots = slots;
+        d.over = c.gathered + 1;
+        d.next = d.over + s->bucketTotal;
+        e = cudaMemsetAsync(c.lowest, 0xff, size_t(places) * (2 * kBucketSlots + 1) * 4, s->capture);
+        if (!e) e = cudaMemsetAsync(c.count, 0, 8, s->capture);
+        if (!e) e = cudaStreamSynchronize(s->capture);
+    }
+    if (!e) {
+        d.slots = block;
     } else {
-        for (void* p : {static_cast<void*>(slots), static_cast<void*>(d.over), static_cast<void*>(d.next),
-                        static_cast<void*>(d.recPos), static_cast<void*>(c.lowest)})
-            if (p) cudaFree(p);
+        if (block) cudaFree(block);
         d.over = d.next = nullptr;
         d.recPos = nullptr;
-        c = Crowds{};
+        d.crowds = Crowds{};
         cudaGetLastError();
     }
     cudaThreadExchangeStreamCaptureMode(&mode);
