@@ -116,6 +116,14 @@ void frameParams(vsim_sim* s) {
 
 // Uploads what changed since the last frame, in stream order.
 int syncParams(vsim_sim* s) {
+    if (s->slotsFilling) {  // their first values come by another stream
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        const cudaError_t e = cudaStreamSynchronize(s->capture);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        CK(e, "fill contact slots");
+        s->slotsFilling = false;
+    }
     if (s->tablesDirty) {
         // Through pinned staging; the staging may still feed a copy queued
         // by an earlier frame, so let the stream drain before rewriting it
@@ -694,10 +702,10 @@ void makeSlots(vsim_sim* s) {
         d.next = d.over + s->bucketTotal;
         e = cudaMemsetAsync(c.lowest, 0xff, size_t(places) * (2 * kBucketSlots + 1) * 4, s->capture);
         if (!e) e = cudaMemsetAsync(c.count, 0, 8, s->capture);
-        if (!e) e = cudaStreamSynchronize(s->capture);
     }
     if (!e) {
         d.slots = block;
+        s->slotsFilling = true;
     } else {
         if (block) cudaFree(block);
         d.over = d.next = nullptr;

@@ -90,6 +90,7 @@ struct vsim_sim {
     // settings
     double gravity[3] = {0, -9.81, 0};
     bool paused = false, pendingStep = false;
+    bool slotsFilling = false;  // the contact slots' first values are on their way (on `capture`)
     bool contact = true, selfContact = false;
     uint32_t iterations = 1;
     bool useGraph = true, pdl = true;
