@@ -50,7 +50,10 @@ for p in (ROOT / "visionary-sim_gb300", ROOT / "oracle"):
         sys.path.insert(0, str(p))
 
 METRIC = "cell-updates/s"
-BYTES_PER_ELASTIC_CELL = 8 * 48  # 8 corner nodes: pos 16 B read, prev 16 B read, pos 16 B written
+BYTES_PER_ELASTIC_CELL = 8 * 48  # a colour pass: 8 corner nodes: pos 16 B read, prev 16 B read, pos 16 B written
+BYTES_PER_ROW_NODE = 48  # a row pass: every material node's once
+BYTES_PER_ROW_CELL = 16  # its place in a group's table
+BYTES_PER_SPLAT = 88  # deformation: 48 B read; mean 12, covariance 24, key 4 written
 VIEW = (0.3, -0.25, -0.92)
 
 
@@ -178,37 +181,53 @@ def replica_throughput(local_seconds: float, units_per_rank: int, device):
     return total, units_per_rank * world / total
 
 
-def colour_pass_rate(sim, sweeps: int = 10):
-    """The elastic passes timed as the frame runs them: `sweeps` sweeps of the
-    eight colours (two to a launch where rows are packed) back to back in one
-    graph (programmatic dependent launch), events at the two ends only
-    (vsim_time_colour_passes; state restored). Returns (algorithmic bytes per
-    colour, average seconds a colour)."""
-    counts = sim.color_counts()
-    passes = sweeps * int(np.count_nonzero(counts))
+def sweep_launches(sim):
+    """Launches of one elastic sweep: four row passes or the eight colours (0
+    where a frame is one launch)."""
+    iterations = sim.stats()["iterations"]
+    sim.set_iterations(iterations + 1)
+    more = sim.frame_launches(1)
+    sim.set_iterations(iterations)
+    return more - sim.frame_launches(1)
+
+
+def elastic_pass_rate(sim, sweeps: int = 10):
+    """The elastic passes timed as the frame runs them: `sweeps` sweeps back to
+    back in one graph (programmatic dependent launch), events at the two ends
+    only (vsim_time_colour_passes; state restored). Returns (algorithmic bytes
+    per launch, average seconds a launch, launches a sweep). A row pass loads
+    and stores every node about once for two colours; a colour pass the eight
+    corners of each of its cells."""
+    launches = sweep_launches(sim)
+    cells = int(sim.color_counts().sum())
+    if launches == 4:
+        sweep_bytes = 4 * BYTES_PER_ROW_NODE * sim.stats()["active_nodes"] + BYTES_PER_ROW_CELL * cells
+    else:
+        launches = int(np.count_nonzero(sim.color_counts()))
+        sweep_bytes = BYTES_PER_ELASTIC_CELL * cells
     ms = sim.time_colour_passes(sweeps)
-    return int(counts.sum()) * sweeps * BYTES_PER_ELASTIC_CELL / passes, ms / 1e3 / passes
+    return sweep_bytes / launches, ms / 1e3 / (sweeps * launches), launches
 
 
 def roofline(sim, scene, hbm):
-    """The dominant kernel's roofline: the elastic passes, per colour.
-    `achieved` is algorithmic bytes per colour over the average time a colour
-    with the passes back to back as in the frame; `isolated_launch_us` is a
-    colour's share of launches bracketed by events on their own (no overlap
-    with their neighbours)."""
+    """The dominant kernel's roofline: the elastic pass, per launch (two colours
+    where rows are packed). `achieved` is algorithmic bytes per launch over the
+    average time a launch with the passes back to back as in the frame;
+    `isolated_launch_us` is a launch bracketed by events on its own (no overlap
+    with its neighbours)."""
     prof = sim.profile_frame(scene.substeps, splats=True, view_dir=VIEW)
     ms, launches = prof["elastic"]
-    per_launch_bytes, per_launch_s = colour_pass_rate(sim)
+    per_launch_bytes, per_launch_s, per_sweep = elastic_pass_rate(sim)
     achieved = per_launch_bytes / per_launch_s / 1e9
-    # The same passes with each cell split over four lanes (vsim_set_cell_lanes).
+    # The same cells split over four lanes each (vsim_set_cell_lanes), a colour a launch.
     sim.set_cell_lanes(4)
-    _, quad_s = colour_pass_rate(sim)
+    _, quad_s, _ = elastic_pass_rate(sim)
     sim.set_cell_lanes(1)
     traffic = profiled_traffic()
     share = {k: round(v[0] / sum(x[0] for x in prof.values()), 4) for k, v in prof.items()}
     return {
         "bound": "hbm",
-        "kernel": "elasticRowKernel (two colours a launch; figures are per colour)",
+        "kernel": "elasticRowKernel (two colours a launch)" if per_sweep == 4 else "elasticKernel (a colour a launch)",
         "achieved": round(achieved, 1),
         "peak": hbm,
         "unit": "GB/s",
@@ -216,10 +235,10 @@ def roofline(sim, scene, hbm):
         "traffic": traffic,
         "bytes_per_launch": round(per_launch_bytes),
         "avg_launch_us": round(per_launch_s * 1e6, 3),
-        "isolated_launch_us": round(1e3 * ms / (scene.substeps * scene.iterations *
-                                                 int(np.count_nonzero(sim.color_counts()))), 3),
+        "isolated_launch_us": round(1e3 * ms / launches, 3),
+        "launches_per_sweep": per_sweep,
         "method": "10 sweeps of the 8 colours back to back in one graph, CUDA events at its ends",
-        "four_lanes_a_cell_launch_us": round(quad_s * 1e6, 3),
+        "four_lanes_a_cell_launch_us": round(quad_s * 1e6, 3),  # one colour
     }, {k: {"ms": round(v[0], 4), "launches": v[1]} for k, v in prof.items()}, share
 
 
@@ -235,16 +254,26 @@ CONTACT_BYTES = {"bin": (48, 0, 0), "segment": (8, 8, 0), "scatter": (16, 0, 0),
                  "gather": (56 + 27 * 8 + 16, 0, 48)}  # (per record, per occupied bucket, per candidate)
 
 
-def contact_roofline(sim, hbm):
-    """The contact chain on the current positions (vsim_contact_census, one
-    launch of each kernel bracketed by events): its work counted from the
-    live grid -- records, occupied buckets, visible candidates -- and each
-    kernel's achieved bandwidth over its algorithmic bytes. Also the total by
-    the per-surface-node formula (key 8 B, an 8 B read+write per sort pass --
-    here 4 passes: bin, segment, scatter, order -- the 27 buckets' 8 B, 36 B
-    per candidate, 32 B to apply)."""
+# The two-launch contact, each record's data once: bin: record 16 + position 16 +
+# activity 4 read, bucket and place 8, position 16, its slot 4 written, its count 8
+# (r/w); gather: place 4 + record 16 + position 16 read, correction 16 written, and
+# every occupied bucket's count 4 and slots 16
+SLOTS_BYTES = (72 + 52, 20)  # (per record, per occupied bucket)
+
+
+def contact_roofline(sim, substeps, hbm):
+    """`two_launches`: contact as the frame runs it (a frame's launches, each
+    bracketed by events). `kernels`: the five-launch chain, which other scenes
+    take, on the current positions (vsim_contact_census, one launch of each
+    kernel bracketed by events): its work counted from the live grid -- records,
+    occupied buckets, visible candidates -- and each kernel's achieved bandwidth
+    over its algorithmic bytes. Also the chain's total by the per-surface-node
+    formula (key 8 B, an 8 B read+write per sort pass -- here 4 passes: bin,
+    segment, scatter, order -- the 27 buckets' 8 B, 36 B per candidate, 32 B to
+    apply)."""
     sim.contact_census()  # the chain's kernels loaded: frames run another
     c = sim.contact_census()
+    frame_ms, frame_launches = sim.profile_frame(substeps).get("contact", (0.0, 0))
     r, b, k = c["records"], c["occupied_buckets"], c["candidates"]
     per = {}
     for name, (pr, pb, pc) in CONTACT_BYTES.items():
@@ -255,13 +284,20 @@ def contact_roofline(sim, hbm):
                      "frac_of_measured_hbm": round(gbs / hbm, 4) if gbs else None}
     formula = r * (8 + 4 * 16 + 27 * 8 + 32) + 36 * k
     total_ms = sum(c["ms"].values())
-    return {"records": r, "occupied_buckets": b, "candidates": k,
+    slots = SLOTS_BYTES[0] * r + SLOTS_BYTES[1] * b
+    two = None
+    if frame_launches == 2 * substeps and frame_ms > 0:
+        gbs = slots / (frame_ms / substeps / 1e3) / 1e9
+        two = {"bytes": slots, "us": round(frame_ms / substeps * 1e3, 2), "achieved_gbs": round(gbs, 1),
+               "frac_of_measured_hbm": round(gbs / hbm, 4),
+               "method": "a frame's contact launches, each bracketed by CUDA events, over its substeps"}
+    return {"records": r, "occupied_buckets": b, "candidates": k, "two_launches": two,
             "candidates_per_record": round(k / r, 2) if r else 0,
             "kernels": per, "chain_us": round(total_ms * 1e3, 2),
             "formula_bytes": formula,
             "formula_gbs": round(formula / (total_ms / 1e3) / 1e9, 1) if total_ms else None,
             "formula_frac_of_measured_hbm": round(formula / (total_ms / 1e3) / 1e9 / hbm, 4) if total_ms else None,
-            "method": "one contact chain on the bench body's current positions, each kernel bracketed by CUDA "
+            "method": "one five-launch chain on the bench body's current positions, each kernel bracketed by CUDA "
                       "events (no overlap between kernels), then the grid emptied without moving a node"}
 
 
@@ -475,23 +511,23 @@ def batch_cpu_baseline(scene, budget_s: float):
 
 
 def single_body_pass(quick: bool, hbm: float):
-    """The colour pass of one large body alone: the stress workload's 192^3
+    """The elastic pass of one large body alone: the stress workload's 192^3
     noise blob without the sheet (48^3 with --quick), timed as
-    colour_pass_rate times it."""
+    elastic_pass_rate times it."""
     import vsim.scenes as sc
     from vsim import Simulator
 
     scene = sc.noise_blob(n=48 if quick else 192, seed=4, splats=0)
     sim = Simulator(scene)
-    per_launch, per_launch_s = colour_pass_rate(sim)
+    per_launch, per_launch_s, per_sweep = elastic_pass_rate(sim)
     achieved = per_launch / per_launch_s / 1e9
     out = {"workload": f"noise blob {scene.bodies[0].cell_dims[0]}^3 alone, {scene.cells} cells",
            "achieved_gbs": round(achieved, 1), "frac_of_measured_hbm": round(achieved / hbm, 4),
-           "bytes_per_launch": round(per_launch), "avg_launch_us": round(per_launch_s * 1e6, 2)}
-    # The same passes in the TMA brick form (vsim_set_tma_pass), measured
-    # against the streaming form it would replace.
+           "bytes_per_launch": round(per_launch), "avg_launch_us": round(per_launch_s * 1e6, 2),
+           "launches_per_sweep": per_sweep}
+    # The same cells in the TMA brick form (vsim_set_tma_pass), a colour a launch.
     sim.set_tma_pass(True)
-    per_launch, per_launch_s = colour_pass_rate(sim)
+    per_launch, per_launch_s, _ = elastic_pass_rate(sim)
     sim.synchronize()
     achieved = per_launch / per_launch_s / 1e9
     out["tma_bricks"] = {"achieved_gbs": round(achieved, 1), "frac_of_measured_hbm": round(achieved / hbm, 4),
@@ -520,7 +556,7 @@ def stress(quick: bool, hbm: float, frames: int = 3):
     times = time_frames(sim, scene, stream, frames, flush)
     prof = sim.profile_frame(scene.substeps, splats=True, view_dir=VIEW)
     ms, launches = prof["elastic"]
-    per_launch, per_launch_s = colour_pass_rate(sim)
+    per_launch, per_launch_s, per_sweep = elastic_pass_rate(sim)
     achieved = per_launch / per_launch_s / 1e9
     n_splats = sim.splat_count
     sort_ms, sort_launches = prof.get("sort", (0.0, 0))
@@ -532,10 +568,10 @@ def stress(quick: bool, hbm: float, frames: int = 3):
            "frame_ms": round(1e3 * statistics.median(times), 3),
            "elastic_pass": {"achieved_gbs": round(achieved, 1), "frac_of_measured_hbm": round(achieved / hbm, 4),
                             "bytes_per_launch": round(per_launch), "avg_launch_us": round(per_launch_s * 1e6, 2),
-                            "isolated_launch_us": round(1e3 * ms / launches, 2),
+                            "isolated_launch_us": round(1e3 * ms / launches, 2), "launches_per_sweep": per_sweep,
                             "method": "10 sweeps of the 8 colours back to back in one graph"},
            "single_body_elastic_pass": single_body_pass(quick, hbm),
-           "splat_deform_gbs": round(92 * n_splats / (splat_ms / 1e3) / 1e9, 1) if splat_ms else None,
+           "splat_deform_gbs": round(BYTES_PER_SPLAT * n_splats / (splat_ms / 1e3) / 1e9, 1) if splat_ms else None,
            "sort_keys_per_s": round(n_splats / (sort_ms / 1e3)) if sort_ms else None,
            "kernel_groups_one_frame": {k: {"ms": round(v[0], 3), "launches": v[1]} for k, v in prof.items()},
            "scene_generation_s": round(gen_s, 1)}
@@ -1049,7 +1085,7 @@ def main():
     e2e_value = units_per_frame(scene) / statistics.mean(e2e_times) * world
 
     detail = {"kernel_groups_one_frame": groups, "time_share": share,
-              "contact_roofline": contact_roofline(sim, hbm),
+              "contact_roofline": contact_roofline(sim, scene.substeps, hbm),
               "frame_ms": {"min": round(min(times) * 1e3, 4), "median": round(statistics.median(times) * 1e3, 4)}}
     if rank == 0 and not args.no_batch:
         detail["batching"] = batched_vs_plain(10, args.quick, cpu=not args.no_cpu)

@@ -371,7 +371,9 @@ typedef struct vsim_profile {
 /* Run one frame of `steps` substeps (plus the splat deformation and sort
    when `with_splats`) with every kernel launched on its own, bracketed by
    CUDA events on the handle's stream, and report the device time of each
-   kernel group. The frame advances the simulation like vsim_dispatch. */
+   kernel group. A small scene whose frame is one launch otherwise
+   (vsim_frame_launches) runs its passes one by one here. The frame advances the
+   simulation like vsim_dispatch. */
 int vsim_profile_frame(vsim_sim* sim, uint32_t steps, int with_splats, const float view_dir[3],
                        vsim_profile* out);
 /* Time `sweeps` Gauss-Seidel sweeps of the elastic colour passes (each all
